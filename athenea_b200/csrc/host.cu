@@ -55,7 +55,8 @@ struct ath_raster {
     uint32_t lastSlots = 0, lastTiles = 0, lastSorted = 0;   // what frame_buffers describes
     FrameConst lastFrame{};
     // the differentiable frame's state (ath_raster_render_params -> ath_raster_backward)
-    DeviceBuffer finalT, lastContrib, grads;
+    DeviceBuffer finalT, lastContrib, live, grads;
+    bool trainingOnePixel = false;
     bool trainingValid = false;
     InstanceConst trainingInstance{};
     const float* trainingDepth = nullptr;
@@ -344,7 +345,7 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     r->slotCapacity = r->pairCapacity = r->tileCapacity = r->instanceCapacity = 0;
     for (DeviceBuffer* b : {&r->recs, &r->rects, &r->keys, &r->offsets, &r->projectFlags, &r->instances,
                             &r->pairKeys[0], &r->pairKeys[1], &r->pairVals[0], &r->pairVals[1], &r->sortHist,
-                            &r->sortFlags, &r->ranges, &r->finalT, &r->lastContrib, &r->grads})
+                            &r->sortFlags, &r->ranges, &r->finalT, &r->lastContrib, &r->live, &r->grads})
         b->release();
     r->trainingValid = false;
     r->frameRecorded = false;
@@ -487,6 +488,12 @@ uint64_t lastFrameNeed(ath_raster* r) {
     return pairsOf(static_cast<const uint32_t*>(r->statusHost.ptr));
 }
 
+// What the last differentiable frame kept, for its blend to write and its backward to read.
+TrainingState trainingState(const ath_raster* r) {
+    return TrainingState{static_cast<float*>(r->finalT.ptr), static_cast<uint32_t*>(r->lastContrib.ptr),
+                         static_cast<uint32_t*>(r->live.ptr), r->trainingOnePixel};
+}
+
 // One frame: project (scan fused), emit, sort, ranges, blend, with nothing read
 // back in between. The pairs are sized from a capacity: a handle's first frame
 // (and its first after release_scratch) reads the pair total back once and sizes
@@ -583,16 +590,22 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                            words + kWordSticky, stream);
     mark(4);
     // --- blend ---------------------------------------------------------------
+    const Contribution contrib{s.contribution_mode, s.contribution, s.final_colour, s.lift_mask};
+    const Matte matte{s.crypto_ids, s.crypto, under ? s.under_crypto : nullptr, s.matte_lift, s.matte,
+                      s.matte_hard != 0 ? 1u : 0u, s.matte_threshold, s.trace};
+    TrainingState keep;
+    if (training) {
+        if (cudaError_t e = r->live.reserve(trainingLiveWords(F, capacity) * sizeof(uint32_t)); e != cudaSuccess)
+            return failCuda(e, "reserving the backward's live bits");
+        r->trainingOnePixel = trainingOnePixel(F, r->sms, contrib, matte);
+        keep = trainingState(r);
+    }
     if (err == cudaSuccess)
         err = launchBlend(F, capacity, slots, static_cast<const uint2*>(r->ranges.ptr), valsBuf[sorted],
                           static_cast<const float4*>(r->recs.ptr), reinterpret_cast<float4*>(targets->colour),
-                          targets->depth, reinterpret_cast<float4*>(targets->position),
-                          training ? static_cast<float*>(r->finalT.ptr) : nullptr,
-                          training ? static_cast<uint32_t*>(r->lastContrib.ptr) : nullptr, words + kWordSticky, stream,
-                          Contribution{s.contribution_mode, s.contribution, s.final_colour, s.lift_mask},
-                          under ? Under{under->colour, under->depth} : Under{},
-                          Matte{s.crypto_ids, s.crypto, under ? s.under_crypto : nullptr, s.matte_lift, s.matte,
-                                s.matte_hard != 0 ? 1u : 0u, s.matte_threshold, s.trace});
+                          targets->depth, reinterpret_cast<float4*>(targets->position), training ? &keep : nullptr,
+                          r->sms, words + kWordSticky, stream, contrib,
+                          under ? Under{under->colour, under->depth} : Under{}, matte);
     mark(5);
     // --- the frame's words: its counters into the ring; its status behind an event
     // (last, so that a wait for the frame covers both)
@@ -780,8 +793,7 @@ extern "C" ath_status ath_raster_backward(ath_raster* r, const float* dlDcolour,
     if (err == cudaSuccess)
         err = launchBlendBackward(F, r->pairCapacity, slots, static_cast<const uint2*>(r->ranges.ptr),
                                   static_cast<const uint32_t*>(r->pairVals[r->lastSorted].ptr),
-                                  static_cast<const float4*>(r->recs.ptr), static_cast<const float*>(r->finalT.ptr),
-                                  static_cast<const uint32_t*>(r->lastContrib.ptr),
+                                  static_cast<const float4*>(r->recs.ptr), trainingState(r),
                                   reinterpret_cast<const float4*>(dlDcolour), dlDdepth, r->trainingDepth,
                                   static_cast<float*>(r->grads.ptr), words + kWordSticky, stream);
     if (err == cudaSuccess)

@@ -77,16 +77,30 @@ struct Matte {
     uint32_t* trace = nullptr;            // the splats a pixel is made of (splat_trace.slang), kTraceWords planes
 };
 
+// What a differentiable frame keeps for its backward: per pixel the final transmittance
+// and one past the last record blended; per box of pixels the records of the tile's list
+// some pixel blended (walk.cuh).
+struct TrainingState {
+    float* finalT = nullptr;
+    uint32_t* lastContrib = nullptr;
+    uint32_t* live = nullptr;
+    bool onePixel = false;
+};
+
 cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
                         const uint32_t* pairValues, const float4* recs, float4* colour, float* depth, float4* position,
-                        float* finalT, uint32_t* lastContrib, uint32_t* status, cudaStream_t stream,
+                        const TrainingState* training, int sms, uint32_t* status, cudaStream_t stream,
                         const Contribution& contrib = Contribution{}, const Under& under = Under{},
                         const Matte& matte = Matte{});
+// Whether a differentiable frame's boxes hold one pixel a lane (onePixelBoxes; always with the
+// contribution or matte hooks), and the words its live bits take.
+bool trainingOnePixel(const FrameConst& F, int sms, const Contribution& contrib, const Matte& matte);
+size_t trainingLiveWords(const FrameConst& F, uint64_t pairs);
 
 // backward.cu
 cudaError_t launchBlendBackward(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
-                                const uint32_t* pairValues, const float4* recs, const float* finalT,
-                                const uint32_t* lastContrib, const float4* dLdColour, const float* dLdDepth,
+                                const uint32_t* pairValues, const float4* recs, const TrainingState& training,
+                                const float4* dLdColour, const float* dLdDepth,
                                 const float* depthOut, float* grads, uint32_t* status, cudaStream_t stream);
 cudaError_t launchProjectBackward(const FrameConst& F, const InstanceConst& I, const uint32_t* keys,
                                   const float* grads, float4* gMeans, float4* gScales, float4* gQuats, float* gSh,
