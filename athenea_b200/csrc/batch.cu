@@ -66,6 +66,8 @@ __global__ void beginStepKernel(uint32_t* words) {
     words[kBatchDegenerate] = 0;
     words[kBatchExpMin] = 0xFFu;
     words[kBatchExpMax] = 0u;
+    words[kBatchLoss] = words[kBatchLoss + 1] = 0u;
+    words[kBatchLossBlocks] = 0u;
 }
 
 // Block b's word of an epoch-tagged look-back: its aggregate (its inclusive
@@ -1072,7 +1074,6 @@ cudaError_t enqueueStep(ath_batch* b, const ath_mixed_params& P, const float* ta
             err = cudaStreamWaitEvent(stream, targetReady,
                                       capturing == cudaStreamCaptureStatusActive ? cudaEventWaitExternal : 0);
     }
-    if (err == cudaSuccess && train) err = cudaMemsetAsync(loss, 0, sizeof(float), stream);
     if (err == cudaSuccess && train && P.count)
         err = cudaMemsetAsync(b->seen.ptr, 0, (size_t)B.views * P.count, stream);
     // the forward blend, the loss and the blend adjoint (the record gradients were cleared by the projection)

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "batch_kernels.cuh"
+#include "walk.cuh"
 
 namespace ath {
 namespace {
@@ -81,33 +82,16 @@ __device__ __forceinline__ float blendFloor(float cutoffExp, float lgOpacity) {
     return fmaxf(cutoffExp + lgOpacity, kLog2Faint);
 }
 
-// Nine values summed over a warp: the first eight by a transposed reduction
-// (each level sends half of the values still held and keeps the other half,
-// so three levels leave value (lane >> 2) spread over lanes differing in their
-// two low bits), the ninth by a butterfly over the same three levels; the last
-// two levels take the pair (value lane >> 2, the ninth) transposed as well.
-// Lanes with lane % 4 == 0 end with value lane >> 2, lanes with lane % 4 == 2
-// with the ninth. Every sum adds the same terms in the same pairs as a
-// butterfly over each value alone, so the results are those of one.
-__device__ __forceinline__ float warpSum9(float v[9], uint32_t lane) {
-#pragma unroll
-    for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-        const bool upper = (lane & (uint32_t)bit) != 0;
-#pragma unroll
-        for (int k = 0; k < half; ++k) {
-            const float send = upper ? v[k] : v[k + half];
-            const float keep = upper ? v[k + half] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, bit);
-        }
-    }
-    float n = v[8];
-#pragma unroll
-    for (int o = 16; o > 2; o >>= 1) n += __shfl_xor_sync(0xFFFFFFFFu, n, o);
-    const bool upper = (lane & 2u) != 0;
-    float s = (upper ? n : v[0]) + __shfl_xor_sync(0xFFFFFFFFu, upper ? v[0] : n, 2);
-    s += __shfl_xor_sync(0xFFFFFFFFu, s, 1);
-    return s;
-}
+// The adjoint's sums over a warp, kSumRecords records at a time through shared memory:
+// each lane stores its nine values of a record in nine columns (a column: one value of
+// one record, the warp's 32 lanes side by side), then lane k sums column k's 32 values
+// by eight 16-byte loads and adds the total into the record's word in global memory.
+// A record's nine sums cost 9 stores and a third of 8 loads and 31 adds; summing them by
+// shuffles (a transposed reduction of eight, the ninth beside it) took 12 shuffles, 12
+// adds and 16 selects a record, and nine lanes' reductions a record instead of 27 lanes'
+// for three.
+constexpr uint32_t kSumWords = 9;     // moments t, dy, tt, t dy, dy dy; alpha; colour r g b
+constexpr uint32_t kSumRecords = 3;   // 27 of 32 lanes take a column
 
 // ---- the blends of a training step: forward, loss and adjoint, a tile at a time ----
 // One block of T*T/2 threads takes tiles off a queue (heaviest first: `order`,
@@ -118,7 +102,8 @@ __device__ __forceinline__ float warpSum9(float v[9], uint32_t lane) {
 // registers between the two walks.
 //
 // Forward: warp w owns an 8x8 box of the tile and each lane two pixels of it,
-// (x, y) and (x, y + 4). Staging a batch of records, the block marks for each
+// (x, y) and (x + 4, y): one dy a lane, so that the terms in dy alone, and in the
+// adjoint the factors dy of the moments, are formed once for both. Staging a batch of records, the block marks for each
 // record the boxes its footprint can reach (a conservative test: the box's least
 // power against the cutoff, with a margin); a warp then walks only the records
 // marked for its box, found 32 at a time by a ballot, in list order. A pixel
@@ -130,8 +115,9 @@ __device__ __forceinline__ float warpSum9(float v[9], uint32_t lane) {
 // block barrier): the forward marked, for each 32-record chunk of the tile's list
 // a warp walked, the records some pixel of its box blended (`live`, one word a
 // chunk and box); the warp gathers those records, last first, 32 at a time into
-// slots of its own and walks them from its pixels' last contributor down. What a
-// lane sums over its two pixels, and the warp over its 64, are moments of
+// slots of its own (shared memory that the forward's staged records held) and walks them
+// from its pixels' last contributor down. What a lane sums over its two pixels, and the
+// warp over its 64 (kSumRecords records at a time), are moments of
 // dP = -2 dL/dpower over the pixel offsets in the factored frame (t = dx + fr dy,
 // dy): sum dP t, sum dP dy, sum dP t^2, sum dP t dy, sum dP dy^2. Each visit's warp
 // sums are added into the record's gradient words in global memory as they are
@@ -157,26 +143,41 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
     constexpr uint32_t kAcross = S / kBox;            // boxes across a block's span
     constexpr uint32_t kSpans = (T / S) * (T / S);    // spans (blocks' work units) a tile
     constexpr uint32_t kBoxes = (T / kBox) * (T / kBox);   // boxes a tile (the live words' row)
-    constexpr uint32_t kWords = 9;   // moments t, dy, tt, t dy, dy dy; alpha; colour r g b
-    // a staged record, 48 bytes at one address: centre (cx, cy, depth); conic (ca, fs
-    // pre-scaled, fr; log2 of the opacity); colour (r g b; the least exponent that blends)
-    __shared__ float4 sStaged[NB][3];
-    __shared__ uint32_t sMask[NB];
-    __shared__ uint32_t sRec[NB];
+    // The forward's staged records: 48 bytes at one address, centre (cx, cy, depth); conic
+    // (ca, fs pre-scaled, fr; log2 of the opacity); colour (r g b; the least exponent that
+    // blends); then each record's boxes and index. The adjoint's, a warp's own, in the same
+    // memory after the forward: 32 gathered records, what the packed arithmetic of a lane's
+    // two pixels takes stored twice, so that a broadcast load gives the pair; then the
+    // columns of the sums.
+    struct Forward {
+        float4 staged[NB][3];
+        uint32_t mask[NB], rec[NB];
+    };
+    struct alignas(16) Gathered {   // 80 bytes: with the columns, eight blocks' fit an SM
+        float nx[2], ny[2];         // minus the centre
+        float ca[2], fr[2];         // the conic, its weights pre-scaled
+        float fs[2], lgo[2];        // and log2 of the opacity
+        float r[2], g[2], bl[2];    // the colour
+        float least;                // the least exponent that blends
+        uint32_t rel;               // its place in the tile's list
+    };
+    struct Adjoint {
+        Gathered records[32];
+        uint32_t rec[32];           // their records
+        float sums[kSumRecords * kSumWords * kColumnStride];
+    };
+    constexpr size_t kAdjointBytes = kTrain ? kThreads / 32 * sizeof(Adjoint) : 0;
+    constexpr size_t kBytes = sizeof(Forward) > kAdjointBytes ? sizeof(Forward) : kAdjointBytes;
+    __shared__ __align__(16) unsigned char sRaw[kBytes];
+    Forward& sF = *reinterpret_cast<Forward*>(sRaw);
     __shared__ uint32_t sTileBase[kMaxBatchViews];
     __shared__ uint32_t sTile;
-    // the adjoint's gather slots, a warp's own: 32 records, each its centre with its
-    // place in the tile's list and its record index (one 16-byte load a visit), its
-    // conic and its colour
-    constexpr uint32_t kWarpsHere = kTrain ? kThreads / 32 : 1;
-    __shared__ float4 sWarpCentre[kWarpsHere][32];
-    __shared__ float4 sWarpConic[kWarpsHere][32];
-    __shared__ float4 sWarpColour[kWarpsHere][32];
     for (uint32_t k = threadIdx.x; k < B.views; k += kThreads) sTileBase[k] = views[k].tileBase;
     const uint64_t slotMask = (1ull << B.slotBits) - 1ull;
     const float kScale = -0.5f * 1.4426950408889634f;   // power -> base-2 exponent
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t lx = (warp % kAcross) * kBox + (lane & 7u), ly = (warp / kAcross) * kBox + (lane >> 3);
+    const uint32_t lx = (warp % kAcross) * kBox + (lane & 3u), ly = (warp / kAcross) * kBox + (lane >> 2);
+    const uint32_t sumRecord = lane / kSumWords, sumWord = lane % kSumWords;   // the column this lane sums
     uint32_t evaluated = 0;   // (pixel, record) evaluations of the forward this thread made
     uint32_t blended = 0;     // of them, those that blended
     uint32_t adjVisited = 0, adjLive = 0;   // the adjoint's evaluations, and those that blended
@@ -198,25 +199,25 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         const uint32_t tx = local % V.tilesX, ty = local / V.tilesX;
         const uint32_t spanX = tx * T + (span % (T / S)) * S, spanY = ty * T + (span / (T / S)) * S;
         const float tileX0 = (float)spanX, tileY0 = (float)spanY;   // the span's first pixel
-        const uint32_t px = spanX + lx, py[2] = {spanY + ly, spanY + ly + 4};
+        const uint32_t px[2] = {spanX + lx, spanX + lx + 4}, py = spanY + ly;
         const uint2 range = ranges[tile];
-        const float pxc = (float)px + 0.5f, pyc[2] = {(float)py[0] + 0.5f, (float)py[1] + 0.5f};
+        const float pxc[2] = {(float)px[0] + 0.5f, (float)px[1] + 0.5f}, pyc = (float)py + 0.5f;
         const size_t recBase = (size_t)v * B.count;
         // record s of this view into slot k: the factored conic's two weights pre-scaled
         // to base-2 exponent units, log2 of its opacity, the least exponent that blends,
         // and the boxes it can reach
         auto stage = [&](uint32_t k, uint32_t s) {
             if constexpr (kCount) ++staged;
-            sRec[k] = s;
+            sF.rec[k] = s;
             const size_t at = (recBase + s) * 3;
             const float4 sc = recs[at + 0];
             const float4 c = recs[at + 1];
             const float4 rgb = recs[at + 2];
-            sStaged[k][0] = make_float4(sc.x, sc.y, sc.z, 0.0f);
+            sF.staged[k][0] = make_float4(sc.x, sc.y, sc.z, 0.0f);
             const float lgo = log2Of(c.w);
-            sStaged[k][1] = make_float4(c.x * kScale, c.y, c.z * kScale, lgo);
-            sStaged[k][2] = make_float4(rgb.x, rgb.y, rgb.z, blendFloor(kScale * sc.w, lgo));
-            sMask[k] = boxMask<S>(tileX0, tileY0, sc, c.x, c.y, c.z);
+            sF.staged[k][1] = make_float4(c.x * kScale, c.y, c.z * kScale, lgo);
+            sF.staged[k][2] = make_float4(rgb.x, rgb.y, rgb.z, blendFloor(kScale * sc.w, lgo));
+            sF.mask[k] = boxMask<S>(tileX0, tileY0, sc, c.x, c.y, c.z);
         };
 
         // ---- forward
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         uint32_t last[2] = {0, 0};
         bool done[2];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) done[p] = !(px < V.width && py[p] < V.height);
+        for (int p = 0; p < 2; ++p) done[p] = !(px[p] < V.width && py < V.height);
         for (uint32_t first = range.x; first < range.y; first += NB) {
             if (__syncthreads_count(done[0] && done[1]) == kThreads) break;
             const uint32_t count = min(NB, range.y - first);
@@ -233,26 +234,26 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
             __syncthreads();
             if (__all_sync(0xFFFFFFFFu, done[0] && done[1])) continue;
             for (uint32_t base = 0; base < count; base += 32) {
-                const uint32_t m = base + lane < count ? sMask[base + lane] : 0u;
+                const uint32_t m = base + lane < count ? sF.mask[base + lane] : 0u;
                 uint32_t todo = __ballot_sync(0xFFFFFFFFu, (m >> warp) & 1u);
                 uint32_t laneBits = 0;   // the records of this chunk a pixel of this lane blended
                 while (todo) {
                     const uint32_t j = base + (uint32_t)__ffs(todo) - 1u;
                     todo &= todo - 1u;
                     if constexpr (kCount) ++fwdVisits;
-                    const float4 ce = sStaged[j][0];
-                    const float4 k = sStaged[j][1];
-                    const float dx = pxc - ce.x;
-                    const float4 cc = sStaged[j][2];
+                    const float4 ce = sF.staged[j][0];
+                    const float4 k = sF.staged[j][1];
+                    const float4 cc = sF.staged[j][2];
+                    const float dy = pyc - ce.y;
+                    const float ey = __fmaf_rn(k.z * dy, dy, k.w);
                     bool hit = false;
                     // both pixels evaluated without branching: a pixel that does not blend the
                     // record (done, outside the cutoff, or under 1/255) takes alpha 0, which
                     // leaves its sums and transmittance as they were
 #pragma unroll
                     for (int p = 0; p < 2; ++p) {
-                        const float dy = pyc[p] - ce.y;
-                        const float t = __fmaf_rn(k.y, dy, dx);
-                        const float e = __fmaf_rn(k.x * t, t, __fmaf_rn(k.z * dy, dy, k.w));
+                        const float t = __fmaf_rn(k.y, dy, pxc[p] - ce.x);
+                        const float e = __fmaf_rn(k.x * t, t, ey);
                         const float a0 = fminf(0.99f, fastExp2(e));
                         const bool blend = !done[p] && e >= cc.w;
                         if constexpr (kCount) { evaluated += done[p] ? 0u : 1u; blended += blend ? 1u : 0u; }
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                     // the records some pixel blended take a gradient in the adjoint: mark them
                     // (lane l for record base + l; a plain store, every writer stores 1), by which
                     // the projection's adjoint groups Gaussians
-                    if ((liveWord >> lane) & 1u) seen[recBase + sRec[base + lane]] = 1u;
+                    if ((liveWord >> lane) & 1u) seen[recBase + sF.rec[base + lane]] = 1u;
                 }
                 if (__all_sync(0xFFFFFFFFu, done[0] && done[1])) break;
             }
@@ -289,9 +290,9 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         if constexpr (!kTrain) {
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-                if (!(px < V.width && py[p] < V.height)) continue;
+                if (!(px[p] < V.width && py < V.height)) continue;
                 const float coverage = 1.0f - Tr[p];
-                const uint32_t at = V.pixelBase + py[p] * V.width + px;
+                const uint32_t at = V.pixelBase + py * V.width + px[p];
                 colour[at] = make_float4(r[p] + Tr[p] * B.bg[0], g[p] + Tr[p] * B.bg[1], bl[p] + Tr[p] * B.bg[2],
                                          coverage + Tr[p] * B.bg[3]);
                 if (depth)
@@ -302,12 +303,12 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         }
 
         // ---- the pixels' colour, the loss (the view's mean L2 over its pixels and r g b) and its gradient
-        float sd[2], dC[2][3];
+        Px<2> sd, dR, dG, dB;
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            dC[p][0] = dC[p][1] = dC[p][2] = 0.0f;
-            if (px < V.width && py[p] < V.height) {
-                const uint32_t at = V.pixelBase + py[p] * V.width + px;
+            dR.v[p] = dG.v[p] = dB.v[p] = 0.0f;
+            if (px[p] < V.width && py < V.height) {
+                const uint32_t at = V.pixelBase + py * V.width + px[p];
                 const float coverage = 1.0f - Tr[p];
                 const float4 c = make_float4(r[p] + Tr[p] * B.bg[0], g[p] + Tr[p] * B.bg[1],
                                              bl[p] + Tr[p] * B.bg[2], coverage + Tr[p] * B.bg[3]);
@@ -316,16 +317,20 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                             eb = c.z - target[(size_t)at * 3 + 2];
                 lossSum += (er * er + eg * eg + eb * eb) * V.lossScale;
                 const float k2 = 2.0f * V.lossScale;
-                dC[p][0] = k2 * er;
-                dC[p][1] = k2 * eg;
-                dC[p][2] = k2 * eb;
+                dR.v[p] = k2 * er;
+                dG.v[p] = k2 * eg;
+                dB.v[p] = k2 * eb;
             }
-            sd[p] = (B.bg[0] * dC[p][0] + B.bg[1] * dC[p][1]) + B.bg[2] * dC[p][2];   // S.dC, S the colour behind
+            sd.v[p] = (B.bg[0] * dR.v[p] + B.bg[1] * dG.v[p]) + B.bg[2] * dB.v[p];   // S.dC, S the colour behind
         }
 
         // ---- adjoint: each warp on its own, over the records its box blended, last first
         // (the forward's live bits), gathered 32 at a time into the warp's own slots; no
         // block barrier, no staging and no box tests
+        __syncthreads();   // the block's warps are done with the staged records, whose memory the adjoint takes
+        Adjoint& sA = reinterpret_cast<Adjoint*>(sRaw)[warp];
+        const Px<2> xc{{pxc[0], pxc[1]}}, yc = both<2>(pyc);
+        Px<2> light{{Tr[0], Tr[1]}};   // the pixels' transmittance, from the last record back
         const uint32_t warpLast = __reduce_max_sync(0xFFFFFFFFu, max(last[0], last[1]));
         const uint32_t nChunks = (warpLast + 31u) >> 5;
         const uint32_t* liveOf = live + ((size_t)(range.x >> 5) + tile) * kBoxes + span * (kAcross * kAcross) + warp;
@@ -344,25 +349,10 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
             const uint32_t excl = incl - n;
             for (uint32_t r0 = 0; r0 < total; r0 += 32) {
                 // the records of ranks r0 .. r0 + 31 (ranked last first) into the warp's slots:
-                // lane q takes rank r0 + q. Its chunk is the last lane c whose exclusive count
-                // is at most the rank (a search over the lanes' counts); in that chunk's word,
-                // the record is the set bit of the remaining rank, counted down from bit 31 (a
-                // search over the word's halves, quarters, ...). No lane walks bits one by one.
+                // lane q takes rank r0 + q
                 const uint32_t want = r0 + lane;
-                uint32_t c = 0;
-#pragma unroll
-                for (uint32_t step = 16; step; step >>= 1)
-                    if (__shfl_sync(0xFFFFFFFFu, excl, c + step) <= want) c += step;
-                const uint32_t wc = __shfl_sync(0xFFFFFFFFu, word, c);
-                uint32_t rem = want - __shfl_sync(0xFFFFFFFFu, excl, c), bit = 31;
-#pragma unroll
-                for (uint32_t step = 16; step; step >>= 1) {
-                    const uint32_t below = __popc((wc >> (bit - step + 1u)) & ((1u << step) - 1u));
-                    if (below <= rem) {
-                        rem -= below;
-                        bit -= step;
-                    }
-                }
+                uint32_t c, bit;
+                liveRecord(word, excl, want, c, bit);
                 const uint32_t cnt = min(32u, total - r0);   // lane < cnt exactly when want < total
                 if (lane < cnt) {
                     const uint32_t rel = (uint32_t)(hi - (int32_t)c) * 32u + bit;
@@ -371,79 +361,102 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                     const float4 sc = recs[at + 0];
                     const float4 k = recs[at + 1];
                     const float4 rgb = recs[at + 2];
-                    sWarpCentre[warp][lane] =
-                        make_float4(sc.x, sc.y, __uint_as_float(rel), __uint_as_float((uint32_t)(recBase + gs)));
-                    const float lgo = log2Of(k.w);
-                    sWarpConic[warp][lane] = make_float4(k.x * kScale, k.y, k.z * kScale, lgo);
-                    sWarpColour[warp][lane] = make_float4(rgb.x, rgb.y, rgb.z, blendFloor(kScale * sc.w, lgo));
-                }
-                __syncwarp();
-                for (uint32_t q = 0; q < cnt; ++q) {
-                    if constexpr (kCount) ++adjVisits;
-                    const float4 ce = sWarpCentre[warp][q];
-                    const uint32_t rel = __float_as_uint(ce.z);
-                    const float4 k = sWarpConic[warp][q];
-                    const float4 c = sWarpColour[warp][q];
-                    const float dx = pxc - ce.x;
-                    // the sums start at -0, which adding leaves any value as it is (+0 would
-                    // turn a -0 term into +0): the first pixel's terms are taken as they come
-                    float gv[kWords];
-#pragma unroll
-                    for (int e = 0; e < (int)kWords; ++e) gv[e] = -0.0f;
-                    // as the forward, without branching: a pixel past its last contributor or
-                    // that does not blend the record takes alpha 0 (T unchanged, no terms)
+                    const float lgo = log2Of(k.w), ca = k.x * kScale, fs = k.z * kScale;
+                    Gathered& G = sA.records[lane];
 #pragma unroll
                     for (int p = 0; p < 2; ++p) {
-                        const float dy = pyc[p] - ce.y;
-                        const float t = __fmaf_rn(k.y, dy, dx);
-                        const float e = __fmaf_rn(k.x * t, t, __fmaf_rn(k.z * dy, dy, k.w));
-                        const float raw = fastExp2(e);
-                        const float a0 = fminf(0.99f, raw);
-                        const bool on = rel < last[p] && e >= c.w;
-                        if constexpr (kCount) { adjVisited += rel < last[p] ? 1u : 0u; adjLive += on ? 1u : 0u; }
-                        const float alpha = on ? a0 : 0.0f;
-                        const float inv = fastRcp(1.0f - alpha);
-                        const float Tb = Tr[p] * inv;
-                        const float w = Tb * alpha;
-                        gv[6] = __fmaf_rn(w, dC[p][0], gv[6]);
-                        gv[7] = __fmaf_rn(w, dC[p][1], gv[7]);
-                        gv[8] = __fmaf_rn(w, dC[p][2], gv[8]);
-                        const float cd = (c.x * dC[p][0] + c.y * dC[p][1]) + c.z * dC[p][2];
+                        G.nx[p] = -sc.x; G.ny[p] = -sc.y;
+                        G.ca[p] = ca; G.fr[p] = k.y; G.fs[p] = fs; G.lgo[p] = lgo;
+                        G.r[p] = rgb.x; G.g[p] = rgb.y; G.bl[p] = rgb.z;
+                    }
+                    G.least = blendFloor(kScale * sc.w, lgo);
+                    G.rel = rel;
+                    sA.rec[lane] = (uint32_t)(recBase + gs);
+                }
+                __syncwarp();
+                for (uint32_t q0 = 0; q0 < cnt; q0 += kSumRecords) {
+                    const uint32_t batch = min(kSumRecords, cnt - q0);
+                    float* column = sA.sums + lane;
+                    for (uint32_t q = q0; q < q0 + batch; ++q, column += kSumWords * kColumnStride) {
+                        if constexpr (kCount) { ++adjVisits; ++adjSummed; }
+                        const Gathered& G = sA.records[q];
+                        auto pair = [](const float (&v)[2]) { return Px<2>{{v[0], v[1]}}; };
+                        const Px<2> dy = yc + pair(G.ny);
+                        const Px<2> t = fused(pair(G.fr), dy, xc + pair(G.nx));
+                        const Px<2> e = fused(pair(G.ca) * t, t, fused(pair(G.fs) * dy, dy, pair(G.lgo)));
+                        Px<2> alpha, raw, inv;
+                        // as the forward, without branching: a pixel past its last contributor or
+                        // that does not blend the record takes alpha 0 (T unchanged, no terms)
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) {
+                            raw.v[p] = fastExp2(e.v[p]);
+                            const float a0 = fminf(0.99f, raw.v[p]);
+                            const bool on = G.rel < last[p] && e.v[p] >= G.least;
+                            if constexpr (kCount) { adjVisited += G.rel < last[p] ? 1u : 0u; adjLive += on ? 1u : 0u; }
+                            alpha.v[p] = on ? a0 : 0.0f;
+                        }
+                        const Px<2> om = fused(alpha, both<2>(-1.0f), both<2>(1.0f));
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) inv.v[p] = fastRcp(om.v[p]);
+                        light = light * inv;
+                        const Px<2> w = light * alpha;
+                        const Px<2> cd = fused(pair(G.bl), dB, fused(pair(G.g), dG, pair(G.r) * dR));
                         // alpha dL/dalpha where alpha is not clamped (dL/dalpha = T before it
                         // times (c - S).dC): the opacity times dL/dopacity, and -2 dL/dpower
-                        const float u = cd - sd[p];
-                        const float dP = on && raw < 0.99f && k.w <= 0.0f ? w * u : 0.0f;
-                        sd[p] = __fmaf_rn(alpha, u, sd[p]);
-                        Tr[p] = Tb;
-                        gv[5] += dP;
-                        const float dPt = dP * t, dPy = dP * dy;
-                        gv[0] += dPt;
-                        gv[1] += dPy;
-                        gv[2] = __fmaf_rn(dPt, t, gv[2]);
-                        gv[3] = __fmaf_rn(dPt, dy, gv[3]);
-                        gv[4] = __fmaf_rn(dPy, dy, gv[4]);
+                        const Px<2> u = fused(sd, both<2>(-1.0f), cd);
+                        Px<2> dP = w * u;
+                        sd = fused(alpha, u, sd);
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) dP.v[p] = raw.v[p] < 0.99f ? dP.v[p] : 0.0f;
+                        // the lane's two pixels: dy is theirs both
+                        const Px<2> dPt = dP * t, dPtt = dPt * t, wr = w * dR, wg = w * dG, wb = w * dB;
+                        const float m0 = dP.v[0] + dP.v[1], mt = dPt.v[0] + dPt.v[1], my = dy.v[0] * m0;
+                        column[0 * kColumnStride] = mt;
+                        column[1 * kColumnStride] = my;
+                        column[2 * kColumnStride] = dPtt.v[0] + dPtt.v[1];
+                        column[3 * kColumnStride] = dy.v[0] * mt;
+                        column[4 * kColumnStride] = dy.v[0] * my;
+                        column[5 * kColumnStride] = m0;
+                        column[6 * kColumnStride] = wr.v[0] + wr.v[1];
+                        column[7 * kColumnStride] = wg.v[0] + wg.v[1];
+                        column[8 * kColumnStride] = wb.v[0] + wb.v[1];
                     }
-                    // no test that some lane is live: a gathered record's forward live bit says a
-                    // pixel of this box blended it, and the adjoint decides that pixel the same way
-                    // (a record with no live lane would only add zeros, which are not stored)
-                    if constexpr (kCount) ++adjSummed;
-                    // the warp's sums, however few lanes are live, added by nine lanes at once
-                    // into the record's words in global memory (reductions, not read back):
-                    // the five moments, dL/dalpha and dL/dcolour, which the projection's
-                    // adjoint turns into centre and conic gradients (linear in the moments,
-                    // so sums from every box, tile and batch add up)
-                    const float val = warpSum9(gv, lane);
-                    const uint32_t slot = (lane & 3u) == 0u ? lane >> 2 : lane == 2u ? 8u : kWords;
-                    if (slot < kWords && val != 0.0f)
-                        atomicAdd(grads + (size_t)__float_as_uint(ce.w) * kGradWords + slot, val);
+                    __syncwarp();
+                    // lane k sums column k and adds it into its record's words in global memory (a
+                    // reduction, not read back): the five moments, dL/dalpha and dL/dcolour, which the
+                    // projection's adjoint turns into centre and conic gradients (linear in the
+                    // moments, so sums from every box, tile and batch add up). A gathered record's
+                    // forward live bit says a pixel of this box blended it; sums that come to zero
+                    // (all its pixels clamped) are not added.
+                    if (lane < batch * kSumWords) {
+                        float val = columnSum(sA.sums + lane * kColumnStride);
+                        // an opacity over 1 takes no geometry or opacity gradient (its kernel has no moments)
+                        if (sumWord < 6 && sA.records[q0 + sumRecord].lgo[0] > 0.0f) val = 0.0f;
+                        if (val != 0.0f)
+                            atomicAdd(grads + (size_t)sA.rec[q0 + sumRecord] * kGradWords + sumWord, val);
+                    }
+                    __syncwarp();   // the next records' values overwrite the columns
                 }
                 __syncwarp();   // the next round's gathers overwrite the slots
             }
         }
     }
+    if constexpr (kTrain) {
+        // the loss: the threads' shares summed in 64 bits (a warp, the batch's word, and the last
+        // block to finish writes it): thousands of 32-bit atomic additions into one word each
+        // rounded it, which cost it up to 2e-6 of its value
+        double sum = (double)lossSum;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lossSum += __shfl_xor_sync(0xFFFFFFFFu, lossSum, o);
-    if (kTrain && lane == 0 && lossSum != 0.0f) atomicAdd(loss, lossSum);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        double* total = reinterpret_cast<double*>(words + kBatchLoss);
+        if (lane == 0 && sum != 0.0) atomicAdd(total, sum);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0 && atomicAdd(&words[kBatchLossBlocks], 1u) == gridDim.x - 1) {
+            __threadfence();
+            *loss = (float)*reinterpret_cast<volatile double*>(total);
+        }
+    }
     if constexpr (!kCount) return;
     // the work counts: a warp's sums, one atomic each
     const uint32_t visits = lane == 0;   // a warp's visits, once

@@ -66,6 +66,8 @@ enum BatchWord : uint32_t {
     kBatchAdjVisits = 34,    // 64-bit (34, 35): (warp, record) visits of the adjoint walk
     kBatchAdjSummed = 36,    // 64-bit (36, 37): adjoint visits with a live lane, whose sums the warp reduced
     kBatchStaged = 38,       // 64-bit (38, 39): records a block staged (loaded and box-tested) for the forward
+    kBatchLoss = 40,         // a step's loss as a double (40, 41), and the blend blocks that have added their
+    kBatchLossBlocks = 42,   // share to it: the last one writes the loss
     kBatchWords = 48,
 };
 
@@ -168,8 +170,7 @@ inline size_t liveWords(uint64_t capacity, uint32_t totalTiles, uint32_t tile) {
 
 // A training step's blends over every view's tiles, in one kernel: the forward
 // blend into `colour`; the loss, each view's mean L2 against `target` (float3 a
-// pixel) over its pixels and r g b, summed over views into *loss (which the
-// caller zeroes); and the adjoint, dL/d(record) for every (view, Gaussian)
+// pixel) over its pixels and r g b, summed over views into *loss; and the adjoint, dL/d(record) for every (view, Gaussian)
 // record, added into `grads` (which start at zero). A null `target`: the
 // forward blend alone, colour and (when `depth` is given) depth.
 cudaError_t launchBatchBlendStep(const BatchConst& B, const BlendLaunch& L, cudaStream_t stream, float4* colour,
