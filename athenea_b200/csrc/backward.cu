@@ -55,7 +55,7 @@ __device__ __forceinline__ float reciprocal(float x) {
 template <int kPx, bool kDepth>
 __global__ void __launch_bounds__(Box<kPx>::kThreads)
     blendBackwardKernel(const FrameConst F, uint32_t pairs, uint32_t slots, const uint2* __restrict__ ranges,
-                        const uint32_t* __restrict__ pairValues, const float4* __restrict__ recs,
+                        const uint64_t* __restrict__ sorted, const float4* __restrict__ recs,
                         const TrainingState training, const float4* __restrict__ dLdColour,
                         const float* __restrict__ dLdDepth, const float* __restrict__ depthOut,
                         float* __restrict__ grads, uint32_t* __restrict__ status) {
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
             const uint32_t count = min(32u, total - r0);
             if (lane < count) {
                 const uint32_t rel = (uint32_t)(hi - (int32_t)chunk) * 32u + bit;
-                uint32_t s = pairValues[range.x + rel];
+                uint32_t s = (uint32_t)sorted[range.x + rel];
                 if (s >= slots) {
                     atomicOr(status, kStatusIndexRange);
                     s = 0;
@@ -255,14 +255,14 @@ __global__ void __launch_bounds__(256)
 }   // namespace
 
 cudaError_t launchBlendBackward(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
-                                const uint32_t* pairValues, const float4* recs, const TrainingState& training,
+                                const uint64_t* sorted, const float4* recs, const TrainingState& training,
                                 const float4* dLdColour, const float* dLdDepth, const float* depthOut, float* grads,
                                 uint32_t* status, cudaStream_t stream) {
     const uint32_t tiles = F.tilesX * F.tilesY;
     if (tiles == 0) return cudaSuccess;
     const bool d = dLdDepth != nullptr && F.depthMode == 0;
 #define ATH_BACKWARD(P_, D_)                                                                                   \
-    blendBackwardKernel<P_, D_><<<tiles, Box<P_>::kThreads, 0, stream>>>(F, pairs, slots, ranges, pairValues, recs, \
+    blendBackwardKernel<P_, D_><<<tiles, Box<P_>::kThreads, 0, stream>>>(F, pairs, slots, ranges, sorted, recs, \
                                                                         training, dLdColour, dLdDepth, depthOut, grads, \
                                                                         status)
     if (training.onePixel) {

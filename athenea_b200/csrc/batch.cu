@@ -1043,7 +1043,7 @@ cudaError_t enqueueStep(ath_batch* b, const ath_mixed_params& P, const float* ta
     err = launchSortDevice(keys, B.wide ? vals : nullptr, (uint32_t)b->capacity, words + kBatchPairsLo,
                            words + kBatchEpoch, B.slotBits, bits, static_cast<uint32_t*>(b->sortHist.ptr),
                            static_cast<uint64_t*>(b->sortFlags.ptr), words + kBatchSortTickets, words + kBatchStatus,
-                           stream);
+                           stream, kClearHistograms);   // the step's first kernel clears the tickets
     const uint32_t sorted = sortResultIndex(2, bits);
     mark(2);
     b->lastSorted = sorted;
@@ -1216,13 +1216,13 @@ ath_status sizePairs(ath_batch* b, const ath_mixed_params& P, cudaStream_t strea
         b->capacity = room;
     }
     const uint32_t bits = b->depthBits + b->tileBits;
-    err = b->sortFlags.reserve(sortFlagWords((uint32_t)b->capacity, bits) * 8);
+    err = b->sortFlags.reserve(sortFlagWords((uint32_t)b->capacity, bits, b->planWide) * 8);
     if (err != cudaSuccess) return failCuda(err, "reserving the sort's look-back words");
     // the blends' live bits (written by the forward before the adjoint reads them; no clearing)
     err = b->live.reserve(liveWords(b->capacity, b->totalTiles, b->tile) * sizeof(uint32_t));
     if (err != cudaSuccess) return failCuda(err, "reserving the blends' live bits");
     // the look-back words carry epochs: start them all at "not ready"
-    err = cudaMemsetAsync(b->sortFlags.ptr, 0, sortFlagWords((uint32_t)b->capacity, bits) * 8, stream);
+    err = cudaMemsetAsync(b->sortFlags.ptr, 0, sortFlagWords((uint32_t)b->capacity, bits, b->planWide) * 8, stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(b->words.ptr, 0, kBatchWords * sizeof(uint32_t), stream);
     if (err == cudaSuccess) err = cudaMemsetAsync(b->projFlags.ptr, 0, b->projFlags.bytes, stream);
     if (err != cudaSuccess) return failCuda(err, "clearing the batch's look-back words");
@@ -1253,7 +1253,7 @@ extern "C" ath_status ath_batch_create(ath_batch** out) {
     if (!b) return fail(ATH_E_OUT_OF_MEMORY, "ath_batch_create: host allocation failed");
     cudaError_t err = cudaGetDevice(&b->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
-    if (err == cudaSuccess) err = sortPrepare();
+    if (err == cudaSuccess) err = sortPrepare(kSortsKeys | kSortsPairs);
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&b->captureStream, cudaStreamNonBlocking);
     if (err != cudaSuccess) {
         delete b;

@@ -179,7 +179,7 @@ struct CryptoList {
 template <int kPx, bool kTrain, bool kContribution, bool kUnder, bool kMatte>
 __global__ void __launch_bounds__(Box<kPx>::kThreads)
     blendKernel(const FrameConst F, uint32_t pairs, uint32_t slots, const uint2* __restrict__ ranges,
-                const uint32_t* __restrict__ pairValues, const float4* __restrict__ recs, float4* __restrict__ colour,
+                const uint64_t* __restrict__ sorted, const float4* __restrict__ recs, float4* __restrict__ colour,
                 float* __restrict__ depth, float4* __restrict__ position, float* __restrict__ finalT,
                 uint32_t* __restrict__ lastContrib, uint32_t* __restrict__ live, uint32_t* __restrict__ status,
                 Contribution contrib, Under under, Matte matte) {
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
     screen = conic = tint = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     auto load = [&](uint32_t first) {
         if (first + lane >= range.y) return;
-        slot = pairValues[first + lane];
+        slot = (uint32_t)sorted[first + lane];
         if (slot >= slots) {
             atomicOr(status, kStatusIndexRange);
             slot = 0;
@@ -438,7 +438,7 @@ bool trainingOnePixel(const FrameConst& F, int sms, const Contribution& contrib,
 size_t trainingLiveWords(const FrameConst& F, uint64_t pairs) { return frameLiveWords(pairs, F.tilesX * F.tilesY); }
 
 cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
-                        const uint32_t* pairValues, const float4* recs, float4* colour, float* depth, float4* position,
+                        const uint64_t* sorted, const float4* recs, float4* colour, float* depth, float4* position,
                         const TrainingState* training, int sms, uint32_t* status, cudaStream_t stream,
                         const Contribution& contrib, const Under& under, const Matte& matte) {
     const uint32_t tiles = F.tilesX * F.tilesY;
@@ -446,7 +446,7 @@ cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, con
     const TrainingState keep = training ? *training : TrainingState{};
 #define ATH_BLEND(P_, T_, C_, U_, M_)                                                                              \
     blendKernel<P_, T_, C_, U_, M_><<<tiles, Box<P_>::kThreads, 0, stream>>>(                                      \
-        F, pairs, slots, ranges, pairValues, recs, colour, depth, position, keep.finalT, keep.lastContrib, keep.live, \
+        F, pairs, slots, ranges, sorted, recs, colour, depth, position, keep.finalT, keep.lastContrib, keep.live, \
         status, contrib, under, matte)
     const bool c = contrib.mode != 0u, u = under.depth != nullptr,
                m = matte.out != nullptr || matte.lifted != nullptr || matte.trace != nullptr;

@@ -26,11 +26,14 @@ struct ath_raster {
     int sms = 148;
     bool tight = false;   // after release_scratch: grow to the need exactly
     uint32_t slotCapacity = 0, pairCapacity = 0, tileCapacity = 0, instanceCapacity = 0;
-    DeviceBuffer recs, rects, keys, offsets, projectFlags, instances;
-    DeviceBuffer pairKeys[2], pairVals[2], sortHist, sortFlags, ranges;
-    DeviceBuffer words;          // kFrameWords
+    DeviceBuffer recs, rects, masks, keys, offsets, instances;
+    DeviceBuffer depthKeys[2], depthSlots[2];   // the depth sort's
+    DeviceBuffer pairs[2], sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
+    DeviceBuffer inspectSplats;   // ath_raster_frame_buffers' slots, a pair each (its keys: the spare pair buffer)
+    DeviceBuffer zeroed;         // what a frame starts at zero, cleared at once (FrameZeroed): its words first
+    uint2* ranges = nullptr;     // the last frame's, there
     PinnedBuffer wordsHost;      // kFrameWords: a frame that waits (its handle's first, or timed) reads them here
-    PinnedBuffer instanceStage;  // InstanceConst staging for the H2D copy
+    std::vector<InstanceConst> instanceStage;   // pageable: the copy to the device takes it before it returns
     // The last frame's words, copied at its end behind `frameDone` (ath_raster_check,
     // and the next frame's capacity, read them once that event has passed).
     PinnedBuffer statusHost;
@@ -64,7 +67,7 @@ struct ath_raster {
 
 struct ath_sorter {
     int device = 0;
-    DeviceBuffer hist, flags, words;   // words: 8 pass tickets, then the status, kept until ath_sorter_check
+    DeviceBuffer scratch, words;       // scratch: tickets, histograms, look-back words; words: the status, kept until ath_sorter_check
     PinnedBuffer wordsHost;
     cudaEvent_t done = nullptr;        // after the last sort
     bool recorded = false;
@@ -306,8 +309,8 @@ extern "C" ath_status ath_raster_create(ath_raster** out) {
     if (!r) return fail(ATH_E_OUT_OF_MEMORY, "ath_raster_create: host allocation failed");
     cudaError_t err = cudaGetDevice(&r->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, r->device);
-    if (err == cudaSuccess) err = sortPrepare();
-    if (err == cudaSuccess) err = r->words.reserve(kFrameWords * sizeof(uint32_t));
+    if (err == cudaSuccess) err = sortPrepare(kSortsKeys | kSortsDepths);
+    if (err == cudaSuccess) err = r->zeroed.reserve(kFrameWords * sizeof(uint32_t));
     if (err == cudaSuccess) err = r->wordsHost.reserve(kFrameWords * sizeof(uint32_t));
     if (err == cudaSuccess) err = r->statusHost.reserve(kFrameWords * sizeof(uint32_t));
     for (int k = 0; k < ath_raster::kCountDepth && err == cudaSuccess; ++k) {
@@ -315,7 +318,7 @@ extern "C" ath_status ath_raster_create(ath_raster** out) {
         if (err == cudaSuccess) err = cudaEventCreateWithFlags(&r->countDone[k], cudaEventDisableTiming);
     }
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&r->frameDone, cudaEventDisableTiming);
-    if (err == cudaSuccess) err = cudaMemset(r->words.ptr, 0, kFrameWords * sizeof(uint32_t));
+    if (err == cudaSuccess) err = cudaMemset(r->zeroed.ptr, 0, kFrameWords * sizeof(uint32_t));
     for (int k = 0; k < 8 && err == cudaSuccess; ++k) err = cudaEventCreate(&r->marks[k]);
     if (err != cudaSuccess) {
         ath_status s = failCuda(err, "ath_raster_create");
@@ -343,13 +346,15 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     cudaDeviceSynchronize();
     r->tight = true;
     r->slotCapacity = r->pairCapacity = r->tileCapacity = r->instanceCapacity = 0;
-    for (DeviceBuffer* b : {&r->recs, &r->rects, &r->keys, &r->offsets, &r->projectFlags, &r->instances,
-                            &r->pairKeys[0], &r->pairKeys[1], &r->pairVals[0], &r->pairVals[1], &r->sortHist,
-                            &r->sortFlags, &r->ranges, &r->finalT, &r->lastContrib, &r->live, &r->grads})
+    for (DeviceBuffer* b : {&r->recs, &r->rects, &r->masks, &r->keys, &r->offsets, &r->instances,
+                            &r->depthKeys[0], &r->depthKeys[1], &r->depthSlots[0], &r->depthSlots[1], &r->pairs[0],
+                            &r->pairs[1], &r->inspectSplats, &r->sortScratch, &r->zeroed, &r->finalT, &r->lastContrib, &r->live, &r->grads})
         b->release();
     r->trainingValid = false;
     r->frameRecorded = false;
-    r->instanceStage.release();
+    r->ranges = nullptr;
+    r->instanceStage.clear();
+    r->instanceStage.shrink_to_fit();
     return ATH_OK;
 }
 
@@ -410,28 +415,45 @@ ath_status reserveSlots(ath_raster* r, uint32_t slots) {   // reserveSplats (Til
     if (err == cudaSuccess) err = r->rects.reserve((size_t)n * 8);
     if (err == cudaSuccess) err = r->keys.reserve((size_t)n * 4);
     if (err == cudaSuccess) err = r->offsets.reserve((size_t)n * 4);
-    if (err == cudaSuccess) err = r->projectFlags.reserve((size_t)projectBlocks(n) * 8);
+    if (err == cudaSuccess) err = r->masks.reserve((size_t)n * 8);
+    for (int k = 0; k < 2; ++k) {
+        if (err == cudaSuccess) err = r->depthKeys[k].reserve((size_t)n * 4);
+        if (err == cudaSuccess) err = r->depthSlots[k].reserve((size_t)n * 4);
+    }
     if (err != cudaSuccess) return failCuda(err, "reserving the splats' scratch");
     r->slotCapacity = n;
     return ATH_OK;
 }
 
+const size_t kSortHistBytes = sortHistWords() * sizeof(uint32_t);
+
 ath_status reservePairs(ath_raster* r, uint32_t pairs, uint32_t bits) {   // reservePairs (:228-247)
-    if (pairs > r->pairCapacity || !r->pairKeys[0].bytes) {
+    if (pairs > r->pairCapacity || !r->pairs[0].bytes) {
         const uint32_t n = r->tight ? pairs : grow(r->pairCapacity, pairs);
         cudaError_t err = cudaSuccess;
-        for (int k = 0; k < 2 && err == cudaSuccess; ++k) {
-            err = r->pairKeys[k].reserve((size_t)n * 8);
-            if (err == cudaSuccess) err = r->pairVals[k].reserve((size_t)n * 4);
-        }
+        for (int k = 0; k < 2 && err == cudaSuccess; ++k) err = r->pairs[k].reserve((size_t)n * 8);
         if (err != cudaSuccess) return failCuda(err, "reserving the pairs");
         r->pairCapacity = n;
     }
-    cudaError_t err = r->sortFlags.reserve(sortFlagWords(std::max(r->pairCapacity, pairs), std::max(bits, 8u)) * 8);
-    if (err == cudaSuccess) err = r->sortHist.reserve(sortHistWords() * sizeof(uint32_t));
-    if (err != cudaSuccess) return failCuda(err, "reserving the sort's scratch");
+    const size_t bytes = kSortHistBytes + sortFlagWords(r->pairCapacity, bits) * 8;
+    if (cudaError_t err = r->sortScratch.reserve(bytes); err != cudaSuccess)
+        return failCuda(err, "reserving the sort's scratch");
     return ATH_OK;
 }
+
+// What a frame of `slots` splats and `tiles` tiles starts at zero, one after another in
+// ath_raster::zeroed, so that one clearing serves them all.
+struct FrameZeroed {
+    size_t words = 0, projectFlags, emitFlags, depthHist, depthFlags, ranges, bytes;   // byte offsets
+    FrameZeroed(uint32_t slots, uint32_t tiles) {
+        projectFlags = (kFrameWords * sizeof(uint32_t) + 255) / 256 * 256;
+        emitFlags = projectFlags + (size_t)projectBlocks(std::max(slots, 1u)) * 8;
+        depthHist = emitFlags + (size_t)projectBlocks(std::max(slots, 1u)) * 8;
+        depthFlags = depthHist + kSortHistBytes;
+        ranges = depthFlags + sortFlagWords(slots, kDepthBits) * 8;
+        bytes = ranges + (size_t)tiles * 8;
+    }
+};
 
 }   // namespace
 
@@ -511,14 +533,15 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                      ath_frame_stats* stats, cudaStream_t stream, bool training, const ath_targets* under = nullptr) {
     const auto frameStart = std::chrono::steady_clock::now();
     const uint32_t tiles = F.tilesX * F.tilesY;
-    const uint32_t bits = 24 + F.tileBits;
+    const uint32_t bits = F.tileBits;   // the pairs sort by tile alone, their splats in depth order already
     ath_status st = reserveSlots(r, std::max(slots, 1u));
     if (st != ATH_OK) return st;
-    if (tiles > r->tileCapacity || !r->ranges.bytes) {
-        if (cudaError_t err = r->ranges.reserve((size_t)tiles * 8); err != cudaSuccess)
-            return failCuda(err, "reserving the tiles' ranges");
-        r->tileCapacity = tiles;
-    }
+    r->tileCapacity = std::max(r->tileCapacity, tiles);
+    if (cudaError_t err = r->zeroed.reserve(FrameZeroed(r->slotCapacity, r->tileCapacity).bytes); err != cudaSuccess)
+        return failCuda(err, "reserving the frame's words, ranges and look-back words");
+    const FrameZeroed zeroed(slots, tiles);
+    char* const zero = static_cast<char*>(r->zeroed.ptr);
+    uint2* const ranges = reinterpret_cast<uint2*>(zero + zeroed.ranges);
     if (training) {
         const size_t pixels = (size_t)F.width * F.height;
         cudaError_t err = r->finalT.reserve(pixels * 4);
@@ -531,25 +554,24 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
         if ((st = reservePairs(r, (uint32_t)std::min<uint64_t>(need + need / 7 + 4096, 0xFFFFFFFFull), bits)) != ATH_OK)
             return st;
     }
-    uint32_t* words = static_cast<uint32_t*>(r->words.ptr);
+    uint32_t* words = reinterpret_cast<uint32_t*>(zero + zeroed.words);
     uint32_t* wordsHost = static_cast<uint32_t*>(r->wordsHost.ptr);
     const bool timed = s.time_stages != 0;
-    const bool sizing = r->pairCapacity == 0 || !r->pairKeys[0].bytes;   // no capacity yet: read the total once
+    const bool sizing = r->pairCapacity == 0 || !r->pairs[0].bytes;   // no capacity yet: read the total once
     auto mark = [&](int k) { if (timed) cudaEventRecord(r->marks[k], stream); };
 
     // --- project, with the tiles-touched scan fused in --------------------
     mark(0);
-    cudaError_t err = cudaMemsetAsync(words, 0, kFrameWords * sizeof(uint32_t), stream);
-    if (err == cudaSuccess && slots)
-        err = cudaMemsetAsync(r->projectFlags.ptr, 0, (size_t)projectBlocks(slots) * 8, stream);
-    if (err == cudaSuccess && instanceCount)
+    cudaError_t err = cudaMemsetAsync(zero, 0, zeroed.bytes, stream);
+    if (err == cudaSuccess && instanceCount > 1)
         err = cudaMemcpyAsync(r->instances.ptr, staged, instanceCount * sizeof(InstanceConst), cudaMemcpyHostToDevice,
                               stream);
     if (err == cudaSuccess)
-        err = launchProject(F, static_cast<const InstanceConst*>(r->instances.ptr), instanceCount, slots, layout,
+        err = launchProject(F, staged[0], static_cast<const InstanceConst*>(r->instances.ptr), instanceCount, slots, layout,
                             s.count_splats != 0, static_cast<float4*>(r->recs.ptr), static_cast<uint2*>(r->rects.ptr),
-                            static_cast<uint32_t*>(r->keys.ptr), static_cast<uint32_t*>(r->offsets.ptr),
-                            static_cast<uint64_t*>(r->projectFlags.ptr), words, stream);
+                            static_cast<unsigned long long*>(r->masks.ptr), static_cast<uint32_t*>(r->keys.ptr),
+                            static_cast<uint32_t*>(r->offsets.ptr), reinterpret_cast<uint64_t*>(zero + zeroed.projectFlags),
+                            words, stream);
     mark(1);
     bool haveTotals = false;
     if (sizing && err == cudaSuccess) {
@@ -570,25 +592,34 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     if ((st = reservePairs(r, r->pairCapacity, bits)) != ATH_OK) return st;   // the sort's scratch for this frame's bits
     mark(2);
 
-    // --- emit, sort, ranges (the pair count on the device) ------------------
+    // --- depth sort, emit, tile sort, ranges (the pair count on the device) --
     const uint32_t capacity = r->pairCapacity;
     uint32_t* kept = words + kWordPairsKept;
-    uint64_t* keysBuf[2] = {static_cast<uint64_t*>(r->pairKeys[0].ptr), static_cast<uint64_t*>(r->pairKeys[1].ptr)};
-    uint32_t* valsBuf[2] = {static_cast<uint32_t*>(r->pairVals[0].ptr), static_cast<uint32_t*>(r->pairVals[1].ptr)};
-    err = launchEmit(F, slots, static_cast<const float4*>(r->recs.ptr), static_cast<const uint2*>(r->rects.ptr),
-                     static_cast<const uint32_t*>(r->keys.ptr), static_cast<const uint32_t*>(r->offsets.ptr), words,
-                     capacity, keysBuf[0], valsBuf[0], stream);
+    uint32_t* keys = static_cast<uint32_t*>(r->keys.ptr);
+    uint32_t* hist = static_cast<uint32_t*>(r->sortScratch.ptr);
+    uint64_t* flags = reinterpret_cast<uint64_t*>(static_cast<char*>(r->sortScratch.ptr) + kSortHistBytes);
+    uint32_t* depthKeys[2] = {static_cast<uint32_t*>(r->depthKeys[0].ptr), static_cast<uint32_t*>(r->depthKeys[1].ptr)};
+    uint32_t* depthSlots[2] = {static_cast<uint32_t*>(r->depthSlots[0].ptr),
+                               static_cast<uint32_t*>(r->depthSlots[1].ptr)};
+    uint64_t* pairs[2] = {static_cast<uint64_t*>(r->pairs[0].ptr), static_cast<uint64_t*>(r->pairs[1].ptr)};
+    err = launchSortDepths(keys, depthKeys, depthSlots, slots, reinterpret_cast<uint32_t*>(zero + zeroed.depthHist),
+                           reinterpret_cast<uint64_t*>(zero + zeroed.depthFlags), words + kWordDepthTickets,
+                           words + kWordSticky, stream);
     mark(3);
     if (err == cudaSuccess)
-        err = launchSortDevice(keysBuf, valsBuf, capacity, kept, nullptr, 0, bits, static_cast<uint32_t*>(r->sortHist.ptr),
-                               static_cast<uint64_t*>(r->sortFlags.ptr), words + kWordSortTickets, words + kWordSticky,
-                               stream);
-    const uint32_t sorted = sortPasses(bits) & 1u;
-    if (err == cudaSuccess) err = cudaMemsetAsync(r->ranges.ptr, 0, (size_t)tiles * 8, stream);
-    if (err == cudaSuccess)
-        err = launchRanges(capacity, kept, tiles, keysBuf[sorted], static_cast<uint2*>(r->ranges.ptr),
-                           words + kWordSticky, stream);
+        err = launchEmit(F, slots, depthSlots[0], static_cast<const float4*>(r->recs.ptr),
+                         static_cast<const uint2*>(r->rects.ptr), static_cast<const unsigned long long*>(r->masks.ptr),
+                         keys, static_cast<const uint32_t*>(r->offsets.ptr),
+                         reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
     mark(4);
+    if (err == cudaSuccess)
+        err = cudaMemsetAsync(hist, 0, kSortHistBytes + sortFlagWords(capacity, bits) * 8, stream);
+    if (err == cudaSuccess)
+        err = launchSortDevice(pairs, nullptr, capacity, kept, nullptr, 32, bits, hist, flags, words + kWordSortTickets,
+                               words + kWordSticky, stream, kClearNone);
+    const uint32_t sorted = sortPasses(bits) & 1u;
+    if (err == cudaSuccess) err = launchRanges(capacity, kept, tiles, pairs[sorted], ranges, words + kWordSticky, stream);
+    mark(5);
     // --- blend ---------------------------------------------------------------
     const Contribution contrib{s.contribution_mode, s.contribution, s.final_colour, s.lift_mask};
     const Matte matte{s.crypto_ids, s.crypto, under ? s.under_crypto : nullptr, s.matte_lift, s.matte,
@@ -601,12 +632,12 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
         keep = trainingState(r);
     }
     if (err == cudaSuccess)
-        err = launchBlend(F, capacity, slots, static_cast<const uint2*>(r->ranges.ptr), valsBuf[sorted],
+        err = launchBlend(F, capacity, slots, ranges, pairs[sorted],
                           static_cast<const float4*>(r->recs.ptr), reinterpret_cast<float4*>(targets->colour),
                           targets->depth, reinterpret_cast<float4*>(targets->position), training ? &keep : nullptr,
                           r->sms, words + kWordSticky, stream, contrib,
                           under ? Under{under->colour, under->depth} : Under{}, matte);
-    mark(5);
+    mark(6);
     // --- the frame's words: its counters into the ring; its status behind an event
     // (last, so that a wait for the frame covers both)
     if (err == cudaSuccess && s.count_splats) {
@@ -626,6 +657,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     r->lastTiles = tiles;
     r->lastSorted = sorted;
     r->lastFrame = F;
+    r->ranges = ranges;
 
     ath_frame_stats out{};
     out.splats = slots;
@@ -647,9 +679,10 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
         };
         out.project_ms = ms(0, 1);
         out.counts_ms = ms(1, 2);
-        out.emit_ms = ms(2, 3);
-        out.tile_sort_ms = ms(3, 4);
-        out.blend_ms = ms(4, 5);
+        out.depth_sort_ms = ms(2, 3);
+        out.emit_ms = ms(3, 4);
+        out.tile_sort_ms = ms(4, 5);
+        out.blend_ms = ms(5, 6);
     }
     out.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - frameStart).count();
     if (stats) *stats = out;
@@ -660,10 +693,10 @@ ath_status reserveInstances(ath_raster* r, uint32_t instanceCount) {
     if (instanceCount > r->instanceCapacity || !r->instances.bytes) {
         const uint32_t n = std::max(instanceCount, 4u);
         cudaError_t err = r->instances.reserve((size_t)n * sizeof(InstanceConst));
-        if (err == cudaSuccess) err = r->instanceStage.reserve((size_t)n * sizeof(InstanceConst));
         if (err != cudaSuccess) return failCuda(err, "reserving the instance table");
         r->instanceCapacity = n;
     }
+    r->instanceStage.resize(std::max(instanceCount, 1u));
     return ATH_OK;
 }
 
@@ -693,7 +726,7 @@ ath_status renderPacked(ath_raster* r, const ath_projection* projection, const a
     if (total > 0xFFFFFFFFull) return fail(ATH_E_UNSUPPORTED, "more than 2^32 splats in one frame");
     DeviceGuard guard(r->device);
     if ((st = reserveInstances(r, instanceCount)) != ATH_OK) return st;
-    InstanceConst* staged = static_cast<InstanceConst*>(r->instanceStage.ptr);
+    InstanceConst* staged = r->instanceStage.data();
     uint32_t base = 0;
     for (uint32_t k = 0; k < instanceCount; ++k) {
         staged[k] = instanceConstFor(*projection, s, instances[k], base);
@@ -764,7 +797,7 @@ extern "C" ath_status ath_raster_render_params(ath_raster* r, const ath_projecti
             return fail(ATH_E_INVALID_ARGUMENT, "ath_raster_render_params: means, scales and quats must be 16-byte aligned");
     DeviceGuard guard(r->device);
     if ((st = reserveInstances(r, 1)) != ATH_OK) return st;
-    InstanceConst* staged = static_cast<InstanceConst*>(r->instanceStage.ptr);
+    InstanceConst* staged = r->instanceStage.data();
     staged[0] = instanceConstForParams(*projection, s, P);
     r->trainingValid = false;
     st = drawFrame(r, frameConstFor(*projection, s), staged, 1, P.count, kLayoutParams, s, targets, stats,
@@ -789,10 +822,10 @@ extern "C" ath_status ath_raster_backward(ath_raster* r, const float* dlDcolour,
     const uint32_t slots = r->lastSlots;
     cudaError_t err = r->grads.reserve((size_t)std::max(slots, 1u) * kGradWords * sizeof(float));
     if (err == cudaSuccess) err = cudaMemsetAsync(r->grads.ptr, 0, (size_t)slots * kGradWords * sizeof(float), stream);
-    uint32_t* words = static_cast<uint32_t*>(r->words.ptr);
+    uint32_t* words = static_cast<uint32_t*>(r->zeroed.ptr);
     if (err == cudaSuccess)
-        err = launchBlendBackward(F, r->pairCapacity, slots, static_cast<const uint2*>(r->ranges.ptr),
-                                  static_cast<const uint32_t*>(r->pairVals[r->lastSorted].ptr),
+        err = launchBlendBackward(F, r->pairCapacity, slots, r->ranges,
+                                  static_cast<const uint64_t*>(r->pairs[r->lastSorted].ptr),
                                   static_cast<const float4*>(r->recs.ptr), trainingState(r),
                                   reinterpret_cast<const float4*>(dlDcolour), dlDdepth, r->trainingDepth,
                                   static_cast<float*>(r->grads.ptr), words + kWordSticky, stream);
@@ -843,16 +876,26 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     // inspection: waits for the frame, whose pair count only the device knew
     if (const cudaError_t err = cudaEventSynchronize(r->frameDone); err != cudaSuccess)
         return failCuda(err, "waiting for the frame");
+    // the pairs with their depth keys, in the pair buffer the sort left spare
+    const uint32_t pairs = static_cast<const uint32_t*>(r->statusHost.ptr)[kWordPairsKept];
+    cudaError_t err = r->inspectSplats.reserve((size_t)std::max(pairs, 1u) * 4);
+    uint64_t* pairKeys = static_cast<uint64_t*>(r->pairs[r->lastSorted ^ 1u].ptr);
+    if (err == cudaSuccess)
+        err = launchInspectPairs(static_cast<const uint64_t*>(r->pairs[r->lastSorted].ptr), pairs,
+                                 static_cast<const uint32_t*>(r->keys.ptr), r->lastSlots, pairKeys,
+                                 static_cast<uint32_t*>(r->inspectSplats.ptr), nullptr);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
+    if (err != cudaSuccess) return failCuda(err, "reading the frame's pairs");
     out->slots = r->lastSlots;
-    out->pairs = static_cast<const uint32_t*>(r->statusHost.ptr)[kWordPairsKept];
+    out->pairs = pairs;
     out->tiles = r->lastTiles;
     out->records = static_cast<const float*>(r->recs.ptr);
     out->rects = static_cast<const uint32_t*>(r->rects.ptr);
     out->keys = static_cast<const uint32_t*>(r->keys.ptr);
     out->offsets = static_cast<const uint32_t*>(r->offsets.ptr);
-    out->pair_keys = static_cast<const uint64_t*>(r->pairKeys[r->lastSorted].ptr);
-    out->pair_splats = static_cast<const uint32_t*>(r->pairVals[r->lastSorted].ptr);
-    out->ranges = static_cast<const uint32_t*>(r->ranges.ptr);
+    out->pair_keys = pairKeys;
+    out->pair_splats = static_cast<const uint32_t*>(r->inspectSplats.ptr);
+    out->ranges = reinterpret_cast<const uint32_t*>(r->ranges);
     out->grads = static_cast<const float*>(r->grads.ptr);
     return ATH_OK;
 }
@@ -864,8 +907,7 @@ extern "C" ath_status ath_sorter_create(ath_sorter** out) {
     ath_sorter* s = new (std::nothrow) ath_sorter();
     if (!s) return fail(ATH_E_OUT_OF_MEMORY, "ath_sorter_create: host allocation failed");
     cudaError_t err = cudaGetDevice(&s->device);
-    if (err == cudaSuccess) err = sortPrepare();
-    if (err == cudaSuccess) err = s->hist.reserve(sortHistWords() * sizeof(uint32_t));
+    if (err == cudaSuccess) err = sortPrepare(kSortsPairs);
     if (err == cudaSuccess) err = s->words.reserve(16 * sizeof(uint32_t));
     if (err == cudaSuccess) err = s->wordsHost.reserve(16 * sizeof(uint32_t));
     if (err == cudaSuccess) err = cudaMemset(s->words.ptr, 0, 16 * sizeof(uint32_t));
@@ -897,12 +939,18 @@ extern "C" ath_status ath_sorter_sort(ath_sorter* s, uint64_t* keys, uint32_t* v
     DeviceGuard guard(s->device);
     cudaStream_t stream = static_cast<cudaStream_t>(streamPtr);
     uint32_t* words = static_cast<uint32_t*>(s->words.ptr);
-    cudaError_t err = s->flags.reserve(sortFlagWords(count, keyBits) * 8);
+    constexpr size_t kTicketBytes = 64;
+    const size_t bytes = kTicketBytes + kSortHistBytes + sortFlagWords(count, keyBits, true) * 8;
+    cudaError_t err = s->scratch.reserve(bytes);
     if (err != cudaSuccess) return failCuda(err, "reserving the sort's look-back words");
+    char* scratch = static_cast<char*>(s->scratch.ptr);
+    err = cudaMemsetAsync(scratch, 0, bytes, stream);
+    if (err != cudaSuccess) return failCuda(err, "sorting");
     uint64_t* k[2] = {keys, scratchKeys};
     uint32_t* v[2] = {values, scratchValues};
-    err = launchSort(k, v, count, keyBits, static_cast<uint32_t*>(s->hist.ptr), static_cast<uint64_t*>(s->flags.ptr),
-                     words, words + 8, stream);
+    err = launchSort(k, v, count, keyBits, reinterpret_cast<uint32_t*>(scratch + kTicketBytes),
+                     reinterpret_cast<uint64_t*>(scratch + kTicketBytes + kSortHistBytes),
+                     reinterpret_cast<uint32_t*>(scratch), words + 8, stream, kClearNone);
     if (err == cudaSuccess && sortResultIndex(count, keyBits) == 1) {
         // RadixSort.cpp:165-174: an odd number of passes copies back.
         err = cudaMemcpyAsync(keys, scratchKeys, (size_t)count * 8, cudaMemcpyDeviceToDevice, stream);

@@ -18,36 +18,57 @@ FrameConst frameConstFor(const ath_projection& p, const ath_settings& s);
 InstanceConst instanceConstFor(const ath_projection& p, const ath_settings& s, const ath_instance& in, uint32_t base);
 
 // project.cu
-uint32_t projectBlocks(uint32_t slots);
-cudaError_t launchProject(const FrameConst& F, const InstanceConst* inst, uint32_t nInst, uint32_t slots,
-                          uint32_t layout, bool countCulls, float4* recs, uint2* rects, uint32_t* keys,
-                          uint32_t* offsets, uint64_t* flags, uint32_t* words, cudaStream_t stream);
-// Writes the pairs the buffers hold, min(pairs, capacity), into words[kWordPairsKept],
-// and raises kStatusPairOverflow in words[kWordSticky] past the capacity.
-cudaError_t launchEmit(const FrameConst& F, uint32_t slots, const float4* recs, const uint2* rects,
-                       const uint32_t* keys, const uint32_t* offsets, uint32_t* words, uint64_t capacity,
-                       uint64_t* pairKeys, uint32_t* pairValues, cudaStream_t stream);
-// Ranges over at most `pairs` sorted keys; `pairsDevice`, when given, holds the count.
-cudaError_t launchRanges(uint32_t pairs, const uint32_t* pairsDevice, uint32_t tiles, const uint64_t* pairKeys,
+uint32_t projectBlocks(uint32_t slots);   // also the look-back words of the projection, and of the emit
+// masks: a 64-bit word a slot, the tiles of its rect it touches (rects of at most 64 tiles).
+// inst: the instances in device memory; a single one is passed by value, `one`, and needs none.
+cudaError_t launchProject(const FrameConst& F, const InstanceConst& one, const InstanceConst* inst, uint32_t nInst, uint32_t slots,
+                          uint32_t layout, bool countCulls, float4* recs, uint2* rects, unsigned long long* masks,
+                          uint32_t* keys, uint32_t* offsets, uint64_t* flags, uint32_t* words, cudaStream_t stream);
+// The pairs (tile << 32 | slot) of the slots in `order` (the depth sort's). Writes the pairs the
+// buffers hold, min(pairs, capacity), into words[kWordPairsKept], and raises kStatusPairOverflow in
+// words[kWordSticky] past the capacity. flags: projectBlocks(slots) words, zeroed by the caller.
+cudaError_t launchEmit(const FrameConst& F, uint32_t slots, const uint32_t* order, const float4* recs,
+                       const uint2* rects, const unsigned long long* masks, const uint32_t* keys,
+                       const uint32_t* offsets, uint64_t* flags, uint32_t* words, uint64_t capacity, uint64_t* pairs,
+                       cudaStream_t stream);
+// Ranges over the sorted pairs, *pairsDevice of them, at most `pairs`.
+cudaError_t launchRanges(uint32_t pairs, const uint32_t* pairsDevice, uint32_t tiles, const uint64_t* sorted,
                          uint2* ranges, uint32_t* status, cudaStream_t stream);
+// The sorted pairs as (tile << 24 | depth key) and slot, for inspection.
+cudaError_t launchInspectPairs(const uint64_t* pairs, uint32_t count, const uint32_t* keys, uint32_t slots,
+                               uint64_t* pairKeys, uint32_t* pairSplats, cudaStream_t stream);
 
 // sort.cu
-constexpr uint32_t kSortTileKeys = 8192;   // keys a onesweep block ranks (the look-back's unit)
+constexpr uint32_t kSortTileKeys = 8192;   // keys a onesweep block ranks (the look-back's unit) in a large sort
 uint32_t sortPasses(uint32_t bits);      // 8-bit passes, or 9-bit ones where that saves a pass
 uint32_t sortHistWords();                // the words of a sort's digit histograms (every pass)
-uint32_t sortTiles(uint32_t n);
-size_t sortFlagWords(uint32_t n, uint32_t bits);
+// The look-back words of any sort of at most n keys (or of n keys in tiles of tileKeys); pairs:
+// 64-bit keys with values.
+size_t sortFlagWords(uint32_t n, uint32_t bits, bool pairs = false, uint32_t tileKeys = 0);
 uint32_t sortResultIndex(uint32_t n, uint32_t bits);
-cudaError_t sortPrepare();
+// Allows the kernels of the sorts an owner runs their shared memory.
+enum SortUse : uint32_t { kSortsKeys = 1, kSortsPairs = 2, kSortsDepths = 4 };   // 64-bit keys without and with values, a frame's depths
+cudaError_t sortPrepare(uint32_t uses);
+// What of its histograms, look-back words and tickets a sort clears: all; the histograms
+// (the words carry epochs, the tickets are the caller's); or none (the caller cleared them).
+enum SortClear : uint32_t { kClearAll, kClearHistograms, kClearNone };
 cudaError_t launchSort(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t bits, uint32_t* hist,
-                       uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream);
-cudaError_t launchSortBits(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t firstBit, uint32_t bits,
-                           uint32_t* hist, uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream);
-// The same with the key count on the device (at most n) and, when epochDevice is
-// given, epoch-tagged look-back words that need no clearing (a captured step).
+                       uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream,
+                       SortClear clear = kClearAll, uint32_t tileKeys = 0);
+// The same over bits [firstBit, firstBit + bits), with the key count on the device (at most n) and,
+// when epochDevice is given, epoch-tagged look-back words that need no clearing (a captured step).
 cudaError_t launchSortDevice(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, const uint32_t* nDevice,
                              const uint32_t* epochDevice, uint32_t firstBit, uint32_t bits, uint32_t* hist,
+                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream,
+                             SortClear clear = kClearAll, uint32_t tileKeys = 0);
+
+// A frame's splats front to back: the slots sorted stably by the low 24 bits of `keys` (left as
+// they are), into slots[0]; sortKeys and slots: room for n each. Culled slots (keys of
+// kCulledKey and a reason) come first. hist (three passes' worth), flags and tickets: zeroed by
+// the caller.
+cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n, uint32_t* hist,
                              uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream);
+constexpr uint32_t kDepthBits = 24;
 
 // blend.cu
 // The reference's contributionMode hooks of the blend (modes 1 and 4).
@@ -88,7 +109,7 @@ struct TrainingState {
 };
 
 cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
-                        const uint32_t* pairValues, const float4* recs, float4* colour, float* depth, float4* position,
+                        const uint64_t* sorted, const float4* recs, float4* colour, float* depth, float4* position,
                         const TrainingState* training, int sms, uint32_t* status, cudaStream_t stream,
                         const Contribution& contrib = Contribution{}, const Under& under = Under{},
                         const Matte& matte = Matte{});
@@ -99,7 +120,7 @@ size_t trainingLiveWords(const FrameConst& F, uint64_t pairs);
 
 // backward.cu
 cudaError_t launchBlendBackward(const FrameConst& F, uint32_t pairs, uint32_t slots, const uint2* ranges,
-                                const uint32_t* pairValues, const float4* recs, const TrainingState& training,
+                                const uint64_t* sorted, const float4* recs, const TrainingState& training,
                                 const float4* dLdColour, const float* dLdDepth,
                                 const float* depthOut, float* grads, uint32_t* status, cudaStream_t stream);
 cudaError_t launchProjectBackward(const FrameConst& F, const InstanceConst& I, const uint32_t* keys,

@@ -60,7 +60,9 @@ enum FrameWord : uint32_t {
     kWordMaxTiles = 5,
     kWordCulled = 6,        // 7 words: culled by reason (count_splats)
     kWordPairsKept = 13,    // the pairs the buffers hold: min(pairs, capacity), what the sort sorts
-    kWordSortTickets = 16,  // one a sort pass (up to 8)
+    kWordEmitTicket = 14,   // the emit's block ticket
+    kWordSortTickets = 16,  // one a pass of the pair sort (up to 5)
+    kWordDepthTickets = 21, // one a pass of the depth sort (3)
     kWordClouds = 24,       // 2 words a cloud (visible, pairs) for the first kMaxClouds instances (count_splats)
     kWordSticky = kWordClouds + 2 * kMaxClouds,   // status the emit, sort, ranges, blends and backward raise
     kFrameWords = kWordSticky + 1,                // cleared at the start of every frame

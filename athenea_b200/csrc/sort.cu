@@ -1,5 +1,5 @@
-// Stage (c): a stable LSD radix sort of 64-bit keys with 32-bit values, eight
-// (or nine) bits a pass, in the onesweep form (Adinets and Merrill, "Onesweep: A Faster
+// Stage (c): a stable LSD radix sort of 64-bit keys (32-bit for a frame's depths)
+// with 32-bit values, eight (or nine) bits a pass, in the onesweep form (Adinets and Merrill, "Onesweep: A Faster
 // Least Significant Digit Radix Sort for GPUs", 2022): one read of the keys
 // makes every pass's digit histogram, then each pass is a single kernel whose
 // tiles rank their keys in shared memory, find where each digit of theirs
@@ -21,11 +21,14 @@ namespace {
 constexpr uint32_t kMaxRadix = 512;     // a 9-bit pass's digits: the histograms' stride a pass
 constexpr uint32_t kSortThreads = 512;
 constexpr uint32_t kWarps = kSortThreads / 32;
-constexpr uint32_t kItems = 16;
-constexpr uint32_t kTileKeys = kSortThreads * kItems;   // 8192: fewer tiles for the look-back to walk
-static_assert(kTileKeys == kSortTileKeys, "kernels.h states the sort's tile size");
-// A warp ranks its items in independent chains (an 8-bit pass: items 0-7 and
-// 8-15), each with its own digit counters, so the chains' shared-memory round
+// Keys a thread: 16 (8192-key tiles: fewer tiles for the look-back to walk), or 4 where
+// 8192-key tiles would leave most SMs idle and one block's ranking would be the pass.
+// 64-bit keys with values take 12: with 16 their keys, places and destinations do not fit the
+// registers that two blocks an SM leave.
+constexpr uint32_t kItems = 16, kSmallItems = 4, kPairItems = 12;
+static_assert(kSortThreads * kItems == kSortTileKeys, "kernels.h states the sort's tile size");
+// A warp ranks its items in independent chains (an 8-bit pass of 8192-key tiles: items
+// 0-7 and 8-15), each with its own digit counters, so the chains' shared-memory round
 // trips overlap instead of queueing behind each other; the chains are ordered
 // after each other like warps.
 constexpr uint32_t kMaxPasses = 8;
@@ -50,8 +53,9 @@ struct SortPlan {
     uint32_t shift[kMaxPasses];   // from firstBit
 };
 
+template <typename K>
 __global__ void __launch_bounds__(256)
-    histogramKernel(const uint64_t* __restrict__ keys, uint32_t n, const uint32_t* __restrict__ nDevice,
+    histogramKernel(const K* __restrict__ keys, uint32_t n, const uint32_t* __restrict__ nDevice,
                     uint32_t firstBit, const SortPlan plan, uint32_t* __restrict__ hist) {
     __shared__ uint32_t sHist[kMaxPasses * kMaxRadix];
     n = countOf(n, nDevice);
@@ -62,11 +66,11 @@ __global__ void __launch_bounds__(256)
     constexpr uint32_t kBatch = 8;
     const uint64_t threads = (uint64_t)gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint64_t first = 0; first < n; first += kBatch * threads) {
-        uint64_t key[kBatch];
+        K key[kBatch];
 #pragma unroll
         for (uint32_t k = 0; k < kBatch; ++k) {
             const uint64_t i = first + k * threads + me;
-            key[k] = i < n ? keys[i] >> firstBit : 0ull;
+            key[k] = i < n ? keys[i] >> firstBit : (K)0;
         }
 #pragma unroll
         for (uint32_t k = 0; k < kBatch; ++k) {
@@ -104,24 +108,31 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* sWa
     return base + incl - v;
 }
 
+// What a pass carries beside its keys.
+enum SortValues : uint32_t { kNoValues = 0, kReadValues = 1, kIndexValues = 2 };   // index: a key's place in the input
+
 // kBits: the pass's digit width, 8 or 9 (kRadixT digits, one thread each in the
 // digit phase; a 9-bit pass ranks in one chain, so that its counters fit beside the keys).
-template <bool kValues, uint32_t kBits>
-__global__ void __launch_bounds__(kSortThreads, kValues ? 1 : 2)
-    onesweepKernel(const uint64_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
-                   uint64_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift,
-                   uint32_t digitMask, const uint32_t* __restrict__ globalHist, uint64_t* __restrict__ flags,
-                   uint32_t* __restrict__ ticket,
+// The values take the keys' shared memory once the keys are out, each thread keeping its
+// items' places in the tile and its outputs' destinations in registers: with values as
+// without, two blocks an SM (values beside the keys, 128 KB, left one). 8M pairs of
+// 40 bits: 605 -> 594 us.
+template <typename K, uint32_t kValues, uint32_t kBits, uint32_t kPerThread>
+__global__ void __launch_bounds__(kSortThreads, 2)
+    onesweepKernel(const K* __restrict__ keysIn, const uint32_t* __restrict__ valsIn, K* __restrict__ keysOut,
+                   uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift, uint32_t digitMask,
+                   const uint32_t* __restrict__ globalHist, uint64_t* __restrict__ flags, uint32_t* __restrict__ ticket,
                    uint32_t* __restrict__ status, const uint32_t* __restrict__ nDevice,
                    const uint32_t* __restrict__ epochDevice) {
     constexpr uint32_t kRadix = 1u << kBits;
-    constexpr uint32_t kChains = kBits == 8 ? 2 : 1;
-    constexpr uint32_t kChainItems = kItems / kChains;
+    constexpr uint32_t kChains = kBits == 8 && kPerThread >= 16 ? 2 : 1;
+    constexpr uint32_t kChainItems = kPerThread / kChains;
     constexpr uint32_t kCounters = kWarps * kChains;
+    constexpr uint32_t kTileKeys = kSortThreads * kPerThread;
     extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t* sKeys = reinterpret_cast<uint64_t*>(smem);
-    uint32_t* sVals = reinterpret_cast<uint32_t*>(sKeys + kTileKeys);
-    uint32_t* sWarpCnt = kValues ? sVals + kTileKeys : sVals;   // kCounters x kRadix
+    K* sKeys = reinterpret_cast<K*>(smem);
+    uint32_t* sVals = reinterpret_cast<uint32_t*>(smem);
+    uint32_t* sWarpCnt = reinterpret_cast<uint32_t*>(sKeys + kTileKeys);   // kCounters x kRadix
     __shared__ uint32_t sTile;
     __shared__ uint32_t sStart[kRadix];
     __shared__ uint32_t sAdjust[kRadix];
@@ -141,19 +152,14 @@ __global__ void __launch_bounds__(kSortThreads, kValues ? 1 : 2)
     __syncthreads();
     const uint32_t ltMask = (1u << lane) - 1u;
 
-    // Rank: warp `warp` owns keys [base + warp*32*kItems, +32*kItems), item k of
+    // Rank: warp `warp` owns keys [base + warp*32*kPerThread, +32*kPerThread), item k of
     // lane l being the (k*32 + l)-th; walking k then l is input order, so the
     // ranks are stable.
-    uint64_t key[kItems];
-    uint32_t val[kItems];
-    uint32_t rank[kItems];
+    const uint32_t mine = base + warp * 32 * kPerThread + lane;
+    K key[kPerThread];
+    uint32_t rank[kPerThread];
 #pragma unroll
-    for (uint32_t k = 0; k < kItems; ++k) {
-        const uint32_t idx = base + warp * 32 * kItems + k * 32 + lane;
-        const bool valid = idx < n;
-        key[k] = valid ? keysIn[idx] : 0ull;
-        if constexpr (kValues) val[k] = valid ? valsIn[idx] : 0u;
-    }
+    for (uint32_t k = 0; k < kPerThread; ++k) key[k] = mine + k * 32 < n ? keysIn[mine + k * 32] : (K)0;
 #pragma unroll
     for (uint32_t i = 0; i < kChainItems; ++i) {
         uint32_t d[kChains], peers[kChains], before[kChains];
@@ -161,7 +167,7 @@ __global__ void __launch_bounds__(kSortThreads, kValues ? 1 : 2)
 #pragma unroll
         for (uint32_t c = 0; c < kChains; ++c) {
             const uint32_t k = c * kChainItems + i;
-            valid[c] = base + warp * 32 * kItems + k * 32 + lane < n;
+            valid[c] = mine + k * 32 < n;
             d[c] = valid[c] ? (uint32_t)((key[k] >> shift) & digitMask) : kRadix + lane;
             peers[c] = __match_any_sync(0xFFFFFFFFu, d[c]);
         }
@@ -230,37 +236,66 @@ __global__ void __launch_bounds__(kSortThreads, kValues ? 1 : 2)
     __syncthreads();
 
     // Scatter into shared memory in the tile's sorted order, then out.
+    uint32_t place[kPerThread / 2];   // the items' places in that order, two a word (at most 8191)
 #pragma unroll
-    for (uint32_t k = 0; k < kItems; ++k) {
-        const uint32_t idx = base + warp * 32 * kItems + k * 32 + lane;
-        if (idx < n) {
-            const uint32_t d = (uint32_t)((key[k] >> shift) & digitMask);
-            const uint32_t at = digitSlot(d);
-            const uint32_t s =
-                sStart[at] + sWarpCnt[(warp * kChains + k / kChainItems) * kRadix + at] + rank[k];
+    for (uint32_t k = 0; k < kPerThread; ++k) {
+        uint32_t s = 0;
+        if (mine + k * 32 < n) {
+            const uint32_t at = digitSlot((uint32_t)((key[k] >> shift) & digitMask));
+            s = sStart[at] + sWarpCnt[(warp * kChains + k / kChainItems) * kRadix + at] + rank[k];
             sKeys[s] = key[k];
-            if constexpr (kValues) sVals[s] = val[k];
         }
+        place[k / 2] = k & 1u ? place[k / 2] | (s << 16) : s;
     }
     __syncthreads();
     const uint32_t tileN = min(kTileKeys, n - base);
-    for (uint32_t s = tid; s < tileN; s += kSortThreads) {
-        const uint64_t k = sKeys[s];
-        const uint32_t dst = sAdjust[digitSlot((uint32_t)((k >> shift) & digitMask))] + s;
-        if (dst < n) {
-            keysOut[dst] = k;
-            if constexpr (kValues) valsOut[dst] = sVals[s];
-        } else {
-            atomicOr(status, kStatusIndexRange);
+    uint32_t to[kValues == kNoValues ? 1 : kPerThread];
+#pragma unroll
+    for (uint32_t k = 0; k < kPerThread; ++k) {
+        const uint32_t s = tid + k * kSortThreads;
+        uint32_t dst = 0xFFFFFFFFu;
+        if (s < tileN) {
+            const K out = sKeys[s];
+            dst = sAdjust[digitSlot((uint32_t)((out >> shift) & digitMask))] + s;
+            if (dst < n) {
+                if (keysOut) keysOut[dst] = out;
+            } else {
+                atomicOr(status, kStatusIndexRange);
+                dst = 0xFFFFFFFFu;
+            }
         }
+        if constexpr (kValues != kNoValues) to[k] = dst;
+    }
+    if constexpr (kValues != kNoValues) {
+        uint32_t val[kPerThread];
+#pragma unroll
+        for (uint32_t k = 0; k < kPerThread; ++k)
+            val[k] = kValues == kIndexValues ? mine + k * 32 : mine + k * 32 < n ? valsIn[mine + k * 32] : 0u;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < kPerThread; ++k)
+            if (mine + k * 32 < n) sVals[(place[k / 2] >> (16 * (k & 1u))) & 0xFFFFu] = val[k];
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < kPerThread; ++k)
+            if (to[k] != 0xFFFFFFFFu) valsOut[to[k]] = sVals[tid + k * kSortThreads];
     }
 }
 
-// A pass's dynamic shared memory: its keys (and values) and its chains' digit counters.
-constexpr size_t onesweepSmem(bool values, uint32_t bits) {
-    return (size_t)kTileKeys * 8 + (values ? (size_t)kTileKeys * 4 : 0) +
-           (size_t)kWarps * (bits == 8 ? 2 : 1) * ((size_t)1 << bits) * 4;
+// A pass's dynamic shared memory: its keys and its chains' digit counters.
+template <typename K, uint32_t kBits, uint32_t kPerThread>
+constexpr size_t onesweepSmem() {
+    return (size_t)kSortThreads * kPerThread * sizeof(K) +
+           (size_t)kWarps * (kBits == 8 && kPerThread >= 16 ? 2 : 1) * ((size_t)1 << kBits) * 4;
 }
+
+template <typename K, uint32_t kValues, uint32_t kBits, uint32_t kPerThread>
+cudaError_t allowSmem() {
+    return cudaFuncSetAttribute(onesweepKernel<K, kValues, kBits, kPerThread>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)onesweepSmem<K, kBits, kPerThread>());
+}
+// what a block takes without asking, its static arrays included
+static_assert(onesweepSmem<uint64_t, 8, kSmallItems>() <= 44 * 1024, "small tiles of eight bits ask for no more");
 
 // The passes of a sort of `bits` bits: eight bits a pass, or, where that takes a
 // pass fewer, nine bits in as many passes as needed and eight in the rest
@@ -282,85 +317,149 @@ SortPlan planSort(uint32_t bits) {
 }   // namespace
 
 uint32_t sortPasses(uint32_t bits) { return planSort(bits).passes; }
-uint32_t sortTiles(uint32_t n) { return (n + kTileKeys - 1) / kTileKeys; }
-size_t sortFlagWords(uint32_t n, uint32_t bits) {
+// Small tiles up to the count at which 2048-key tiles fill two blocks on every SM.
+constexpr uint32_t kSmallTile = kSortThreads * kSmallItems, kSmallSort = 2u * 148u * kSmallTile;
+uint32_t sortTileKeys(uint32_t n, bool pairs) {
+    return n <= kSmallSort ? kSmallTile : pairs ? kSortThreads * kPairItems : kSortTileKeys;
+}
+size_t sortFlagWords(uint32_t n, uint32_t bits, bool pairs, uint32_t tileKeys) {
     const SortPlan p = planSort(bits);
-    size_t words = 0;
-    for (uint32_t k = 0; k < p.passes; ++k) words += (size_t)sortTiles(n) << p.width[k];
-    return words;
+    auto words = [&](uint32_t count, uint32_t keys) {
+        size_t w = 0;
+        for (uint32_t k = 0; k < p.passes; ++k) w += (size_t)((count + keys - 1) / keys) << p.width[k];
+        return w;
+    };
+    if (tileKeys) return words(n, tileKeys);
+    // room for any sort of at most n keys: a smaller one may take the small tiles
+    const size_t most = words(n, sortTileKeys(n, pairs));
+    return n > kSmallSort ? max(most, words(kSmallSort, kSmallTile)) : most;
 }
 
-cudaError_t sortPrepare() {
-    cudaError_t err = cudaFuncSetAttribute(onesweepKernel<true, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)onesweepSmem(true, 8));
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(onesweepKernel<false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)onesweepSmem(false, 8));
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(onesweepKernel<true, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)onesweepSmem(true, 9));
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(onesweepKernel<false, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)onesweepSmem(false, 9));
+// Each some 6 us: an owner asks for the sorts it runs.
+cudaError_t sortPrepare(uint32_t uses) {
+    cudaError_t err = cudaSuccess;
+    auto also = [&](cudaError_t (*allow)()) { if (err == cudaSuccess) err = allow(); };
+    if (uses & kSortsKeys) {
+        also(allowSmem<uint64_t, kNoValues, 8, kItems>);
+        also(allowSmem<uint64_t, kNoValues, 9, kItems>);
+        also(allowSmem<uint64_t, kNoValues, 9, kSmallItems>);
+    }
+    if (uses & kSortsPairs) {
+        also(allowSmem<uint64_t, kReadValues, 8, kItems>);
+        also(allowSmem<uint64_t, kReadValues, 9, kItems>);
+        also(allowSmem<uint64_t, kReadValues, 8, kPairItems>);
+        also(allowSmem<uint64_t, kReadValues, 9, kPairItems>);
+        also(allowSmem<uint64_t, kReadValues, 9, kSmallItems>);
+    }
+    if (uses & kSortsDepths) {
+        also(allowSmem<uint32_t, kIndexValues, 8, kItems>);
+        also(allowSmem<uint32_t, kReadValues, 8, kItems>);
+    }
     return err;
 }
+
+namespace {
+
+template <typename K, uint32_t kValues, uint32_t kBits>
+void launchPass(uint32_t tileKeys, uint32_t tiles, const K* keysIn, const uint32_t* valsIn, K* keysOut,
+                uint32_t* valsOut, uint32_t n, uint32_t shift, const uint32_t* hist, uint64_t* flags, uint32_t* ticket,
+                uint32_t* status, const uint32_t* nDevice, const uint32_t* epochDevice, uint32_t digitMask,
+                cudaStream_t stream) {
+#define ATH_TILE(I_)                                                                                                 \
+    onesweepKernel<K, kValues, kBits, I_><<<tiles, kSortThreads, onesweepSmem<K, kBits, I_>(), stream>>>(            \
+        keysIn, valsIn, keysOut, valsOut, n, shift, digitMask, hist, flags, ticket, status, nDevice, epochDevice)
+    if constexpr (sizeof(K) == 8 && kValues != kNoValues)
+        if (tileKeys == kSortThreads * kPairItems) return (void)(ATH_TILE(kPairItems));
+    if (tileKeys == kSortTileKeys) ATH_TILE(kItems);
+    else ATH_TILE(kSmallItems);
+#undef ATH_TILE
+}
+
+// What the sorts share: the clearing, the digit histograms of `in`, then `pass` for each pass.
+template <typename K, typename Pass>
+cudaError_t runSort(uint32_t n, const uint32_t* nDevice, const uint32_t* epochDevice, uint32_t firstBit, uint32_t bits,
+                    uint32_t tileKeys, SortClear clear, uint32_t* hist, uint64_t* flags, uint32_t* tickets,
+                    cudaStream_t stream, const K* in, bool pairs, Pass pass) {
+    const SortPlan plan = planSort(bits);
+    if (plan.passes > kMaxPasses || firstBit + bits > 8 * sizeof(K)) return cudaErrorInvalidValue;
+    const uint32_t keys = tileKeys ? tileKeys : sortTileKeys(n, pairs);
+    const uint32_t tiles = (n + keys - 1) / keys;
+    cudaError_t err = cudaSuccess;
+    if (clear != kClearNone) err = cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kMaxRadix * plan.passes, stream);
+    if (err == cudaSuccess && clear == kClearAll) {
+        err = cudaMemsetAsync(flags, 0, sizeof(uint64_t) * sortFlagWords(n, bits, pairs, keys), stream);
+        if (err == cudaSuccess) err = cudaMemsetAsync(tickets, 0, sizeof(uint32_t) * plan.passes, stream);
+    }
+    if (err != cudaSuccess) return err;
+    int device = 0, sms = 148;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    histogramKernel<K><<<min((n + 255) / 256, (uint32_t)sms * 4), 256, 0, stream>>>(in, n, nDevice, firstBit, plan, hist);
+    for (uint32_t p = 0; p < plan.passes; ++p) {
+        pass(p, plan, keys, tiles, firstBit + plan.shift[p], hist + p * kMaxRadix, flags, tickets + p,
+             (1u << plan.width[p]) - 1u);
+        flags += (size_t)tiles << plan.width[p];
+    }
+    return cudaGetLastError();
+}
+
+}   // namespace
 
 // keys/vals[0] hold the input; the sorted result lands in keys/vals[passes & 1]
 // (the caller reads sortResultIndex). vals may be null (keys only). The passes
 // sort bits [firstBit, firstBit + bits) of the keys, eight or nine at a time
 // (planSort). hist: kMaxPasses * kSortHistStride words, flags: sortFlagWords
-// words, tickets: one word a pass; all three are zeroed here.
+// words, tickets: one word a pass; all three start at zero (`clear`: what of them is
+// zeroed here). tileKeys: kSortTileKeys for callers whose flags hold no more than that
+// takes; 0 by the count.
 cudaError_t launchSortDevice(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, const uint32_t* nDevice,
                              const uint32_t* epochDevice, uint32_t firstBit, uint32_t bits, uint32_t* hist,
-                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream) {
+                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream,
+                             SortClear clear, uint32_t tileKeys) {
     if (n <= 1 && !nDevice) return cudaSuccess;
-    const SortPlan plan = planSort(bits);
-    const uint32_t passes = plan.passes;
-    if (passes > kMaxPasses || firstBit + bits > 64) return cudaErrorInvalidValue;
-    const uint32_t tiles = sortTiles(n);
-    cudaError_t err = cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kMaxRadix * passes, stream);
-    if (err != cudaSuccess) return err;
-    if (!epochDevice) {
-        err = cudaMemsetAsync(flags, 0, sizeof(uint64_t) * sortFlagWords(n, bits), stream);
-        if (err != cudaSuccess) return err;
-    }
-    err = cudaMemsetAsync(tickets, 0, sizeof(uint32_t) * passes, stream);
-    if (err != cudaSuccess) return err;
-    int device = 0, sms = 148;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const uint32_t hblocks = min((n + 255) / 256, (uint32_t)sms * 4);
-    histogramKernel<<<hblocks, 256, 0, stream>>>(keys[0], n, nDevice, firstBit, plan, hist);
     const bool withValues = vals != nullptr && vals[0] != nullptr;
-    size_t flagAt = 0;
-    for (uint32_t p = 0; p < passes; ++p) {
+    auto pass = [&](uint32_t p, const SortPlan& plan, uint32_t tileKeysHere, uint32_t tiles, uint32_t shift,
+                    const uint32_t* h, uint64_t* f, uint32_t* ticket, uint32_t mask) {
         const uint32_t in = p & 1u, out = in ^ 1u;
-        const uint32_t shift = firstBit + plan.shift[p];
-        const uint32_t* h = hist + p * kMaxRadix;
-        const uint32_t digitMask = (1u << plan.width[p]) - 1u;
-        uint64_t* f = flags + flagAt;
-        flagAt += (size_t)tiles << plan.width[p];
-#define ATH_PASS(V_, W_)                                                                                          \
-    onesweepKernel<V_, W_><<<tiles, kSortThreads, onesweepSmem(V_, W_), stream>>>(                             \
-        keys[in], V_ ? vals[in] : nullptr, keys[out], V_ ? vals[out] : nullptr, n, shift, digitMask, h, f,         \
-        tickets + p, status, nDevice, epochDevice)
-        if (withValues && plan.width[p] == 9) ATH_PASS(true, 9);
-        else if (withValues) ATH_PASS(true, 8);
-        else if (plan.width[p] == 9) ATH_PASS(false, 9);
-        else ATH_PASS(false, 8);
+        const uint32_t* vi = withValues ? vals[in] : nullptr;
+        uint32_t* vo = withValues ? vals[out] : nullptr;
+#define ATH_PASS(V_, W_)                                                                                            \
+    launchPass<uint64_t, V_, W_>(tileKeysHere, tiles, keys[in], vi, keys[out], vo, n, shift, h, f, ticket, status, \
+                                 nDevice, epochDevice, mask, stream)
+        if (withValues && plan.width[p] == 9) ATH_PASS(kReadValues, 9);
+        else if (withValues) ATH_PASS(kReadValues, 8);
+        else if (plan.width[p] == 9) ATH_PASS(kNoValues, 9);
+        else ATH_PASS(kNoValues, 8);
 #undef ATH_PASS
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launchSortBits(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t firstBit, uint32_t bits,
-                           uint32_t* hist, uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream) {
-    return launchSortDevice(keys, vals, n, nullptr, nullptr, firstBit, bits, hist, flags, tickets, status, stream);
+    };
+    return runSort<uint64_t>(n, nDevice, epochDevice, firstBit, bits, tileKeys, clear, hist, flags, tickets, stream, keys[0],
+                             withValues, pass);
 }
 
 cudaError_t launchSort(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_t bits, uint32_t* hist,
-                       uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream) {
-    return launchSortBits(keys, vals, n, 0, bits, hist, flags, tickets, status, stream);
+                       uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream, SortClear clear,
+                       uint32_t tileKeys) {
+    return launchSortDevice(keys, vals, n, nullptr, nullptr, 0, bits, hist, flags, tickets, status, stream, clear, tileKeys);
+}
+
+cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n, uint32_t* hist,
+                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream) {
+    if (n == 0) return cudaSuccess;
+    // three 8-bit passes: keys -> [0] -> [1] -> [0], the first carrying its keys' places, the
+    // last writing the slots alone
+    auto pass = [&](uint32_t p, const SortPlan& plan, uint32_t tileKeys, uint32_t tiles, uint32_t shift, const uint32_t* h,
+                    uint64_t* f, uint32_t* ticket, uint32_t mask) {
+        const uint32_t out = p & 1u, in = out ^ 1u;
+        uint32_t* ko = p + 1 == plan.passes ? nullptr : sortKeys[out];
+        if (p == 0)
+            launchPass<uint32_t, kIndexValues, 8>(tileKeys, tiles, keys, nullptr, ko, slots[out], n, shift, h, f, ticket,
+                                                  status, nullptr, nullptr, mask, stream);
+        else
+            launchPass<uint32_t, kReadValues, 8>(tileKeys, tiles, sortKeys[in], slots[in], ko, slots[out], n, shift, h, f,
+                                                 ticket, status, nullptr, nullptr, mask, stream);
+    };
+    static_assert(kDepthBits == 24, "three 8-bit passes");
+    return runSort<uint32_t>(n, nullptr, nullptr, 0, kDepthBits, 0, kClearNone, hist, flags, tickets, stream, keys, false, pass);
 }
 
 uint32_t sortResultIndex(uint32_t n, uint32_t bits) { return n <= 1 ? 0u : (sortPasses(bits) & 1u); }

@@ -60,7 +60,7 @@ ath_status scratchOf(int device, uint64_t** out) {
         void* p = nullptr;
         cudaError_t err = cudaGetSymbolAddress(&p, gSortScratch);
         if (err != cudaSuccess) return failCuda(err, "ath_sort_pairs_static: finding the static working memory");
-        err = sortPrepare();   // the onesweep kernel's shared-memory limit, once a device
+        err = sortPrepare(kSortsPairs);   // the onesweep kernel's shared-memory limit, once a device
         if (err != cudaSuccess) return failCuda(err, "ath_sort_pairs_static: preparing the sort");
         d.ptr = static_cast<uint64_t*>(p);
         d.ready = true;
@@ -96,7 +96,7 @@ extern "C" ath_status ath_sort_pairs_static(uint64_t* keys, uint32_t* values, ui
     uint32_t* hist = reinterpret_cast<uint32_t*>(scratch + kFlagWords);
     uint32_t* counters = reinterpret_cast<uint32_t*>(scratch + kFlagWords + kHistWords);
     uint32_t* status = counters + 8;
-    if (sortFlagWords(count, keyBits) > kFlagWords || sortHistWords() > 2 * kHistWords)
+    if (sortFlagWords(count, keyBits, true, kSortTileKeys) > kFlagWords || sortHistWords() > 2 * kHistWords)
         return fail(ATH_E_INTERNAL, "ath_sort_pairs_static: the static working memory is too small for this sort");
     // The status word is not read here: the call enqueues its work and returns.
     // What a call raises (a look-back that gave up, an index outside the buffers)
@@ -104,7 +104,7 @@ extern "C" ath_status ath_sort_pairs_static(uint64_t* keys, uint32_t* values, ui
     // launchSort clears the histograms, the look-back words and the tickets it uses.
     uint64_t* k[2] = {keys, scratchKeys};
     uint32_t* v[2] = {values, scratchValues};
-    err = launchSort(k, v, count, keyBits, hist, flags, counters, status, stream);
+    err = launchSort(k, v, count, keyBits, hist, flags, counters, status, stream, kClearAll, kSortTileKeys);
     if (err == cudaSuccess && sortResultIndex(count, keyBits) == 1) {
         err = cudaMemcpyAsync(keys, scratchKeys, (size_t)count * 8, cudaMemcpyDeviceToDevice, stream);
         if (err == cudaSuccess)

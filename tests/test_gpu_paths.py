@@ -1,0 +1,84 @@
+"""The paths a call takes by its sizes, alignment and options, at the sizes where they
+change or leave remainders: boxes of one and of two pixels a lane, rects too large for a
+mask, sorts in one block and in small and large tiles, decodes through shared memory and
+not, gradient rows moved by 16 bytes and by values."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import athenea_b200 as A
+from athenea_b200 import _native as N
+from athenea_b200 import scenes
+from perf import cases
+from tests.fixtures import random_cloud
+from tests.test_gpu_parity import _compare, _decode, _settings
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def raster(native):
+    return A.TileRasterizer.create()
+
+
+# On 148 SMs a frame takes boxes of one pixel a lane below 4736 tiles: (1184, 1008) is the last of them here,
+# (1184, 1024) is past it; (1279, 719) leaves part of a box in both directions; (16, 16) is one tile, (3, 5) less than a box
+@pytest.mark.parametrize("size", [(3, 5), (16, 16), (250, 190), (1279, 719), (1184, 1008), (1184, 1024)])
+@pytest.mark.parametrize("opacity", [1.0, 6.0])
+def test_frames_equal_the_restatement_to_the_bit(oracle, native, raster, size, opacity):
+    """Footprints from a pixel to the whole image (rects of more than 64 tiles), with opacities over 1 (the harder
+    kernel) by an edit, over a background."""
+    W, H = size
+    packed = _decode(oracle, random_cloud(900, 17 + W, min_size=0.002, max_size=1.5))
+    cam = A.pinhole_for_vertical_fov((0.3, 0.2, 4.0), (0, 0, 0), W, H, 60.0)
+    s = _settings(W, H, background=(0.1, 0.3, 0.2, 0.4), depth_mode=int(W % 2))
+    edit = A.SplatEdit(active=True, mode=2, size=(1.0, 2.0, 2.0), opacity=opacity) if opacity != 1.0 else None
+    got, want = _compare(oracle, None, raster, [packed], [np.eye(4)], cam.projection_for(W, H), s, edit=edit)
+    np.testing.assert_array_equal(got["colour"], want["colour"])
+    np.testing.assert_array_equal(got["depth"], want["depth"])
+
+
+def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(native, raster):
+    """A frame's pairs around the 8192 a block sorts by itself: the same image with the capacity a hundred pairs
+    need and with that of a frame before it that needed many."""
+    W, H = 160, 120
+    cam = A.pinhole_for_vertical_fov((0, 0, 3), (0, 0, 0), W, H, 60.0).projection_for(W, H)
+    small, large = [cases._records(cases._gaussians(n, True, 1, 5)) for n in (3000, 60_000)]
+    small, large = [A.CloudLoader.upload(*r) for r in (small, large)]
+    images = []
+    for first in (None, large):
+        r = A.TileRasterizer.create()
+        t = A.RenderTargets.make(W, H)
+        if first is not None:
+            r.render(cam, [A.SplatInstance(first)], A.RenderSettings(width=W, height=H), t)
+        r.render(cam, [A.SplatInstance(small)], A.RenderSettings(width=W, height=H), t)
+        images.append((t.colour.cpu(), t.depth.cpu()))
+    assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
+
+
+# A pixel whose walk takes a decision near its threshold (about 1 in 500) may take it the other way in 64 bits: a
+# splat of alpha 1/255 in or out. Images then agree to 1/255 / sqrt(500) = 2e-4 of their norm, gradients, which such a
+# splat's are few of but whole, to 1e-2.
+@pytest.mark.parametrize("case", [
+    dict(kind="train", count=3001, clustered=True, degree=0, width=97, height=61, depth_loss=True),
+    dict(kind="train", count=2500, clustered=False, degree=1, width=480, height=480, depth_loss=False),
+    dict(kind="train", count=4003, clustered=True, degree=2, width=640, height=361, depth_loss=True),
+    dict(kind="train", count=4003, clustered=True, degree=3, width=1281, height=483, depth_loss=True),
+    dict(kind="step", count=2000, clustered=True, degree=3, views=3, width=131, height=77, tile=8, batch=64),
+    dict(kind="step", count=3000, clustered=True, degree=1, views=2, width=320, height=201, tile=16, batch=512),
+    dict(kind="step", count=3000, clustered=True, degree=2, views=5, width=161, height=120, tile=32, batch=128),
+    dict(kind="views", count=3000, clustered=False, degree=3, views=2, width=333, height=251, tile=32, batch=512),
+    dict(kind="frame", count=3000, clustered=True, degree=2, width=801, height=433, clouds=5, extra="matte",
+         threshold=False, wait=True),
+], ids=lambda c: f"{c['kind']}-{c['width']}x{c['height']}-{c['degree']}")
+def test_calls_agree_with_64_bits(native, case):
+    got = cases.run(cases.prepare(case, 5))
+    want = cases.exact(case, 5)
+    for name, value in want.items():
+        if value is None:
+            continue
+        g, w = got[name].double().reshape(-1), value.double().reshape(-1)
+        rel = float((g - w).norm() / w.norm())
+        assert rel <= (1e-3 if name in ("colour", "loss") else 1e-2), (name, rel)
