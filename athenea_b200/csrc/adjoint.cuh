@@ -52,13 +52,12 @@ __device__ __forceinline__ void shBasis(uint32_t degree, float x, float y, float
     dY[14][0] = C3[6] * (3.0f * xx - 3.0f * yy); dY[14][1] = C3[6] * (-6.0f * xy);
 }
 
-// dL/dparameters of one Gaussian, kept in registers so a caller can sum it over views.
+// dL/dparameters of one Gaussian but its SH, kept in registers so a caller can sum it over views.
 struct ParamGrad {
     float dp[3];        // means
     float dLogit;
     float dLogScale[3];
     float dQuat[4];     // w x y z
-    float dSh[48];      // DC rgb, then the rest rgb per basis
 
     __device__ __forceinline__ void clear() {
 #pragma unroll
@@ -66,27 +65,19 @@ struct ParamGrad {
         dLogit = 0.0f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) dQuat[k] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 48; ++k) dSh[k] = 0.0f;
     }
 
-    // Added into the gradient arrays (ath_param_grads' layout).
-    __device__ __forceinline__ void addTo(uint32_t i, uint32_t shStride, float4* gMeans, float4* gScales, float4* gQuats,
-                                          float* gSh, bool overwrite = false) const {
-        float4 m = overwrite ? make_float4(0, 0, 0, 0) : gMeans[i];
+    // All but the SH, added into the gradient arrays (ath_param_grads' layout).
+    __device__ __forceinline__ void addGeometryTo(uint32_t i, float4* gMeans, float4* gScales, float4* gQuats) const {
+        float4 m = gMeans[i];
         m.x += dp[0]; m.y += dp[1]; m.z += dp[2]; m.w += dLogit;
         gMeans[i] = m;
-        float4 s = overwrite ? make_float4(0, 0, 0, 0) : gScales[i];
+        float4 s = gScales[i];
         s.x += dLogScale[0]; s.y += dLogScale[1]; s.z += dLogScale[2];
         gScales[i] = s;
-        float4 q = overwrite ? make_float4(0, 0, 0, 0) : gQuats[i];
+        float4 q = gQuats[i];
         q.x += dQuat[0]; q.y += dQuat[1]; q.z += dQuat[2]; q.w += dQuat[3];
         gQuats[i] = q;
-        float* row = gSh + (size_t)i * shStride;
-        const uint32_t n = shStride < 48 ? shStride : 48;
-#pragma unroll
-        for (uint32_t k = 0; k < 48; ++k)
-            if (k < n) row[k] = (overwrite ? 0.0f : row[k]) + dSh[k];
     }
 };
 
@@ -244,34 +235,22 @@ __device__ __forceinline__ void shapeAdjoint(const InstanceConst& I, uint32_t i,
     acc.dQuat[0] += dQuat.x; acc.dQuat[1] += dQuat.y; acc.dQuat[2] += dQuat.z; acc.dQuat[3] += dQuat.w;
 }
 
-// The projection's adjoint past the colour, for one Gaussian and one view:
-// dL/d(record) `gw` -> dL/d(position, opacity logit, log scales, quaternion).
-template <uint32_t L>
-__device__ __forceinline__ void geometryAdjoint(const FrameConst& F, const InstanceConst& I, uint32_t i, const Gauss& g,
-                                                const Geometry& G, const float gw[kGradWords], float dp[3],
-                                                ParamGrad& acc) {
-    float dM[3][3];
-    geometryAdjointToM(F, I, g, G, gw, dp, acc, dM);
-    shapeAdjoint(I, i, g, G.R, dM, acc);
-}
-
-// The projection's adjoint for one Gaussian and one view: dL/d(record) `gw`
-// (gradient words of raster_types.cuh) -> dL/dparameters, added into `acc`.
-template <uint32_t L>
-__device__ __forceinline__ void projectAdjoint(const FrameConst& F, const InstanceConst& I, uint32_t i,
-                                               const float gw[kGradWords], ParamGrad& acc) {
-    const Gauss g = loadGauss<L>(I, i);
-    const Geometry G = projectGeometry<L == kLayoutMixed>(F, I, g, g.opacity);
+// The projection's adjoint for one Gaussian of FP32 training parameters and one view:
+// dL/d(record) `gw` (gradient words of raster_types.cuh) -> dL/dparameters, added into
+// `acc`; `sh` holds the Gaussian's SH row (DC rgb, then the rest rgb per basis, `bases` of
+// them) and receives dL/dSH in its place.
+__device__ __forceinline__ void projectAdjoint(const FrameConst& F, const InstanceConst& I, uint32_t i, uint32_t degree,
+                                               uint32_t bases, const float gw[kGradWords], float* sh, ParamGrad& acc) {
+    const Gauss g = loadGauss<kLayoutParams>(I, i);
+    const Geometry G = projectGeometry(F, I, g, g.opacity);
 
     // ---- colour: c = decode(base + rest(dir)) ------------------------------
     float dp[3] = {0.0f, 0.0f, 0.0f};
-    const uint32_t degree = min(degreeOf(I.restPerColour), F.shLimit);
     const float ex = g.px - I.eye[0], ey = g.py - I.eye[1], ez = g.pz - I.eye[2];
     const float len = sqrtf((ex * ex + ey * ey) + ez * ez);
     const float dir[3] = {ex / len, ey / len, ez / len};
     float Y[15], dY[15][3];
     shBasis(degree, dir[0], dir[1], dir[2], Y, dY);
-    const uint32_t bases = degree == 3 ? 15 : degree == 2 ? 8 : degree == 1 ? 3 : 0;
     float dDir[3] = {0.0f, 0.0f, 0.0f};
     const float gc[3] = {gw[kGradR], gw[kGradG], gw[kGradB]};
 #pragma unroll
@@ -279,7 +258,7 @@ __device__ __forceinline__ void projectAdjoint(const FrameConst& F, const Instan
         float v = g.base[ch];
 #pragma unroll
         for (uint32_t k = 0; k < 15; ++k)
-            if (k < bases) v += Y[k] * restAt<L>(I, i, k * 3 + (uint32_t)ch);
+            if (k < bases) v += Y[k] * sh[3 + k * 3 + ch];
         float dcdv;
         if (I.linear != 0) {
             dcdv = v > 0.0f ? 1.0f : 0.0f;
@@ -287,12 +266,12 @@ __device__ __forceinline__ void projectAdjoint(const FrameConst& F, const Instan
             dcdv = v <= 0.0f ? 0.0f : v <= 0.04045f ? 1.0f / 12.92f : (2.4f / 1.055f) * pow_f((v + 0.055f) / 1.055f, 1.4f);
         }
         const float dv = gc[ch] * dcdv;
-        acc.dSh[ch] += kSH0 * dv;
+        sh[ch] = kSH0 * dv;
 #pragma unroll
         for (uint32_t k = 0; k < 15; ++k) {
             if (k >= bases) continue;
-            acc.dSh[3 + k * 3 + ch] += Y[k] * dv;
-            const float coef = restAt<L>(I, i, k * 3 + (uint32_t)ch) * dv;
+            const float coef = sh[3 + k * 3 + ch] * dv;
+            sh[3 + k * 3 + ch] = Y[k] * dv;
             dDir[0] += dY[k][0] * coef;
             dDir[1] += dY[k][1] * coef;
             dDir[2] += dY[k][2] * coef;
@@ -305,8 +284,9 @@ __device__ __forceinline__ void projectAdjoint(const FrameConst& F, const Instan
         for (int k = 0; k < 3; ++k) dp[k] += (dDir[k] - dir[k] * dd) / len;
     }
 
-    geometryAdjoint<L>(F, I, i, g, G, gw, dp, acc);
+    float dM[3][3];
+    geometryAdjointToM(F, I, g, G, gw, dp, acc, dM);
+    shapeAdjoint(I, i, g, G.R, dM, acc);
 }
-
 
 }   // namespace ath

@@ -13,6 +13,8 @@
 // those records' power and alpha exactly as the forward did (this file is built
 // with --fmad=false), so it skips the same records, and divides the
 // transmittance back out record by record.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "adjoint.cuh"
@@ -208,23 +210,122 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
     }
 }
 
-// The projection's adjoint, one thread a Gaussian: dL/d(record) -> dL/d(parameters), added in.
-__global__ void __launch_bounds__(128)
-    projectBackwardKernel(const FrameConst F, const InstanceConst I, const uint32_t* __restrict__ keys,
-                          const float* __restrict__ grads, float4* __restrict__ gMeans, float4* __restrict__ gScales,
-                          float4* __restrict__ gQuats, float* __restrict__ gSh) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= I.count) return;
-    const uint32_t slot = I.base + i;
-    if (keys[slot] >= kCulledKey) return;
-    const float* gr = grads + (size_t)slot * kGradWords;
-    float gw[kGradWords];
+// The slots whose records took a gradient, in `list` (their number in *listed, which starts
+// at zero): most records of a frame lie behind their pixels' early stop, or in no pixel's
+// footprint, and take none.
+__global__ void __launch_bounds__(256)
+    listGradientsKernel(uint32_t slots, const uint32_t* __restrict__ keys, const float* __restrict__ grads,
+                        uint32_t* __restrict__ list, uint32_t* __restrict__ listed) {
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    bool some = false;
+    if (slot < slots && keys[slot] < kCulledKey) {
+        const float2* g = reinterpret_cast<const float2*>(grads + (size_t)slot * kGradWords);
 #pragma unroll
-    for (int k = 0; k < (int)kGradWords; ++k) gw[k] = gr[k];
-    ParamGrad acc;
-    acc.clear();
-    projectAdjoint<kLayoutParams>(F, I, i, gw, acc);
-    acc.addTo(i, I.shStride, gMeans, gScales, gQuats, gSh);
+        for (uint32_t k = 0; k < kGradWords / 2; ++k) {
+            const float2 v = g[k];
+            some = some || v.x != 0.0f || v.y != 0.0f;
+        }
+    }
+    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, some);
+    uint32_t first = 0;
+    if (lane == 0 && ballot) first = atomicAdd(listed, (uint32_t)__popc(ballot));
+    first = __shfl_sync(0xFFFFFFFFu, first, 0);
+    if (some) list[first + __popc(ballot & ((1u << lane) - 1u))] = slot;
+}
+
+// The projection's adjoint, one thread a listed Gaussian: dL/d(record) -> dL/d(parameters),
+// added in. A warp brings its 32 SH rows into shared memory a row at a time (stride 49:
+// lane l's value k at bank (17 l + k) mod 32), each thread puts its gradient in its row's
+// place, and the warp adds the rows to the gradients a row at a time: every access covers
+// whole sectors, where a lane at its own row touched a line a load.
+// Over every slot in order, each thread its own rows: 500k Gaussians at 1280x720, degree 3,
+// 308 us; the list 14 and this 49.
+constexpr uint32_t kRowsAtOnce = 8;   // of rows that are not whole pieces
+
+__global__ void __launch_bounds__(128)
+    projectBackwardKernel(const FrameConst F, const InstanceConst I, const uint32_t* __restrict__ list,
+                          const uint32_t* __restrict__ listed, const float* __restrict__ grads,
+                          float4* __restrict__ gMeans, float4* __restrict__ gScales, float4* __restrict__ gQuats,
+                          float* __restrict__ gSh) {
+    __shared__ float sSh[4][32 * 49];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t count = min(*listed, I.count);
+    const uint32_t degree = min(degreeOf(I.restPerColour), F.shLimit);
+    const uint32_t bases = degree >= 3 ? 15u : degree == 2 ? 8u : degree == 1 ? 3u : 0u;
+    const uint32_t cols = 3u + 3u * bases;   // past the degree's the gradient is zero
+    const bool aligned = cols % 4 == 0 && I.shStride % 4 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(I.shf) | reinterpret_cast<uintptr_t>(gSh)) & 15u) == 0;
+    const uint32_t quads = aligned ? cols / 4 : 0u;   // 12 at degree 3, 3 at degree 1; 27 and 3 values are not whole pieces
+    for (uint32_t k0 = (blockIdx.x * 4 + warp) * 32; k0 < count; k0 += gridDim.x * 128) {
+        const bool active = k0 + lane < count;
+        const uint32_t rows = min(32u, count - k0);
+        const uint32_t slot = active ? list[k0 + lane] : I.base, i = slot - I.base;
+        // the warp's rows `quads` 16-byte pieces each where they are aligned so, a lane a piece,
+        // several in flight; else some rows at a time, a lane a value
+        const uint32_t pieces = rows * quads;
+        if (quads) {
+#pragma unroll 6
+            for (uint32_t k = 0; k < 12; ++k) {
+                const uint32_t at = min(k * 32 + lane, pieces - 1u), r = at / quads, q = at % quads;
+                const uint32_t ri = __shfl_sync(0xFFFFFFFFu, i, r);
+                if (k * 32 < pieces) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(I.shf + (size_t)ri * I.shStride) + q);
+                    float* to = sSh[warp] + r * 49 + 4 * q;
+                    to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w;
+                }
+            }
+        } else {
+            for (uint32_t r0 = 0; r0 < rows; r0 += kRowsAtOnce)
+                for (uint32_t c = lane; c < cols; c += 32) {
+                    float v[kRowsAtOnce];
+#pragma unroll
+                    for (uint32_t k = 0; k < kRowsAtOnce; ++k)
+                        if (r0 + k < rows) v[k] = __ldg(I.shf + (size_t)(list[k0 + r0 + k] - I.base) * I.shStride + c);
+#pragma unroll
+                    for (uint32_t k = 0; k < kRowsAtOnce; ++k)
+                        if (r0 + k < rows) sSh[warp][(r0 + k) * 49 + c] = v[k];
+                }
+        }
+        __syncwarp();
+        if (active) {
+            const float* gr = grads + (size_t)slot * kGradWords;
+            float gw[kGradWords];
+#pragma unroll
+            for (int k = 0; k < (int)kGradWords; ++k) gw[k] = gr[k];
+            ParamGrad acc;
+            acc.clear();
+            projectAdjoint(F, I, i, degree, bases, gw, sSh[warp] + lane * 49, acc);
+            acc.addGeometryTo(i, gMeans, gScales, gQuats);
+        }
+        __syncwarp();
+        if (quads) {
+#pragma unroll 6
+            for (uint32_t k = 0; k < 12; ++k) {
+                const uint32_t at = min(k * 32 + lane, pieces - 1u), r = at / quads, q = at % quads;
+                const uint32_t ri = __shfl_sync(0xFFFFFFFFu, i, r);
+                if (k * 32 + lane < pieces) {
+                    float4* to = reinterpret_cast<float4*>(gSh + (size_t)ri * I.shStride) + q;
+                    const float* add = sSh[warp] + r * 49 + 4 * q;
+                    float4 v = *to;
+                    v.x += add[0]; v.y += add[1]; v.z += add[2]; v.w += add[3];
+                    *to = v;
+                }
+            }
+        } else {
+            for (uint32_t r0 = 0; r0 < rows; r0 += kRowsAtOnce)
+                for (uint32_t c = lane; c < cols; c += 32) {
+                    float v[kRowsAtOnce];
+#pragma unroll
+                    for (uint32_t k = 0; k < kRowsAtOnce; ++k)
+                        if (r0 + k < rows) v[k] = gSh[(size_t)(list[k0 + r0 + k] - I.base) * I.shStride + c];
+#pragma unroll
+                    for (uint32_t k = 0; k < kRowsAtOnce; ++k)
+                        if (r0 + k < rows)
+                            gSh[(size_t)(list[k0 + r0 + k] - I.base) * I.shStride + c] = v[k] + sSh[warp][(r0 + k) * 49 + c];
+                }
+        }
+        __syncwarp();
+    }
 }
 
 // L = mean over pixels and r g b of (colour - target)^2: its value (added into
@@ -277,10 +378,12 @@ cudaError_t launchBlendBackward(const FrameConst& F, uint32_t pairs, uint32_t sl
 }
 
 cudaError_t launchProjectBackward(const FrameConst& F, const InstanceConst& I, const uint32_t* keys,
-                                  const float* grads, float4* gMeans, float4* gScales, float4* gQuats, float* gSh,
-                                  cudaStream_t stream) {
+                                  const float* grads, uint32_t* list, uint32_t* listed, float4* gMeans, float4* gScales,
+                                  float4* gQuats, float* gSh, int sms, cudaStream_t stream) {
     if (I.count == 0) return cudaSuccess;
-    projectBackwardKernel<<<(I.count + 127) / 128, 128, 0, stream>>>(F, I, keys, grads, gMeans, gScales, gQuats, gSh);
+    listGradientsKernel<<<(I.count + 255) / 256, 256, 0, stream>>>(I.base + I.count, keys, grads, list, listed);
+    const uint32_t blocks = std::min((I.count + 127) / 128, (uint32_t)sms * 4);   // four an SM by its registers
+    projectBackwardKernel<<<blocks, 128, 0, stream>>>(F, I, list, listed, grads, gMeans, gScales, gQuats, gSh);
     return cudaGetLastError();
 }
 

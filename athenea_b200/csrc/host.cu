@@ -820,8 +820,10 @@ extern "C" ath_status ath_raster_backward(ath_raster* r, const float* dlDcolour,
     const FrameConst& F = r->lastFrame;
     const InstanceConst& I = r->trainingInstance;
     const uint32_t slots = r->lastSlots;
-    cudaError_t err = r->grads.reserve((size_t)std::max(slots, 1u) * kGradWords * sizeof(float));
-    if (err == cudaSuccess) err = cudaMemsetAsync(r->grads.ptr, 0, (size_t)slots * kGradWords * sizeof(float), stream);
+    // the records' gradients, then the number of those that took one
+    const size_t gradBytes = (size_t)slots * kGradWords * sizeof(float);
+    cudaError_t err = r->grads.reserve(gradBytes + sizeof(uint32_t));
+    if (err == cudaSuccess) err = cudaMemsetAsync(r->grads.ptr, 0, gradBytes + sizeof(uint32_t), stream);
     uint32_t* words = static_cast<uint32_t*>(r->zeroed.ptr);
     if (err == cudaSuccess)
         err = launchBlendBackward(F, r->pairCapacity, slots, r->ranges,
@@ -831,8 +833,10 @@ extern "C" ath_status ath_raster_backward(ath_raster* r, const float* dlDcolour,
                                   static_cast<float*>(r->grads.ptr), words + kWordSticky, stream);
     if (err == cudaSuccess)
         err = launchProjectBackward(F, I, static_cast<const uint32_t*>(r->keys.ptr), static_cast<const float*>(r->grads.ptr),
+                                    static_cast<uint32_t*>(r->depthKeys[0].ptr),   // spare after the depth sort
+                                    reinterpret_cast<uint32_t*>(static_cast<char*>(r->grads.ptr) + gradBytes),
                                     reinterpret_cast<float4*>(grads->means), reinterpret_cast<float4*>(grads->scales),
-                                    reinterpret_cast<float4*>(grads->quats), grads->sh, stream);
+                                    reinterpret_cast<float4*>(grads->quats), grads->sh, r->sms, stream);
     // the frame's words again, with what the backward raised, for ath_raster_check
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(r->statusHost.ptr, words, kFrameWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);

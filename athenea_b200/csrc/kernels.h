@@ -123,9 +123,10 @@ cudaError_t launchBlendBackward(const FrameConst& F, uint32_t pairs, uint32_t sl
                                 const uint64_t* sorted, const float4* recs, const TrainingState& training,
                                 const float4* dLdColour, const float* dLdDepth,
                                 const float* depthOut, float* grads, uint32_t* status, cudaStream_t stream);
+// list: room for a slot each; *listed: zeroed by the caller.
 cudaError_t launchProjectBackward(const FrameConst& F, const InstanceConst& I, const uint32_t* keys,
-                                  const float* grads, float4* gMeans, float4* gScales, float4* gQuats, float* gSh,
-                                  cudaStream_t stream);
+                                  const float* grads, uint32_t* list, uint32_t* listed, float4* gMeans, float4* gScales,
+                                  float4* gQuats, float* gSh, int sms, cudaStream_t stream);
 cudaError_t launchL2Loss(const float4* colour, const float* target, uint32_t pixels, float4* dLdColour, float* loss,
                          cudaStream_t stream);
 

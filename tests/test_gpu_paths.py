@@ -82,3 +82,37 @@ def test_calls_agree_with_64_bits(native, case):
         g, w = got[name].double().reshape(-1), value.double().reshape(-1)
         rel = float((g - w).norm() / w.norm())
         assert rel <= (1e-3 if name in ("colour", "loss") else 1e-2), (name, rel)
+
+
+# SH rows that are not whole 16-byte pieces (a stride of 49, a base 4 bytes off) take the values one at a time: the
+# same gradients, to the order of the atomic sums
+@pytest.mark.parametrize("stride,shift", [(48, 0), (49, 0), (48, 1), (52, 0)])
+def test_gradients_do_not_depend_on_the_rows_layout(native, stride, shift):
+    W, H, n = 320, 200, 5003
+    p = scenes.params(n, True, 7, 3)
+    base = A.Params(*[torch.from_numpy(np.ascontiguousarray(p[k])).cuda() for k in ("means", "scales", "quats", "sh")], 3)
+
+    def rows(values):
+        flat = torch.zeros(n * stride + shift, device="cuda")
+        out = flat[shift:].view(n, stride)
+        out[:, :48] = values
+        return out
+
+    def step(params, grads):
+        r, t = A.TileRasterizer.create(), A.RenderTargets.make(W, H)
+        cam = A.pinhole_for_vertical_fov((0, 0, 3), (0, 0, 0), W, H, 60.0).projection_for(W, H)
+        r.render_params(cam, params, A.RenderSettings(width=W, height=H), t)
+        r.backward(torch.ones_like(t.colour), grads)
+        return t.colour
+
+    want = base.zeros_like()
+    image = step(base, want)
+    mine = A.Params(base.means, base.scales, base.quats, rows(base.sh), 3)
+    grads = A.Params(torch.zeros_like(base.means), torch.zeros_like(base.scales), torch.zeros_like(base.quats),
+                     rows(torch.full((n, 48), 0.25, device="cuda")), 3)
+    assert torch.equal(step(mine, grads), image)
+    assert torch.allclose(grads.sh[:, :48] - 0.25, want.sh, rtol=1e-4, atol=1e-5 * float(want.sh.abs().max()))
+    assert torch.equal(grads.sh[:, 48:], torch.zeros_like(grads.sh[:, 48:]))
+    for name in ("means", "scales", "quats"):
+        a, b = getattr(grads, name), getattr(want, name)
+        assert torch.allclose(a, b, rtol=1e-3, atol=1e-5 * float(b.abs().max())), name
