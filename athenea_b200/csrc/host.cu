@@ -340,6 +340,9 @@ extern "C" void ath_raster_destroy(ath_raster* r) {
     delete r;
 }
 
+namespace {
+void trimCallScratch();
+}
 extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     if (!r) return fail(ATH_E_INVALID_ARGUMENT, "ath_raster_release_scratch: null handle");
     DeviceGuard guard(r->device);
@@ -355,6 +358,7 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     r->ranges = nullptr;
     r->instanceStage.clear();
     r->instanceStage.shrink_to_fit();
+    trimCallScratch();
     return ATH_OK;
 }
 
@@ -986,6 +990,50 @@ extern "C" ath_status ath_sorter_check(ath_sorter* s) {
 }
 
 // ---- decode -----------------------------------------------------------------
+namespace {
+
+// Device memory of a call that waits for its own end. Up to kKept bytes stay with the
+// calling thread for its next call (until it ends, or gives scratch back with
+// ath_raster_release_scratch), so that a call does not pay for cudaMalloc and cudaFree,
+// which map memory and wait for the device; more than that is the call's alone. As the call
+// waits, nothing of it is in use when the next one takes the memory, on whatever stream.
+class CallScratch {
+public:
+    cudaError_t reserve(size_t bytes) {
+        int device = 0;
+        cudaError_t err = cudaGetDevice(&device);
+        if (err != cudaSuccess) return err;
+        if (bytes > kKept) {
+            err = own_.reserve(bytes);
+            ptr = own_.ptr;
+            return err;
+        }
+        if (kept().device != device) kept().buffer.release();
+        kept().device = device;
+        err = kept().buffer.reserve(bytes);
+        ptr = kept().buffer.ptr;
+        return err;
+    }
+    static void trim() { kept().buffer.release(); }
+    void* ptr = nullptr;
+
+private:
+    static constexpr size_t kKept = 1u << 20;
+    struct Kept {
+        DeviceBuffer buffer;
+        int device = -1;
+    };
+    static Kept& kept() {
+        static thread_local Kept k;
+        return k;
+    }
+    DeviceBuffer own_;
+};
+
+void trimCallScratch() { CallScratch::trim(); }
+
+}   // namespace
+
 extern "C" ath_status ath_decode_records(const float* records, uint32_t count, const ath_encoding* encoding,
                                          float* positions, uint32_t* shape, uint32_t* sh, uint32_t* kept,
                                          void* streamPtr) {
@@ -1005,21 +1053,19 @@ extern "C" ath_status ath_decode_records(const float* records, uint32_t count, c
     *kept = 0;
     if (count == 0) return ATH_OK;
     cudaStream_t stream = static_cast<cudaStream_t>(streamPtr);
-    DeviceBuffer flags, words;
-    PinnedBuffer host;
-    cudaError_t err = flags.reserve((size_t)decodeBlocks(count) * 8);
-    if (err == cudaSuccess) err = words.reserve(4 * sizeof(uint32_t));
-    if (err == cudaSuccess) err = host.reserve(4 * sizeof(uint32_t));
-    if (err == cudaSuccess) err = cudaMemsetAsync(flags.ptr, 0, (size_t)decodeBlocks(count) * 8, stream);
-    if (err == cudaSuccess) err = cudaMemsetAsync(words.ptr, 0, 4 * sizeof(uint32_t), stream);
+    // the look-back words, then the kernel's ticket, status and count
+    const size_t flagBytes = (size_t)decodeBlocks(count) * 8, bytes = flagBytes + 4 * sizeof(uint32_t);
+    CallScratch scratch;
+    uint32_t w[4] = {};
+    cudaError_t err = scratch.reserve(bytes);
+    uint32_t* words = reinterpret_cast<uint32_t*>(static_cast<char*>(scratch.ptr) + flagBytes);
+    if (err == cudaSuccess) err = cudaMemsetAsync(scratch.ptr, 0, bytes, stream);
     if (err == cudaSuccess)
         err = launchDecode(records, count, e, reinterpret_cast<float4*>(positions), reinterpret_cast<uint4*>(shape), sh,
-                           static_cast<uint64_t*>(flags.ptr), static_cast<uint32_t*>(words.ptr), stream);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(host.ptr, words.ptr, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+                           static_cast<uint64_t*>(scratch.ptr), words, stream);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(w, words, sizeof(w), cudaMemcpyDeviceToHost, stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) return failCuda(err, "decoding the records");
-    const uint32_t* w = static_cast<const uint32_t*>(host.ptr);
     if (w[1] & kStatusLookbackTimeout) return fail(ATH_E_TIMEOUT, "the decode's compaction gave up waiting");
     if (w[1] & kStatusIndexRange) return fail(ATH_E_INTERNAL, "the decode's compaction went outside its buffers");
     *kept = w[2];

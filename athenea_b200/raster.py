@@ -156,7 +156,7 @@ class CloudLoader:
         dev = records.device
         positions = torch.empty((max(count, 1), 4), dtype=torch.float32, device=dev)
         shape = torch.empty((max(count, 1), 4), dtype=torch.int32, device=dev)
-        sh = torch.zeros((max(count, 1), sh_words), dtype=torch.int32, device=dev)
+        sh = torch.empty((max(count, 1), sh_words), dtype=torch.int32, device=dev)
         e = N.Encoding(keep_per_colour=keep, **{k: encoding[k] for k in (
             "stride", "x", "y", "z", "opacity", "scale0", "scale1", "scale2", "rot_w", "rot_x", "rot_y", "rot_z",
             "dc0", "dc1", "dc2", "rest_base", "file_per_colour")})
@@ -165,6 +165,8 @@ class CloudLoader:
         check(N.lib().ath_decode_records(_ptr(records.contiguous()), count, C.byref(e), _ptr(positions),
                                          _ptr(shape), _ptr(sh), C.byref(kept), C.c_void_p(s.cuda_stream)))
         n = kept.value
+        if n == 0:
+            sh.zero_()   # the row an empty cloud keeps
         return GpuSplats(positions[:max(n, 1)], shape[:max(n, 1)], sh[:max(n, 1)], n, keep, sh_words, linear)
 
 

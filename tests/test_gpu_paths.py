@@ -58,6 +58,22 @@ def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(native, raster)
     assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
 
 
+# strides whose records' 16-byte pieces end in the middle, that fill shared memory, and that do not fit it;
+# counts around a warp and a block
+@pytest.mark.parametrize("pad,shift", [(0, 1), (1, 0), (2, 3), (330, 0), (600, 0)])
+@pytest.mark.parametrize("count", [1, 31, 33, 128, 1291])
+def test_decode_takes_any_stride_and_base(native, count, pad, shift):
+    records, enc = cases._records(cases._file(dict(count=count, degree=3), 3))
+    want = A.CloudLoader.upload(records, enc)
+    stride = enc["stride"] + pad
+    flat = torch.full((count * stride + shift,), 7.0, device="cuda")
+    flat[shift:].view(count, stride)[:, :enc["stride"]] = records
+    got = A.CloudLoader.upload(flat[shift:], dict(enc, stride=stride))
+    assert got.count == want.count
+    for name in ("positions", "shape", "sh"):
+        assert torch.equal(getattr(got, name)[:want.count], getattr(want, name)[:want.count]), name
+
+
 # A pixel whose walk takes a decision near its threshold (about 1 in 500) may take it the other way in 64 bits: a
 # splat of alpha 1/255 in or out. Images then agree to 1/255 / sqrt(500) = 2e-4 of their norm, gradients, which such a
 # splat's are few of but whole, to 1e-2.
