@@ -252,9 +252,8 @@ __device__ __forceinline__ bool footprintTouches(float4 fa, float4 fb, bool wide
     const float lx = ((float)(tx * T) + 0.5f) - fa.x, ly = ((float)(ty * T) + 0.5f) - fa.y;
     const float hx = ((float)(min((tx + 1) * T, width) - 1) + 0.5f) - fa.x;
     const float hy = ((float)(min((ty + 1) * T, height) - 1) + 0.5f) - fa.y;
-    const float best = wide ? minPowerOverBoxFactored(fa.z, fa.w, fb.x, fb.z, fb.w, lx, ly, hx, hy)
-                            : minPowerOverBox(fa.z, fa.w, fb.x, lx, ly, hx, hy);
-    return best <= fb.y;
+    return wide ? minPowerOverBoxFactored(fa.z, fa.w, fb.x, fb.z, fb.w, lx, ly, hx, hy) <= fb.y
+                : powerWithin(fa.z, fa.w, fb.x, fb.y, lx, ly, hx, hy);
 }
 
 // The least lane k whose inclusive sum `incl` passes q (q below the warp's total).
@@ -307,6 +306,7 @@ __global__ void __launch_bounds__(kProjThreads, 5)   // five blocks an SM: the k
         F.width = sView.width; F.height = sView.height; F.tilesX = sView.tilesX; F.tilesY = sView.tilesY;
         F.focalX = sView.focalX; F.focalY = sView.focalY; F.centreX = sView.centreX; F.centreY = sView.centreY;
         F.nearZ = sView.nearZ; F.farZ = sView.farZ; F.orthographic = sView.orthographic; F.shLimit = B.shLimit;
+        F.limLoX = sView.limLoX; F.limHiX = sView.limHiX; F.limLoY = sView.limLoY; F.limHiY = sView.limHiY;
         sF = F;
     }
     __syncthreads();
@@ -784,6 +784,7 @@ __global__ void __launch_bounds__(128)
         F.width = V.width; F.height = V.height; F.tilesX = V.tilesX; F.tilesY = V.tilesY;
         F.focalX = V.focalX; F.focalY = V.focalY; F.centreX = V.centreX; F.centreY = V.centreY;
         F.nearZ = V.nearZ; F.farZ = V.farZ; F.orthographic = V.orthographic; F.shLimit = B.shLimit;
+        F.limLoX = V.limLoX; F.limHiX = V.limHiX; F.limLoY = V.limLoY; F.limHiY = V.limHiY;
 #pragma unroll
         for (int k = 0; k < 12; ++k) I.m[k] = V.m[k];
         I.eye[0] = V.eye[0]; I.eye[1] = V.eye[1]; I.eye[2] = V.eye[2];
@@ -912,6 +913,7 @@ ath_status buildViews(ath_batch* b) {
         const FrameConst F = frameConstFor(p, s);
         V.focalX = F.focalX; V.focalY = F.focalY; V.centreX = F.centreX; V.centreY = F.centreY;
         V.nearZ = F.nearZ; V.farZ = F.farZ; V.orthographic = F.orthographic;
+        V.limLoX = F.limLoX; V.limHiX = F.limHiX; V.limLoY = F.limLoY; V.limHiY = F.limHiY;
         V.tileBase = tileBase;
         V.pixelBase = pixelBase;
         V.lossScale = 1.0f / (3.0f * (float)V.width * (float)V.height);

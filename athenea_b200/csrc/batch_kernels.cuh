@@ -15,6 +15,7 @@ namespace ath {
 struct BatchView {
     uint32_t width, height, tilesX, tilesY;
     float focalX, focalY, centreX, centreY, nearZ, farZ;
+    float limLoX, limHiX, limLoY, limHiY;   // FrameConst's
     uint32_t orthographic;
     uint32_t tileBase;    // its first tile among all views' tiles
     uint32_t pixelBase;   // its first pixel in the concatenated images

@@ -255,15 +255,11 @@ __device__ __forceinline__ Geometry projectGeometry(const FrameConst& F, const I
         const float invZ = 1.0f / G.tz;
         G.cx = (F.focalX * G.tx) * invZ + F.centreX;
         G.cy = (F.focalY * G.ty) * invZ + F.centreY;
-        const float limLoX = ((-0.15f) * (float)F.width - F.centreX) / F.focalX;
-        const float limHiX = (1.15f * (float)F.width - F.centreX) / F.focalX;
-        const float limLoY = ((-0.15f) * (float)F.height - F.centreY) / F.focalY;
-        const float limHiY = (1.15f * (float)F.height - F.centreY) / F.focalY;
         const float ux = G.tx * invZ, uy = G.ty * invZ;
-        G.clampX = ux < limLoX || ux > limHiX;
-        G.clampY = uy < limLoY || uy > limHiY;
-        G.txc = clampf(ux, limLoX, limHiX) * G.tz;
-        G.tyc = clampf(uy, limLoY, limHiY) * G.tz;
+        G.clampX = ux < F.limLoX || ux > F.limHiX;
+        G.clampY = uy < F.limLoY || uy > F.limHiY;
+        G.txc = clampf(ux, F.limLoX, F.limHiX) * G.tz;
+        G.tyc = clampf(uy, F.limLoY, F.limHiY) * G.tz;
         G.jx0 = F.focalX * invZ;
         G.jx2 = (((-F.focalX) * G.txc) * invZ) * invZ;
         G.jy1 = F.focalY * invZ;

@@ -243,6 +243,7 @@ FrameConst frameConstFor(const ath_projection& p, const ath_settings& s) {
     F.centreY = (float)p.centre_y;
     F.nearZ = (float)p.near_z;
     F.farZ = (float)p.far_z;
+    frustumLimits(F);
     F.orthographic = p.orthographic ? 1u : 0u;
     F.tileBits = bitsFor(F.tilesX * F.tilesY);
     F.shLimit = s.max_sh_degree;

@@ -18,11 +18,22 @@ struct EditConst {
 struct FrameConst {
     uint32_t width, height, tilesX, tilesY;
     float focalX, focalY, centreX, centreY, nearZ, farZ;
+    float limLoX, limHiX, limLoY, limHiY;   // the frustum's 1.3x, as x / z and y / z (frustumLimits)
     uint32_t orthographic, tileBits, shLimit, depthMode;
     float depthThreshold;
     float bg[4];
     float viewToWorld[12];   // rows of the view -> world 3x4, for P
 };
+
+// The Jacobian's limits (splat_project.slang:566-571), once a frame or view in the
+// projection's own 32-bit operations: four divisions fewer a splat.
+template <typename T>
+inline void frustumLimits(T& F) {
+    F.limLoX = ((-0.15f) * (float)F.width - F.centreX) / F.focalX;
+    F.limHiX = (1.15f * (float)F.width - F.centreX) / F.focalX;
+    F.limLoY = ((-0.15f) * (float)F.height - F.centreY) / F.focalY;
+    F.limHiY = (1.15f * (float)F.height - F.centreY) / F.focalY;
+}
 
 // The per-instance part (setObject, setCloudSpace, setEdit: FrameParams.h:84-165),
 // with the cloud's device buffers in one of the layouts of gauss.cuh.
