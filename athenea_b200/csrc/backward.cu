@@ -45,14 +45,14 @@ __device__ __forceinline__ float reciprocal(float x) {
 // One block a tile, its warps independent, a box of pixels each, as the forward
 // (walk.cuh). A warp gathers the records its box blended (the forward's live bits), last
 // first, 32 at a time into slots of its own, and walks them down from its pixels' last
-// contributor. A lane sums its pixels' terms (two pixels share their dy, so the moments
-// of dL/dpower in dy are formed once for both), the warp its lanes' through columns in
-// shared memory, kRecords records at a time: lane k then adds column k's sum into that
-// record's word in global memory.
+// contributor. A lane sums its pixels' terms, the warp its lanes' through columns in
+// shared memory, kRecords records at a time: lane k then sums column k and adds what it
+// gives into that record's words in global memory. The moments in dy come from the
+// columns' row sums (walk.cuh's rowSums).
 //
 // Bound by instruction issue. Against one thread a pixel over every record of the tile
 // up to its last contributor, ten values summed by shuffles a record and warp, then
-// through shared memory by atomics: 0.30 ms for 500k Gaussians at 1280x720 (0.71), 75 us
+// through shared memory by atomics: 0.28 ms for 500k Gaussians at 1280x720 (0.71), 75 us
 // for 20k at 333x251 (201).
 template <int kPx, bool kDepth>
 __global__ void __launch_bounds__(Box<kPx>::kThreads)
@@ -61,12 +61,13 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                         const TrainingState training, const float4* __restrict__ dLdColour,
                         const float* __restrict__ dLdDepth, const float* __restrict__ depthOut,
                         float* __restrict__ grads, uint32_t* __restrict__ status) {
-    constexpr uint32_t kWords = kDepth ? 10 : 9;          // the view z's word last
-    constexpr uint32_t kRecords = kPx == 2 ? 3 : 2;       // kRecords * kWords lanes sum a column each
-    static_assert(kRecords * kWords <= 32 && kGradZ == 9, "a column a lane");
+    // of alpha dL/dalpha: its sum, its moments dx and dx dx; dL/dcolour r g b; dL/dz
+    constexpr uint32_t kValues = kDepth ? 7 : 6;
+    constexpr uint32_t kRecords = kPx == 2 ? 4 : 3;       // kRecords * kValues lanes sum a column each
+    static_assert(kRecords * kValues <= 32, "a column a lane");
     struct Shared {
         WalkRecord<kPx> records[32];
-        float sums[kRecords * kWords * kColumnStride];
+        float sums[kRecords * kValues * kColumnStride];
     };
     __shared__ Shared sShared[Box<kPx>::kCount];
     const uint32_t tile = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -111,7 +112,8 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         }
         most = max(most, last[p]);
     }
-    const uint32_t sumRecord = lane / kWords, sumWord = lane % kWords;   // the column this lane sums
+    const uint32_t sumRecord = lane / kValues, sumValue = lane % kValues;   // the column this lane sums
+    const float rowMid = (float)boxY + 0.5f * (float)Box<kPx>::kHeight;      // the box's middle row
     const int32_t chunks = (int32_t)((__reduce_max_sync(0xFFFFFFFFu, most) + 31u) >> 5);
     const uint32_t* liveOf = training.live + ((size_t)(range.x >> 5) + tile) * Box<kPx>::kCount + warp;
     for (int32_t hi = chunks - 1; hi >= 0; hi -= 32) {
@@ -140,13 +142,16 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 sh.records[lane].set(recs[(size_t)s * 3 + 0], recs[(size_t)s * 3 + 1], recs[(size_t)s * 3 + 2], s, rel + 1u);
             }
             __syncwarp();
+            const bool odd = __any_sync(0xFFFFFFFFu, lane < count && sh.records[lane].odd != 0u);
+            auto walk = [&](auto oddHere) {
+            constexpr bool kOdd = decltype(oddHere)::value;
             for (uint32_t q0 = 0; q0 < count; q0 += kRecords) {
                 const uint32_t batch = min(kRecords, count - q0);
                 float* column = sh.sums + lane;
-                for (uint32_t q = q0; q < q0 + batch; ++q, column += kWords * kColumnStride) {
+                for (uint32_t q = q0; q < q0 + batch; ++q, column += kValues * kColumnStride) {
                     using Rec = WalkRecord<kPx>;
                     const Rec& R = sh.records[q];
-                    const WalkPoint<kPx> at(R, xc, yc);
+                    const WalkPoint<kPx, kOdd> at(R, xc, yc);
                     Px<kPx> alpha, inv;
                     bool on[kPx];
 #pragma unroll
@@ -167,7 +172,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     Px<kPx> cd = fused(Rec::px(R.bl), dB, fused(Rec::px(R.g), dG, Rec::px(R.r) * dR));
                     if (kDepth) cd = fused(Rec::px(R.z), dDepth, cd);
                     Px<kPx> u = fused(sd, both<kPx>(-1.0f), cd);
-                    if (R.odd) {   // a colour that is not finite stays out of the pixels that did not blend it
+                    if (kOdd && R.odd) {   // a colour that is not finite stays out of the pixels that did not blend it
 #pragma unroll
                         for (int p = 0; p < kPx; ++p)
                             if (!on[p]) u.v[p] = 0.0f;
@@ -181,31 +186,47 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     for (int p = 0; p < kPx; ++p)
                         if (!(at.raw.v[p] < 0.99f && R.alpha[0] <= 1.0f)) aDA.v[p] = 0.0f;
                     const Px<kPx> x1 = aDA * at.dx, x2 = x1 * at.dx;
-                    const Px<kPx> wr = w * dR, wg = w * dG, wb = w * dB;
                     auto sum = [](const Px<kPx>& v) { return kPx == 2 ? v.v[0] + v.v[kPx - 1] : v.v[0]; };
-                    // the moments of dL/dpower = -1/2 alpha dL/dalpha over (dx, dy), then the centre's
-                    // and the conic's gradients
-                    const float dy = at.dy.v[0], m0 = sum(aDA), mx = -0.5f * sum(x1), my = -0.5f * (m0 * dy);
-                    column[kGradCx * kColumnStride] = -__fmaf_rn(2.0f * R.a[0], mx, R.b2[0] * my);
-                    column[kGradCy * kColumnStride] = -__fmaf_rn(R.b2[0], mx, (2.0f * R.c[0]) * my);
-                    column[kGradA * kColumnStride] = -0.5f * sum(x2);
-                    column[kGradB2 * kColumnStride] = 2.0f * (mx * dy);
-                    column[kGradC * kColumnStride] = my * dy;
-                    column[kGradAlpha * kColumnStride] = m0;
-                    column[kGradR * kColumnStride] = sum(wr);
-                    column[kGradG * kColumnStride] = sum(wg);
-                    column[kGradB * kColumnStride] = sum(wb);
-                    if (kDepth) column[kGradZ * kColumnStride] = sum(w * dDepth);
+                    column[0 * kColumnStride] = sum(aDA);
+                    column[1 * kColumnStride] = sum(x1);
+                    column[2 * kColumnStride] = sum(x2);
+                    column[3 * kColumnStride] = sum(w * dR);
+                    column[4 * kColumnStride] = sum(w * dG);
+                    column[5 * kColumnStride] = sum(w * dB);
+                    if (kDepth) column[6 * kColumnStride] = sum(w * dDepth);
                 }
                 __syncwarp();
-                if (lane < batch * kWords) {
-                    const WalkRecord<kPx>& R = sh.records[q0 + sumRecord];
-                    float v = columnSum(sh.sums + lane * kColumnStride);
-                    if (sumWord == kGradAlpha) v = v / R.alpha[0];
-                    if (v != 0.0f) atomicAdd(&grads[(size_t)R.slot * kGradWords + sumWord], v);
+                // dL/dpower is -1/2 alpha dL/dalpha; its moments over (dx, dy) give the centre's and
+                // the conic's gradients, the centre's x and y both in the lane of the moment dx
+                const bool mine = lane < batch * kValues;
+                RowSums v{0.0f, 0.0f, 0.0f};
+                if (mine) v = rowSums<(int)Box<kPx>::kHeight>(sh.sums + lane * kColumnStride);
+                const WalkRecord<kPx>& R = sh.records[q0 + min(sumRecord, batch - 1u)];
+                const float dy = rowMid + R.ny[0];
+                const float overRows = __fmaf_rn(dy, v.sum, v.first);   // dy, or dx dy
+                const float my = __shfl_up_sync(0xFFFFFFFFu, overRows, 1);
+                if (mine) {
+                    float* words = grads + (size_t)R.slot * kGradWords;
+                    auto add = [&](uint32_t word, float value) {
+                        if (value != 0.0f) atomicAdd(words + word, value);
+                    };
+                    if (sumValue == 0) {
+                        add(kGradAlpha, v.sum / R.alpha[0]);
+                        add(kGradC, -0.5f * __fmaf_rn(dy, __fmaf_rn(dy, v.sum, 2.0f * v.first), v.second));
+                    } else if (sumValue == 1) {
+                        add(kGradCx, __fmaf_rn(R.a[0], v.sum, 0.5f * R.b2[0] * my));
+                        add(kGradCy, __fmaf_rn(0.5f * R.b2[0], v.sum, R.c[0] * my));
+                        add(kGradB2, -overRows);
+                    } else {
+                        add(sumValue == 2 ? (uint32_t)kGradA : (uint32_t)kGradR + sumValue - 3u,
+                            sumValue == 2 ? -0.5f * v.sum : v.sum);
+                    }
                 }
                 __syncwarp();   // the next records overwrite the columns
             }
+            };
+            if (odd) walk(std::true_type());
+            else walk(std::false_type());
         }
     }
 }

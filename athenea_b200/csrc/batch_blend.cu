@@ -22,44 +22,35 @@ constexpr uint32_t kBox = 8;
 // and a span whose pixels are done stops staging the tile's records.
 constexpr uint32_t kBlendSpan = 16;
 
-// The footprint's half extents from the factored conic: the covariance's
-// diagonal a' = cutoff (1/ca + fr^2/fs) and c' = cutoff / fs.
-__device__ __forceinline__ void footprintExtent(float ca, float fr, float fs, float cutoff, float& ex, float& ey) {
-    ex = ca > 0.0f && fs > 0.0f ? sqrtf(cutoff * (1.0f / ca + (fr * fr) / fs)) * 1.0001f + 1e-3f : 3.4e38f;
-    ey = fs > 0.0f ? sqrtf(cutoff / fs) * 1.0001f + 1e-3f : 3.4e38f;
-}
-
-// Bit b set when box b of the tile (boxes row-major, T/8 a row) may hold a pixel
-// centre inside the footprint: among the boxes whose pixel-centre columns and
-// rows overlap the footprint's bounding box [cx - ex, cx + ex] x [cy - ey, cy + ey],
-// those whose least power (minPowerOverBoxFactored) is within the cutoff.
-// Conservative: extents and cutoff carry a margin over the per-pixel test's
-// rounding.
+// Bit b set when box b of the tile (boxes row-major, T/8 a row) may hold a pixel centre
+// inside the footprint: unless the footprint's least power over the box's pixel centres is
+// past the cutoff. The least power lies on an edge facing the centre (walk.cuh's reachesBox,
+// here for the factored conic). Conservative: the limit carries a margin over the per-pixel
+// test's rounding, in absolute and relative terms and for the cancellation in t = dx + fr dy
+// (an error of 2 ca t over the roundings of dx and fr dy, with ca t^2 near the limit).
 template <uint32_t T>
 __device__ __forceinline__ uint32_t boxMask(float tileX0, float tileY0, float4 screen, float ca, float fr, float fs) {
     constexpr int kAcross = (int)(T / kBox);
-    float ex, ey;
-    footprintExtent(ca, fr, fs, screen.w, ex, ey);
-    // box column b holds pixel centres tileX0 + 8 b + 0.5 .. tileX0 + 8 b + 7.5
-    const float x0 = (screen.x - ex) - (tileX0 + 0.5f), x1 = (screen.x + ex) - (tileX0 + 0.5f);
-    const float y0 = (screen.y - ey) - (tileY0 + 0.5f), y1 = (screen.y + ey) - (tileY0 + 0.5f);
-    const float lim = (float)kAcross;
-    const int bx0 = (int)ceilf(clampf((x0 - 7.0f) * 0.125f, -1.0f, lim));
-    const int bx1 = (int)floorf(clampf(x1 * 0.125f, -1.0f, lim));
-    const int by0 = (int)ceilf(clampf((y0 - 7.0f) * 0.125f, -1.0f, lim));
-    const int by1 = (int)floorf(clampf(y1 * 0.125f, -1.0f, lim));
-    const int cx0 = max(bx0, 0), cx1 = min(bx1, kAcross - 1), cy0 = max(by0, 0), cy1 = min(by1, kAcross - 1);
-    if (cx0 > cx1 || cy0 > cy1) return 0u;
-    const float cb = ca * fr, cc = fs + ca * fr * fr;
+    const float cc = __fmaf_rn(ca * fr, fr, fs);
+    if (!(cc > 1e-12f)) return (1u << (kAcross * kAcross)) - 1u;
+    const float perX = __fdividef(-ca * fr, cc);   // an edge at x: the least power's y over x
     const float limit = screen.w * 1.0001f + 1e-4f;
+    const float cancel = 3e-7f * __fsqrt_rn(ca * limit);
     uint32_t mask = 0;
-    for (int r = cy0; r <= cy1; ++r) {
-        const float loy = (tileY0 + (float)(r * (int)kBox) + 0.5f) - screen.y;
-        for (int c = cx0; c <= cx1; ++c) {
-            const float lox = (tileX0 + (float)(c * (int)kBox) + 0.5f) - screen.x;
-            const float least = minPowerOverBoxFactored(ca, cb, cc, fr, fs, lox, loy, lox + (float)(kBox - 1),
-                                                        loy + (float)(kBox - 1));
-            if (least <= limit) mask |= 1u << (r * kAcross + c);
+#pragma unroll
+    for (int r = 0; r < kAcross; ++r) {
+        const float loy = (tileY0 + (float)(r * (int)kBox) + 0.5f) - screen.y, hiy = loy + (float)(kBox - 1);
+        const float ey = clampf(0.0f, loy, hiy), Y = fmaxf(fabsf(loy), fabsf(hiy));
+#pragma unroll
+        for (int c = 0; c < kAcross; ++c) {
+            const float lox = (tileX0 + (float)(c * (int)kBox) + 0.5f) - screen.x, hix = lox + (float)(kBox - 1);
+            const float ex = clampf(0.0f, lox, hix), X = fmaxf(fabsf(lox), fabsf(hix));
+            const float y = clampf(perX * ex, loy, hiy), x = clampf(-fr * ey, lox, hix);
+            const float t = __fmaf_rn(fr, y, ex), u = __fmaf_rn(fr, ey, x);
+            const float onX = ex != 0.0f ? __fmaf_rn(ca * t, t, (fs * y) * y) : 3.4e38f;
+            const float onY = ey != 0.0f ? __fmaf_rn(ca * u, u, (fs * ey) * ey) : 3.4e38f;
+            const float least = ex == 0.0f && ey == 0.0f ? 0.0f : fminf(onX, onY);
+            if (!(least > __fmaf_rn(cancel, __fmaf_rn(fabsf(fr), Y, X), limit))) mask |= 1u << (r * kAcross + c);
         }
     }
     return mask;
@@ -83,15 +74,15 @@ __device__ __forceinline__ float blendFloor(float cutoffExp, float lgOpacity) {
 }
 
 // The adjoint's sums over a warp, kSumRecords records at a time through shared memory:
-// each lane stores its nine values of a record in nine columns (a column: one value of
-// one record, the warp's 32 lanes side by side), then lane k sums column k's 32 values
-// by eight 16-byte loads and adds the total into the record's word in global memory.
-// A record's nine sums cost 9 stores and a third of 8 loads and 31 adds; summing them by
-// shuffles (a transposed reduction of eight, the ninth beside it) took 12 shuffles, 12
-// adds and 16 selects a record, and nine lanes' reductions a record instead of 27 lanes'
-// for three.
-constexpr uint32_t kSumWords = 9;     // moments t, dy, tt, t dy, dy dy; alpha; colour r g b
-constexpr uint32_t kSumRecords = 3;   // 27 of 32 lanes take a column
+// each lane stores six values of a record in six columns (a column: one value of one
+// record, the warp's 32 lanes side by side), then lane k sums column k by eight 16-byte
+// loads and adds the record's words into global memory. A lane's two pixels and a column's
+// runs of four share their row, so the moments in dy come from the row sums (walk.cuh's
+// rowSums) and need no columns: six values for nine words. Shared memory bounds this (its
+// pipe 76% busy with nine columns); summing by shuffles (a transposed reduction) took 12
+// shuffles, 12 adds and 16 selects a record.
+constexpr uint32_t kSumValues = 6;    // of -2 dL/dpower: its sum, its moments t and t t; dL/dcolour r g b
+constexpr uint32_t kSumRecords = 4;   // 24 of 32 lanes take a column: five records' would cost a block an SM
 
 // ---- the blends of a training step: forward, loss and adjoint, a tile at a time ----
 // One block of T*T/2 threads takes tiles off a queue (heaviest first: `order`,
@@ -164,7 +155,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
     struct Adjoint {
         Gathered records[32];
         uint32_t rec[32];           // their records
-        float sums[kSumRecords * kSumWords * kColumnStride];
+        float sums[kSumRecords * kSumValues * kColumnStride];
     };
     constexpr size_t kAdjointBytes = kTrain ? kThreads / 32 * sizeof(Adjoint) : 0;
     constexpr size_t kBytes = sizeof(Forward) > kAdjointBytes ? sizeof(Forward) : kAdjointBytes;
@@ -177,7 +168,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
     const float kScale = -0.5f * 1.4426950408889634f;   // power -> base-2 exponent
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lx = (warp % kAcross) * kBox + (lane & 3u), ly = (warp / kAcross) * kBox + (lane >> 2);
-    const uint32_t sumRecord = lane / kSumWords, sumWord = lane % kSumWords;   // the column this lane sums
+    const uint32_t sumRecord = lane / kSumValues, sumValue = lane % kSumValues;   // the column this lane sums
     uint32_t evaluated = 0;   // (pixel, record) evaluations of the forward this thread made
     uint32_t blended = 0;     // of them, those that blended
     uint32_t adjVisited = 0, adjLive = 0;   // the adjoint's evaluations, and those that blended
@@ -330,6 +321,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         __syncthreads();   // the block's warps are done with the staged records, whose memory the adjoint takes
         Adjoint& sA = reinterpret_cast<Adjoint*>(sRaw)[warp];
         const Px<2> xc{{pxc[0], pxc[1]}}, yc = both<2>(pyc);
+        const float rowMid = tileY0 + (float)((warp / kAcross) * kBox) + 0.5f * (float)kBox;   // the box's middle row
         Px<2> light{{Tr[0], Tr[1]}};   // the pixels' transmittance, from the last record back
         const uint32_t warpLast = __reduce_max_sync(0xFFFFFFFFu, max(last[0], last[1]));
         const uint32_t nChunks = (warpLast + 31u) >> 5;
@@ -377,7 +369,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                 for (uint32_t q0 = 0; q0 < cnt; q0 += kSumRecords) {
                     const uint32_t batch = min(kSumRecords, cnt - q0);
                     float* column = sA.sums + lane;
-                    for (uint32_t q = q0; q < q0 + batch; ++q, column += kSumWords * kColumnStride) {
+                    for (uint32_t q = q0; q < q0 + batch; ++q, column += kSumValues * kColumnStride) {
                         if constexpr (kCount) { ++adjVisits; ++adjSummed; }
                         const Gathered& G = sA.records[q];
                         auto pair = [](const float (&v)[2]) { return Px<2>{{v[0], v[1]}}; };
@@ -408,32 +400,36 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                         sd = fused(alpha, u, sd);
 #pragma unroll
                         for (int p = 0; p < 2; ++p) dP.v[p] = raw.v[p] < 0.99f ? dP.v[p] : 0.0f;
-                        // the lane's two pixels: dy is theirs both
                         const Px<2> dPt = dP * t, dPtt = dPt * t, wr = w * dR, wg = w * dG, wb = w * dB;
-                        const float m0 = dP.v[0] + dP.v[1], mt = dPt.v[0] + dPt.v[1], my = dy.v[0] * m0;
-                        column[0 * kColumnStride] = mt;
-                        column[1 * kColumnStride] = my;
+                        column[0 * kColumnStride] = dP.v[0] + dP.v[1];
+                        column[1 * kColumnStride] = dPt.v[0] + dPt.v[1];
                         column[2 * kColumnStride] = dPtt.v[0] + dPtt.v[1];
-                        column[3 * kColumnStride] = dy.v[0] * mt;
-                        column[4 * kColumnStride] = dy.v[0] * my;
-                        column[5 * kColumnStride] = m0;
-                        column[6 * kColumnStride] = wr.v[0] + wr.v[1];
-                        column[7 * kColumnStride] = wg.v[0] + wg.v[1];
-                        column[8 * kColumnStride] = wb.v[0] + wb.v[1];
+                        column[3 * kColumnStride] = wr.v[0] + wr.v[1];
+                        column[4 * kColumnStride] = wg.v[0] + wg.v[1];
+                        column[5 * kColumnStride] = wb.v[0] + wb.v[1];
                     }
                     __syncwarp();
-                    // lane k sums column k and adds it into its record's words in global memory (a
-                    // reduction, not read back): the five moments, dL/dalpha and dL/dcolour, which the
-                    // projection's adjoint turns into centre and conic gradients (linear in the
-                    // moments, so sums from every box, tile and batch add up). A gathered record's
+                    // lane k sums column k and adds what it gives into the record's words in global
+                    // memory (reductions, not read back): the five moments, dL/dalpha and dL/dcolour,
+                    // which the projection's adjoint turns into centre and conic gradients (linear in
+                    // the moments, so sums from every box, tile and batch add up). A gathered record's
                     // forward live bit says a pixel of this box blended it; sums that come to zero
                     // (all its pixels clamped) are not added.
-                    if (lane < batch * kSumWords) {
-                        float val = columnSum(sA.sums + lane * kColumnStride);
+                    if (lane < batch * kSumValues) {
+                        const Gathered& G = sA.records[q0 + sumRecord];
+                        const RowSums v = rowSums<8>(sA.sums + lane * kColumnStride);
+                        const float dy = rowMid + G.ny[0];   // of the box's middle row
+                        float* words = grads + (size_t)sA.rec[q0 + sumRecord] * kGradWords;
                         // an opacity over 1 takes no geometry or opacity gradient (its kernel has no moments)
-                        if (sumWord < 6 && sA.records[q0 + sumRecord].lgo[0] > 0.0f) val = 0.0f;
-                        if (val != 0.0f)
-                            atomicAdd(grads + (size_t)sA.rec[q0 + sumRecord] * kGradWords + sumWord, val);
+                        const bool some = v.sum != 0.0f || v.first != 0.0f || v.second != 0.0f;
+                        if (some && (sumValue >= 3 || G.lgo[0] <= 0.0f)) {
+                            // words: moments t, dy, t t, t dy, dy dy; the opacity's; the colour's
+                            atomicAdd(words + (sumValue == 0 ? 5u : sumValue == 1 ? 0u : sumValue == 2 ? 2u : 3u + sumValue),
+                                      v.sum);
+                            if (sumValue < 2) atomicAdd(words + (sumValue == 0 ? 1u : 3u), __fmaf_rn(dy, v.sum, v.first));
+                            if (sumValue == 0)
+                                atomicAdd(words + 4, __fmaf_rn(dy, __fmaf_rn(dy, v.sum, 2.0f * v.first), v.second));
+                        }
                     }
                     __syncwarp();   // the next records' values overwrite the columns
                 }

@@ -13,10 +13,9 @@
 // passes, and a pixel that does not blend a visited record takes alpha 0, which
 // leaves its sums and its transmittance as they were.
 //
-// Bound by instruction issue, and on small images by latency. Against one thread a
-// pixel over every record of the tile, staged for the whole block behind barriers: a
-// frame of 1.5M splats at 1920x1080 blends in 0.35 ms (0.50), 100k at 960x540 in 0.15
-// (0.22), 5k at 160x120 in 32 us (69).
+// Bound by instruction issue. Against one thread a pixel over every record of the
+// tile, staged for the whole block behind barriers: 1.5M splats at 1920x1080 0.50 -> 0.30 ms, 6M at
+// 3840x2160 1.53 -> 0.96, 500k Gaussians at 1280x720 (training) 0.30 -> 0.18.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -265,12 +264,15 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         const uint32_t count = __popc(hits);
         __syncwarp();   // the walk of the chunk before has read its slots
         if (hit) sRecords[warp][rank].set(screen, conic, tint, slot, first - range.x + lane + 1u);
+        if ((count & 1u) && lane == 0) sRecords[warp][count].setNone();   // the last pair's second
         __syncwarp();
+        const bool odd = __any_sync(0xFFFFFFFFu, hit && sRecords[warp][rank].odd != 0u);
         load(first + 32);
         uint32_t laneBits = 0;   // the walked records some pixel of this lane blended
-        for (uint32_t j = 0; j < count; ++j) {
-            const WalkRecord<kPx>& R = sRecords[warp][j];
-            const WalkPoint<kPx> at(R, xc, yc);
+        // one record blended into the lane's pixels; kOdd: some record of the chunk is odd;
+        // kThreshold: the depth layer's threshold crossing is wanted
+        auto blendOne = [&](uint32_t j, const WalkRecord<kPx>& R, const auto& at, auto oddHere, auto thresholdHere) {
+            constexpr bool kOdd = decltype(oddHere)::value, kThreshold = decltype(thresholdHere)::value;
             Px<kPx> alpha;
             bool blend[kPx], any = false;
 #pragma unroll
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 }
             }
             using Rec = WalkRecord<kPx>;
-            if (R.odd) {   // a colour that is not finite stays out of the pixels that do not blend it
+            if (kOdd && R.odd) {   // a colour that is not finite stays out of the pixels that do not blend it
 #pragma unroll
                 for (int p = 0; p < kPx; ++p)
                     if (blend[p]) {
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 depthSum = depthSum + weight * Rec::px(R.z);
             }
             T = T * fused(alpha, both<kPx>(-1.0f), both<kPx>(1.0f));   // T (1 - alpha)
-            if (thresholded) {
+            if (kThreshold) {
 #pragma unroll
                 for (int p = 0; p < kPx; ++p)
                     if (blend[p] && depthAt[p] < 0.0f && 1.0f - T.v[p] >= F.depthThreshold) depthAt[p] = R.z[0];
@@ -372,7 +374,30 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 done[p] = done[p] || T.v[p] < 1e-4f;
             }
             if (kTrain) laneBits |= any ? 1u << j : 0u;
-        }
+        };
+        // the chunk's walk, two records at a time: the second's power and exponential do not
+        // wait for the first's transmittance (a long chain that a warp alone on its scheduler
+        // waits out)
+        auto walk = [&](auto oddHere, auto thresholdHere) {
+            constexpr bool kOdd = decltype(oddHere)::value;
+            if (kContribution || kMatte) {
+                for (uint32_t j = 0; j < count; ++j) {
+                    const WalkRecord<kPx>& R = sRecords[warp][j];
+                    blendOne(j, R, WalkPoint<kPx, kOdd>(R, xc, yc), oddHere, thresholdHere);
+                }
+            } else {
+                for (uint32_t j = 0; j < count; j += 2) {
+                    const WalkRecord<kPx>& R = sRecords[warp][j];
+                    const WalkRecord<kPx>& S = sRecords[warp][j + 1];
+                    const WalkPoint<kPx, kOdd> first(R, xc, yc), second(S, xc, yc);
+                    blendOne(j, R, first, oddHere, thresholdHere);
+                    blendOne(j + 1, S, second, oddHere, thresholdHere);
+                }
+            }
+        };
+        if (odd) walk(std::true_type(), std::true_type());
+        else if (thresholded) walk(std::false_type(), std::true_type());
+        else walk(std::false_type(), std::false_type());
         if (kTrain) {
             const uint32_t walked = __reduce_or_sync(0xFFFFFFFFu, laneBits);
             const uint32_t word = __ballot_sync(0xFFFFFFFFu, hit && ((walked >> rank) & 1u));
@@ -433,7 +458,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
 
 bool trainingOnePixel(const FrameConst& F, int sms, const Contribution& contrib, const Matte& matte) {
     return contrib.mode != 0u || matte.out != nullptr || matte.lifted != nullptr || matte.trace != nullptr ||
-           onePixelBoxes(F.tilesX * F.tilesY, (uint32_t)sms);
+           onePixelBoxes(F.tilesX * F.tilesY, (uint32_t)sms, true);
 }
 size_t trainingLiveWords(const FrameConst& F, uint64_t pairs) { return frameLiveWords(pairs, F.tilesX * F.tilesY); }
 
@@ -451,7 +476,7 @@ cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, con
     const bool c = contrib.mode != 0u, u = under.depth != nullptr,
                m = matte.out != nullptr || matte.lifted != nullptr || matte.trace != nullptr;
     // an under-layer is never part of a differentiable frame
-    const bool one = training ? keep.onePixel : onePixelBoxes(tiles, (uint32_t)sms);
+    const bool one = training ? keep.onePixel : onePixelBoxes(tiles, (uint32_t)sms, false);
     if (m) {
         if (c && training) ATH_BLEND(1, true, true, false, true);
         else if (training) ATH_BLEND(1, true, false, false, true);

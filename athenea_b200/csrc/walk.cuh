@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "raster_types.cuh"
 #include "splat_math.cuh"
@@ -63,10 +64,14 @@ struct Box {
 
 // Images whose boxes of two pixels a lane are fewer than this many an SM take boxes of
 // one pixel a lane: half the work a warp, twice the warps, where warps are too few to
-// hide each other's latency (5k splats at 160x120: the blend 32 us; 20k Gaussians at
-// 333x251: blend and adjoint 49 and 75 us).
-constexpr uint32_t kBoxesAnSm = 24;
-inline bool onePixelBoxes(uint32_t tiles, uint32_t sms) { return tiles * Box<2>::kCount < sms * kBoxesAnSm; }
+// hide each other's latency and the longest lists' boxes end last. A training pass, whose
+// adjoint reads and tests each record once a box, does so up to 64 boxes an SM, a frame up to 128.
+// By one and by two: frames of 100k splats at 960x540 (55 an SM) 233 and 262 us, of 1.5M at
+// 1280x720 (97) 743 and 755, at 1920x1080 (221) 876 and 870; passes over 500k Gaussians at
+// 960x540 763 and 793 us, at 1280x720 885 and 856.
+inline bool onePixelBoxes(uint32_t tiles, uint32_t sms, bool training) {
+    return tiles * Box<2>::kCount < sms * (training ? 64u : 128u);
+}
 
 // The live bits a differentiable frame keeps: chunk c of tile t's list (its records 32 c
 // to 32 c + 31) and box b at word ((range start >> 5) + t + c) * boxes + b, bit k set when
@@ -99,18 +104,32 @@ __device__ __forceinline__ void liveRecord(uint32_t word, uint32_t excl, uint32_
     }
 }
 
-// The sum of a column: 32 floats, the warp's lanes side by side.
-__device__ __forceinline__ float columnSum(const float* column) {
+// The sums of a column: 32 floats, the warp's lanes side by side, four lanes a row of the
+// box. `sum`, and with each value times its row's offset from the box's middle row and the
+// square of that (`first`, `second`): a lane's pixels share their row, so a moment in y is
+// taken over rows here rather than a pixel at a time.
+struct RowSums {
+    float sum, first, second;
+};
+template <int kRows>
+__device__ __forceinline__ RowSums rowSums(const float* column) {
+    static_assert(kRows == 8 || kRows == 4, "8x8 boxes take four lanes a row, 8x4 ones eight");
     const float4* in = reinterpret_cast<const float4*>(column);
-    Px<2> a{{in[0].x, in[0].y}}, b{{in[0].z, in[0].w}};
+    RowSums r;
 #pragma unroll
-    for (uint32_t k = 1; k < 8; ++k) {
-        const float4 v = in[k];
-        a = a + Px<2>{{v.x, v.y}};
-        b = b + Px<2>{{v.z, v.w}};
+    for (int row = 0; row < kRows; ++row) {
+        float4 v = in[row * (8 / kRows)];
+        if (kRows == 4) {
+            const float4 u = in[row * 2 + 1];
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        const Px<2> two = Px<2>{{v.x, v.y}} + Px<2>{{v.z, v.w}};
+        const float s = two.v[0] + two.v[1], at = (float)row - 0.5f * (float)(kRows - 1);
+        r.sum = row ? r.sum + s : s;
+        r.first = row ? __fmaf_rn(at, s, r.first) : at * s;
+        r.second = row ? __fmaf_rn(at * at, s, r.second) : (at * at) * s;
     }
-    a = a + b;
-    return a.v[0] + a.v[1];
+    return r;
 }
 constexpr uint32_t kColumnStride = 36;   // floats: 16-byte aligned, eight lanes' loads in eight banks of four
 
@@ -168,6 +187,11 @@ struct alignas(16) WalkRecord {
         slot = atSlot;
         place = atPlace;
     }
+    // A record no pixel blends.
+    __device__ __forceinline__ void setNone() {
+        set(make_float4(0.0f, 0.0f, 0.0f, -3.4e38f), make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f),
+            0u, 0u);
+    }
     static __device__ __forceinline__ Px<kPx> px(const float (&m)[kPx]) {
         Px<kPx> o;
 #pragma unroll
@@ -207,19 +231,20 @@ __device__ __forceinline__ Px<kPx> expWalk(Px<kPx> power) {
 }
 
 // A record at a lane's pixels: the offsets, the power, the unclamped alpha and its
-// Gaussian, each rounded as splat_blend.slang:340-362 has them.
-template <int kPx>
+// Gaussian, each rounded as splat_blend.slang:340-362 has them. kOdd: the record may be one
+// of WalkRecord::odd.
+template <int kPx, bool kOdd>
 struct WalkPoint {
-    Px<kPx> dx, dy, power, gauss, raw;
+    Px<kPx> dx, dy, power, raw;
 
     __device__ __forceinline__ WalkPoint(const WalkRecord<kPx>& R, Px<kPx> xc, Px<kPx> yc) {
         using Rec = WalkRecord<kPx>;
         dx = xc + Rec::px(R.nx);
         dy = yc + Rec::px(R.ny);
         power = ((Rec::px(R.a) * dx) * dx + (Rec::px(R.b2) * dx) * dy) + (Rec::px(R.c) * dy) * dy;
-        gauss = expWalk<kPx>(power);
+        const Px<kPx> gauss = expWalk<kPx>(power);
         raw = Rec::px(R.alpha) * gauss;
-        if (R.odd && R.alpha[0] > 1.0f) {   // Spark's harder kernel (frame.slang:337-348)
+        if (kOdd && R.alpha[0] > 1.0f) {   // Spark's harder kernel (frame.slang:337-348)
 #pragma unroll
             for (int p = 0; p < kPx; ++p) raw.v[p] = falloffAlpha(R.alpha[0], gauss.v[p]);
         }
