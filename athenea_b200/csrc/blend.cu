@@ -124,27 +124,30 @@ struct CryptoList {
             weights[k] = 0.0f;
         }
     }
-    __device__ __forceinline__ void add(uint32_t id, float weight) {
-        if (weight <= 0.0f || id == 0) return;
+    // `weight` of `id` (where `on`): added to the id's slot, or in the place of the lightest
+    // when the id is new and heavier. Without branches: a warp's pixels differ in which of
+    // these they take, and an id is in at most one slot.
+    __device__ __forceinline__ void add(bool on, uint32_t id, float weight) {
+        on = on && weight > 0.0f && id != 0;
+        bool found = false;
         uint32_t lightest = 0;
         float lightestWeight = weights[0];
 #pragma unroll
         for (uint32_t k = 0; k < kCryptoSlots; ++k) {
-            if (ids[k] == id && weights[k] > 0.0f) {
-                weights[k] += weight;
-                return;
-            }
-            if (weights[k] < lightestWeight) {
-                lightest = k;
-                lightestWeight = weights[k];
-            }
+            const bool here = ids[k] == id && weights[k] > 0.0f;
+            const bool less = weights[k] < lightestWeight;
+            lightest = less ? k : lightest;
+            lightestWeight = less ? weights[k] : lightestWeight;
+            found = found || here;
+            weights[k] = on && here ? weights[k] + weight : weights[k];
         }
+        const bool enter = on && !found && weight > lightestWeight;
 #pragma unroll
-        for (uint32_t k = 0; k < kCryptoSlots; ++k)
-            if (k == lightest && weight > weights[k]) {
-                ids[k] = id;
-                weights[k] = weight;
-            }
+        for (uint32_t k = 0; k < kCryptoSlots; ++k) {
+            const bool here = enter && k == lightest;
+            ids[k] = here ? id : ids[k];
+            weights[k] = here ? weight : weights[k];
+        }
     }
     __device__ __forceinline__ void write(float4* out, uint32_t at, uint32_t pixels) const {
         uint32_t order[kCryptoSlots];
@@ -168,6 +171,10 @@ struct CryptoList {
     }
 };
 
+// Which of the matte's layers a blend makes: Cryptomatte alone, or any of it (Cryptomatte,
+// the lifted matte, the trace), whose lists take more registers.
+enum MatteKind : uint32_t { kNoMatte = 0, kCryptomatte = 1, kAnyMatte = 2 };
+
 // kContribution: the contributionMode hooks of splat_blend.slang:364-407 (modes
 // 1 to 4). kUnder: the composite over an opaque layer under the splats
 // (:249-251,329-333,516-523,555-575): a pixel's walk stops at the first record
@@ -175,7 +182,7 @@ struct CryptoList {
 // kMatte: Cryptomatte, the lifted matte and the trace. The plain frame builds
 // without any; kTrain also keeps what the backward needs. The hooks run a pixel at
 // a time, so those kernels take one pixel a lane.
-template <int kPx, bool kTrain, bool kContribution, bool kUnder, bool kMatte>
+template <int kPx, bool kTrain, bool kContribution, bool kUnder, MatteKind kMatte>
 __global__ void __launch_bounds__(Box<kPx>::kThreads)
     blendKernel(const FrameConst F, uint32_t pairs, uint32_t slots, const uint2* __restrict__ ranges,
                 const uint64_t* __restrict__ sorted, const float4* __restrict__ recs, float4* __restrict__ colour,
@@ -184,10 +191,11 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 Contribution contrib, Under under, Matte matte) {
     static_assert(kPx == 1 || !(kContribution || kMatte), "the hooks take one pixel a lane");
     __shared__ WalkRecord<kPx> sRecords[Box<kPx>::kCount][32];
+    __shared__ uint32_t sIds[kMatte ? Box<kPx>::kCount : 1][kMatte ? 32 : 1];   // the records' Cryptomatte ids
     CryptoList list;
     if (kMatte) list.clear();
     TraceList trace;
-    if (kMatte && matte.trace) trace.clear();
+    if (kMatte == kAnyMatte && matte.trace) trace.clear();
 
     const uint32_t tile = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t boxX = (tile % F.tilesX) * kTile + Box<kPx>::x0(warp);
@@ -237,7 +245,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         return __all_sync(0xFFFFFFFFu, d);
     };
     // the list a chunk ahead: lane l's record of the next chunk is loaded while this one is walked
-    uint32_t slot = 0;
+    uint32_t slot = 0, id = 0;
     float4 screen, conic, tint;
     screen = conic = tint = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     auto load = [&](uint32_t first) {
@@ -250,6 +258,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         screen = recs[(size_t)slot * 3 + 0];
         conic = recs[(size_t)slot * 3 + 1];
         tint = recs[(size_t)slot * 3 + 2];
+        if (kMatte && matte.out) id = matte.ids[slot];
     };
     load(range.x);
     for (uint32_t first = range.x; first < range.y; first += 32) {
@@ -264,6 +273,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         const uint32_t count = __popc(hits);
         __syncwarp();   // the walk of the chunk before has read its slots
         if (hit) sRecords[warp][rank].set(screen, conic, tint, slot, first - range.x + lane + 1u);
+        if (kMatte && hit) sIds[warp][rank] = id;
         if ((count & 1u) && lane == 0) sRecords[warp][count].setNone();   // the last pair's second
         __syncwarp();
         const bool odd = __any_sync(0xFFFFFFFFu, hit && sRecords[warp][rank].odd != 0u);
@@ -322,9 +332,9 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     atomicAdd(&contrib.words[s * 4 + 3], (uint32_t)(w * kColourGradScale + 0.5f));
                 }
             }
-            if (kMatte && blend[0]) {
+            if (kMatte && matte.out) list.add(blend[0], sIds[warp][j], weight.v[0]);
+            if (kMatte == kAnyMatte && blend[0] && (matte.trace || matte.lifted)) {
                 const float w = weight.v[0];
-                if (matte.out) list.add(matte.ids[R.slot], w);
                 if (matte.trace) {
                     // splat_blend.slang:445-451
                     trace.total = trace.total + w;
@@ -417,16 +427,16 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
             if (depthAt[p] < 0.0f) depthAt[p] = underZ[p];
         }
         const float total = kUnder && underHit[p] ? 1.0f : coverage;
-        if (kMatte && matte.trace)   // splat_blend.slang:545-551: what closed the walk from behind is `under`
+        if (kMatte == kAnyMatte && matte.trace)   // splat_blend.slang:545-551: what closed the walk from behind is `under`
             trace.write(matte.trace, at, F.width * F.height, kUnder && underHit[p] ? left : 0.0f, recs);
-        if (kMatte && matte.lifted) {
+        if (kMatte == kAnyMatte && matte.lifted) {
             // splat_blend.slang:536-539: the untold weight at the share of the known
             const float share = matteKnown > 0.0f ? matteInside / matteKnown : 0.0f;
             matte.lifted[at] = fminf(fmaxf(matteInside + matteUntold * share, 0.0f), 1.0f);
         }
         if (kMatte && matte.out) {
             // what closed the walk takes the rest of the pixel (splat_blend.slang:525-534)
-            list.add(kUnder && underHit[p] && matte.underIds ? matte.underIds[at] : 0u, kUnder && underHit[p] ? left : 0.0f);
+            if (kUnder && underHit[p] && matte.underIds) list.add(true, matte.underIds[at], left);
             list.write(reinterpret_cast<float4*>(matte.out), at, F.width * F.height);
         }
         colour[at] = make_float4(r.v[p] + left * behind.x, g.v[p] + left * behind.y, bl.v[p] + left * behind.z,
@@ -477,26 +487,29 @@ cudaError_t launchBlend(const FrameConst& F, uint32_t pairs, uint32_t slots, con
                m = matte.out != nullptr || matte.lifted != nullptr || matte.trace != nullptr;
     // an under-layer is never part of a differentiable frame
     const bool one = training ? keep.onePixel : onePixelBoxes(tiles, (uint32_t)sms, false);
-    if (m) {
-        if (c && training) ATH_BLEND(1, true, true, false, true);
-        else if (training) ATH_BLEND(1, true, false, false, true);
-        else if (c && u) ATH_BLEND(1, false, true, true, true);
-        else if (c) ATH_BLEND(1, false, true, false, true);
-        else if (u) ATH_BLEND(1, false, false, true, true);
-        else ATH_BLEND(1, false, false, false, true);
+    if (m && !c && !training && matte.lifted == nullptr && matte.trace == nullptr) {
+        if (u) ATH_BLEND(1, false, false, true, kCryptomatte);
+        else ATH_BLEND(1, false, false, false, kCryptomatte);
+    } else if (m) {
+        if (c && training) ATH_BLEND(1, true, true, false, kAnyMatte);
+        else if (training) ATH_BLEND(1, true, false, false, kAnyMatte);
+        else if (c && u) ATH_BLEND(1, false, true, true, kAnyMatte);
+        else if (c) ATH_BLEND(1, false, true, false, kAnyMatte);
+        else if (u) ATH_BLEND(1, false, false, true, kAnyMatte);
+        else ATH_BLEND(1, false, false, false, kAnyMatte);
     } else if (c) {
-        if (training) ATH_BLEND(1, true, true, false, false);
-        else if (u) ATH_BLEND(1, false, true, true, false);
-        else ATH_BLEND(1, false, true, false, false);
+        if (training) ATH_BLEND(1, true, true, false, kNoMatte);
+        else if (u) ATH_BLEND(1, false, true, true, kNoMatte);
+        else ATH_BLEND(1, false, true, false, kNoMatte);
     } else if (training) {
-        if (one) ATH_BLEND(1, true, false, false, false);
-        else ATH_BLEND(2, true, false, false, false);
+        if (one) ATH_BLEND(1, true, false, false, kNoMatte);
+        else ATH_BLEND(2, true, false, false, kNoMatte);
     } else if (u) {
-        if (one) ATH_BLEND(1, false, false, true, false);
-        else ATH_BLEND(2, false, false, true, false);
+        if (one) ATH_BLEND(1, false, false, true, kNoMatte);
+        else ATH_BLEND(2, false, false, true, kNoMatte);
     } else {
-        if (one) ATH_BLEND(1, false, false, false, false);
-        else ATH_BLEND(2, false, false, false, false);
+        if (one) ATH_BLEND(1, false, false, false, kNoMatte);
+        else ATH_BLEND(2, false, false, false, kNoMatte);
     }
 #undef ATH_BLEND
     return cudaGetLastError();
