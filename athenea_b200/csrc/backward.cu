@@ -15,6 +15,7 @@
 // transmittance back out record by record.
 #include <algorithm>
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "adjoint.cuh"
@@ -26,12 +27,6 @@
 
 namespace ath {
 namespace {
-
-__device__ __forceinline__ float warpSum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
 
 // 1 / x, x in [0.01, 1]: the hardware's approximation and one Newton step.
 __device__ __forceinline__ float reciprocal(float x) {
@@ -350,28 +345,42 @@ __global__ void __launch_bounds__(128)
 }
 
 // L = mean over pixels and r g b of (colour - target)^2: its value (added into
-// *loss) and dL/dcolour (float4 a pixel, alpha 0).
-__global__ void __launch_bounds__(256)
+// *loss) and dL/dcolour (float4 a pixel, alpha 0). The threads' shares are summed in 64
+// bits over a cluster of blocks, one 32-bit addition into *loss a cluster: one a block of
+// 256 pixels, thousands an image, each rounded *loss, up to 2e-6 of it in all.
+constexpr uint32_t kLossThreads = 256, kLossCluster = 8, kLossBlocks = 148 * kLossCluster;
+
+__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
     l2LossKernel(const float4* __restrict__ colour, const float* __restrict__ target, uint32_t pixels, float scale,
                  float4* __restrict__ dLdColour, float* __restrict__ loss) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (p < pixels) {
+    __shared__ double sPart[kLossThreads / 32], sBlock;
+    float share = 0.0f;
+#pragma unroll 4
+    for (uint64_t p = blockIdx.x * kLossThreads + threadIdx.x; p < pixels; p += (uint64_t)gridDim.x * kLossThreads) {
         const float4 c = colour[p];
         const float er = c.x - target[p * 3 + 0], eg = c.y - target[p * 3 + 1], eb = c.z - target[p * 3 + 2];
-        l = (er * er + eg * eg + eb * eb) * scale;
+        share += (er * er + eg * eg + eb * eb) * scale;
         dLdColour[p] = make_float4(2.0f * scale * er, 2.0f * scale * eg, 2.0f * scale * eb, 0.0f);
     }
-    __shared__ float sPart[8];
-    l = warpSum(l);
-    if ((threadIdx.x & 31u) == 0) sPart[threadIdx.x >> 5] = l;
+    double sum = (double)share;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if ((threadIdx.x & 31u) == 0) sPart[threadIdx.x >> 5] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float b = 0.0f;
+        sum = 0.0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) b += sPart[w];
-        if (b != 0.0f) atomicAdd(loss, b);
+        for (uint32_t w = 0; w < kLossThreads / 32; ++w) sum += sPart[w];
+        sBlock = sum;
     }
+    const auto cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    if (threadIdx.x == 0 && cluster.block_rank() == 0) {
+        sum = 0.0;
+        for (uint32_t b = 0; b < kLossCluster; ++b) sum += *cluster.map_shared_rank(&sBlock, b);
+        if (sum != 0.0) atomicAdd(loss, (float)sum);
+    }
+    cluster.sync();   // the others' shared memory is read until here
 }
 
 }   // namespace
@@ -411,8 +420,9 @@ cudaError_t launchProjectBackward(const FrameConst& F, const InstanceConst& I, c
 cudaError_t launchL2Loss(const float4* colour, const float* target, uint32_t pixels, float4* dLdColour, float* loss,
                          cudaStream_t stream) {
     if (pixels == 0) return cudaSuccess;
-    l2LossKernel<<<(pixels + 255) / 256, 256, 0, stream>>>(colour, target, pixels, 1.0f / (3.0f * (float)pixels),
-                                                          dLdColour, loss);
+    const uint32_t blocks = std::min((pixels + kLossThreads - 1) / kLossThreads, kLossBlocks);
+    l2LossKernel<<<(blocks + kLossCluster - 1) / kLossCluster * kLossCluster, kLossThreads, 0, stream>>>(
+        colour, target, pixels, 1.0f / (3.0f * (float)pixels), dLdColour, loss);
     return cudaGetLastError();
 }
 
