@@ -1046,7 +1046,7 @@ cudaError_t enqueueStep(ath_batch* b, const ath_mixed_params& P, const float* ta
                            words + kBatchEpoch, B.slotBits, bits, static_cast<uint32_t*>(b->sortHist.ptr),
                            static_cast<uint64_t*>(b->sortFlags.ptr), words + kBatchSortTickets, words + kBatchStatus,
                            stream, kClearHistograms);   // the step's first kernel clears the tickets
-    const uint32_t sorted = sortResultIndex(2, bits);
+    const uint32_t sorted = sortResultIndex((uint32_t)b->capacity, bits);
     mark(2);
     b->lastSorted = sorted;
     b->lastSlotBits = B.slotBits;

@@ -617,12 +617,12 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                          keys, static_cast<const uint32_t*>(r->offsets.ptr),
                          reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
     mark(4);
-    if (err == cudaSuccess)
+    if (err == cudaSuccess && capacity > kSortTileKeys)   // a sort in one block needs none of it
         err = cudaMemsetAsync(hist, 0, kSortHistBytes + sortFlagWords(capacity, bits) * 8, stream);
     if (err == cudaSuccess)
         err = launchSortDevice(pairs, nullptr, capacity, kept, nullptr, 32, bits, hist, flags, words + kWordSortTickets,
                                words + kWordSticky, stream, kClearNone);
-    const uint32_t sorted = sortPasses(bits) & 1u;
+    const uint32_t sorted = sortResultIndex(capacity, bits);
     if (err == cudaSuccess) err = launchRanges(capacity, kept, tiles, pairs[sorted], ranges, words + kWordSticky, stream);
     mark(5);
     // --- blend ---------------------------------------------------------------
@@ -953,7 +953,7 @@ extern "C" ath_status ath_sorter_sort(ath_sorter* s, uint64_t* keys, uint32_t* v
     cudaError_t err = s->scratch.reserve(bytes);
     if (err != cudaSuccess) return failCuda(err, "reserving the sort's look-back words");
     char* scratch = static_cast<char*>(s->scratch.ptr);
-    err = cudaMemsetAsync(scratch, 0, bytes, stream);
+    if (count > kSortTileKeys) err = cudaMemsetAsync(scratch, 0, bytes, stream);   // a sort in one block needs none of it
     if (err != cudaSuccess) return failCuda(err, "sorting");
     uint64_t* k[2] = {keys, scratchKeys};
     uint32_t* v[2] = {values, scratchValues};

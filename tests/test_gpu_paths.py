@@ -58,6 +58,27 @@ def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(native, raster)
     assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
 
 
+# one block up to 8192; 2048-key tiles up to 606,208; then tiles of 6144 (pairs)
+@pytest.mark.parametrize("count", [2, 511, 513, 8191, 8192, 8193, 10_240, 606_208, 606_209, 700_001])
+@pytest.mark.parametrize("bits", [1, 9, 24, 45, 64])
+def test_sorts_are_stable_at_every_tile_size(native, count, bits):
+    gen = torch.Generator(device="cuda").manual_seed(count + bits)
+    keys = (torch.randint(0, 1 << 32, (count,), generator=gen, device="cuda") << 32) | \
+        torch.randint(0, 1 << 32, (count,), generator=gen, device="cuda")
+    keys[::3] = keys[0].clone()   # ties
+    values = torch.arange(count, dtype=torch.int32, device="cuda")
+    k, v, k2, v2 = keys.clone(), values.clone(), torch.empty_like(keys), torch.empty_like(values)
+    sorter = cases._Sorter()
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    N.check(N.lib().ath_sorter_sort(sorter.handle, ptr(k), ptr(v), ptr(k2), ptr(v2), count, bits,
+                                    C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    N.check(N.lib().ath_sorter_check(sorter.handle))
+    host = keys.cpu().numpy().view(np.uint64)
+    order = np.argsort(host & np.uint64((1 << max(bits, 8)) - 1), kind="stable")   # a pass takes a whole digit
+    np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), order.astype(np.uint32))
+    np.testing.assert_array_equal(k.cpu().numpy().view(np.uint64), host[order])
+
+
 # strides whose records' 16-byte pieces end in the middle, that fill shared memory, and that do not fit it;
 # counts around a warp and a block
 @pytest.mark.parametrize("pad,shift", [(0, 1), (1, 0), (2, 3), (330, 0), (600, 0)])
