@@ -69,7 +69,9 @@ enum BatchWord : uint32_t {
     kBatchStaged = 38,       // 64-bit (38, 39): records a block staged (loaded and box-tested) for the forward
     kBatchLoss = 40,         // a step's loss as a double (40, 41), and the blend blocks that have added their
     kBatchLossBlocks = 42,   // share to it: the last one writes the loss
-    kBatchWords = 48,
+    kBatchTileCounts = 48,   // the tiles of each bit length of their pair counts (33), and how many of each
+    kBatchTileCursors = 81,  // have been placed in the blends' queue (33)
+    kBatchWords = 114,
 };
 
 // An epoch-tagged look-back word: [epoch:30][status:2][value:32]. A word with
