@@ -111,12 +111,26 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* sWa
 // What a pass carries beside its keys.
 enum SortValues : uint32_t { kNoValues = 0, kReadValues = 1, kIndexValues = 2 };   // index: a key's place in the input
 
+// A pass's shared memory: its keys, their place taken by its chains' digit masks while it
+// ranks; then its chains' digit counters.
+template <uint32_t kBits, uint32_t kPerThread>
+__host__ __device__ constexpr uint32_t rankChains() { return kWarps * (kBits == 8 && kPerThread >= 16 ? 2 : 1); }
+template <typename K, uint32_t kBits, uint32_t kPerThread>
+__host__ __device__ constexpr size_t rankSmem() {
+    const size_t keys = (size_t)kSortThreads * kPerThread * sizeof(K), masks = ((size_t)rankChains<kBits, kPerThread>() << kBits) * 4;
+    return keys > masks ? keys : masks;
+}
+template <typename K, uint32_t kBits, uint32_t kPerThread>
+constexpr size_t onesweepSmem() {
+    return rankSmem<K, kBits, kPerThread>() + ((size_t)rankChains<kBits, kPerThread>() << kBits) * 4;
+}
+
 // kBits: the pass's digit width, 8 or 9 (kRadixT digits, one thread each in the
 // digit phase; a 9-bit pass ranks in one chain, so that its counters fit beside the keys).
 // The values take the keys' shared memory once the keys are out, each thread keeping its
 // items' places in the tile and its outputs' destinations in registers: with values as
 // without, two blocks an SM (values beside the keys, 128 KB, left one). 8M pairs of
-// 40 bits: 605 -> 594 us.
+// 40 bits: 605 -> 549 us with the masks below.
 template <typename K, uint32_t kValues, uint32_t kBits, uint32_t kPerThread>
 __global__ void __launch_bounds__(kSortThreads, 2)
     onesweepKernel(const K* __restrict__ keysIn, const uint32_t* __restrict__ valsIn, K* __restrict__ keysOut,
@@ -125,14 +139,14 @@ __global__ void __launch_bounds__(kSortThreads, 2)
                    uint32_t* __restrict__ status, const uint32_t* __restrict__ nDevice,
                    const uint32_t* __restrict__ epochDevice) {
     constexpr uint32_t kRadix = 1u << kBits;
-    constexpr uint32_t kChains = kBits == 8 && kPerThread >= 16 ? 2 : 1;
+    constexpr uint32_t kCounters = rankChains<kBits, kPerThread>(), kChains = kCounters / kWarps;
     constexpr uint32_t kChainItems = kPerThread / kChains;
-    constexpr uint32_t kCounters = kWarps * kChains;
     constexpr uint32_t kTileKeys = kSortThreads * kPerThread;
     extern __shared__ __align__(16) unsigned char smem[];
     K* sKeys = reinterpret_cast<K*>(smem);
     uint32_t* sVals = reinterpret_cast<uint32_t*>(smem);
-    uint32_t* sWarpCnt = reinterpret_cast<uint32_t*>(sKeys + kTileKeys);   // kCounters x kRadix
+    uint32_t* sMasks = reinterpret_cast<uint32_t*>(smem);   // kCounters x kRadix, while the keys are ranked
+    uint32_t* sWarpCnt = reinterpret_cast<uint32_t*>(smem + rankSmem<K, kBits, kPerThread>());   // kCounters x kRadix
     __shared__ uint32_t sTile;
     __shared__ uint32_t sStart[kRadix];
     __shared__ uint32_t sAdjust[kRadix];
@@ -148,13 +162,19 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     const uint32_t tile = sTile;
     const uint32_t base = tile * kTileKeys;
     if (base >= n) return;   // a tile past the keys (the grid was sized for a bound): out before any work
-    for (uint32_t j = tid; j < kCounters * kRadix; j += kSortThreads) sWarpCnt[j] = 0;
+#pragma unroll
+    for (uint32_t j = tid; j < kCounters * kRadix / 4; j += kSortThreads) {
+        reinterpret_cast<uint4*>(sWarpCnt)[j] = make_uint4(0, 0, 0, 0);
+        reinterpret_cast<uint4*>(sMasks)[j] = make_uint4(0, 0, 0, 0);
+    }
     __syncthreads();
     const uint32_t ltMask = (1u << lane) - 1u;
 
     // Rank: warp `warp` owns keys [base + warp*32*kPerThread, +32*kPerThread), item k of
     // lane l being the (k*32 + l)-th; walking k then l is input order, so the
-    // ranks are stable.
+    // ranks are stable. A key's peers, the warp's keys of its digit, are the bits their lanes
+    // set in the digit's mask: __match_any_sync takes some 240 cycles of an SM's quarter where
+    // 32 digits differ, and was most of a pass; the masks take 35 there, 130 where all agree.
     const uint32_t mine = base + warp * 32 * kPerThread + lane;
     K key[kPerThread];
     uint32_t rank[kPerThread];
@@ -162,23 +182,28 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     for (uint32_t k = 0; k < kPerThread; ++k) key[k] = mine + k * 32 < n ? keysIn[mine + k * 32] : (K)0;
 #pragma unroll
     for (uint32_t i = 0; i < kChainItems; ++i) {
-        uint32_t d[kChains], peers[kChains], before[kChains];
+        uint32_t at[kChains], peers[kChains], before[kChains];
         bool valid[kChains];
 #pragma unroll
         for (uint32_t c = 0; c < kChains; ++c) {
             const uint32_t k = c * kChainItems + i;
             valid[c] = mine + k * 32 < n;
-            d[c] = valid[c] ? (uint32_t)((key[k] >> shift) & digitMask) : kRadix + lane;
-            peers[c] = __match_any_sync(0xFFFFFFFFu, d[c]);
+            at[c] = (warp * kChains + c) * kRadix + digitSlot((uint32_t)((key[k] >> shift) & digitMask));
+            if (valid[c]) atomicOr(&sMasks[at[c]], 1u << lane);
         }
+        __syncwarp();
 #pragma unroll
-        for (uint32_t c = 0; c < kChains; ++c)
-            before[c] = valid[c] ? sWarpCnt[(warp * kChains + c) * kRadix + digitSlot(d[c])] : 0u;
+        for (uint32_t c = 0; c < kChains; ++c) {
+            peers[c] = valid[c] ? sMasks[at[c]] : 0u;
+            before[c] = valid[c] ? sWarpCnt[at[c]] : 0u;
+        }
         __syncwarp();
 #pragma unroll
         for (uint32_t c = 0; c < kChains; ++c)
-            if (valid[c] && lane == (uint32_t)(__ffs(peers[c]) - 1))
-                sWarpCnt[(warp * kChains + c) * kRadix + digitSlot(d[c])] = before[c] + __popc(peers[c]);
+            if (valid[c] && (peers[c] & ltMask) == 0) {   // the digit's first lane
+                sMasks[at[c]] = 0;
+                sWarpCnt[at[c]] = before[c] + __popc(peers[c]);
+            }
         __syncwarp();
 #pragma unroll
         for (uint32_t c = 0; c < kChains; ++c) rank[c * kChainItems + i] = before[c] + __popc(peers[c] & ltMask);
@@ -285,16 +310,20 @@ __global__ void __launch_bounds__(kSortThreads, 2)
 // A whole sort of at most kSortTileKeys keys in one block: the passes of `plan` one after
 // another, the keys (and values) carried in registers and reordered through shared memory.
 // A small sort's passes are latency alone, each some 6 us as a kernel; in one block they
-// need no histograms, look-back, tickets or clearing either. A frame of 5k splats: 144 -> 140 us. Every key is
+// need no histograms, look-back, tickets or clearing either. A frame of 5k splats: 144 -> 127 us. Every key is
 // read before the first is written, so the output may be the input.
+template <typename K, uint32_t kValues>
+__host__ __device__ constexpr size_t smallKeysSmem() { return kSortTileKeys * (sizeof(K) + (kValues == kNoValues ? 0 : 4)); }
 template <typename K, uint32_t kValues>
 __global__ void __launch_bounds__(kSortThreads)
     smallSortKernel(const K* keysIn, const uint32_t* valsIn, K* keysOut, uint32_t* valsOut, uint32_t n,
                     const uint32_t* __restrict__ nDevice, uint32_t firstBit, const SortPlan plan) {
     extern __shared__ __align__(16) unsigned char smem[];
+    static_assert(smallKeysSmem<K, kValues>() >= (size_t)kWarps * kMaxRadix * 4, "the masks take the keys' place");
     K* sKeys = reinterpret_cast<K*>(smem);
     uint32_t* sVals = reinterpret_cast<uint32_t*>(sKeys + kSortTileKeys);
-    uint32_t* sWarpCnt = kValues == kNoValues ? sVals : sVals + kSortTileKeys;   // kWarps x kMaxRadix
+    uint32_t* sMasks = reinterpret_cast<uint32_t*>(smem);   // kWarps x kMaxRadix at most, while the keys are ranked
+    uint32_t* sWarpCnt = reinterpret_cast<uint32_t*>(smem + smallKeysSmem<K, kValues>());   // kWarps x kMaxRadix at most
     __shared__ uint32_t sStart[kMaxRadix];
     __shared__ uint32_t sScan[kWarps];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -315,20 +344,28 @@ __global__ void __launch_bounds__(kSortThreads)
     }
     for (uint32_t p = 0; p < plan.passes; ++p) {
         const uint32_t radix = 1u << plan.width[p], digitMask = radix - 1u, shift = firstBit + plan.shift[p];
-        for (uint32_t j = tid; j < kWarps * radix; j += kSortThreads) sWarpCnt[j] = 0;
+        for (uint32_t j = tid; j < kWarps * radix / 4; j += kSortThreads) {
+            reinterpret_cast<uint4*>(sWarpCnt)[j] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(sMasks)[j] = make_uint4(0, 0, 0, 0);
+        }
         __syncthreads();
-        uint32_t* counts = sWarpCnt + warp * radix;
+        uint32_t *counts = sWarpCnt + warp * radix, *masks = sMasks + warp * radix;
 #pragma unroll
         for (uint32_t k = 0; k < kItems; ++k) {
             if (k >= perThread) break;
             const bool valid = mine + k * 32 < n;
-            const uint32_t d = valid ? (uint32_t)((key[k] >> shift) & digitMask) : radix + lane;
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-            const uint32_t before = valid ? counts[digitSlot(d)] : 0u;
+            const uint32_t at = digitSlot((uint32_t)((key[k] >> shift) & digitMask));
+            if (valid) atomicOr(&masks[at], 1u << lane);
             __syncwarp();
-            if (valid && lane == (uint32_t)(__ffs(peers) - 1)) counts[digitSlot(d)] = before + __popc(peers);
+            const uint32_t peers = valid ? masks[at] : 0u, before = valid ? counts[at] : 0u;
+            const uint32_t lower = peers & ((1u << lane) - 1u);
             __syncwarp();
-            rank[k] = before + __popc(peers & ((1u << lane) - 1u));
+            if (valid && lower == 0) {   // the digit's first lane
+                masks[at] = 0;
+                counts[at] = before + __popc(peers);
+            }
+            __syncwarp();
+            rank[k] = before + __popc(lower);
         }
         __syncthreads();
         uint32_t count = 0;
@@ -364,7 +401,7 @@ __global__ void __launch_bounds__(kSortThreads)
                 if constexpr (kValues != kNoValues) val[k] = sVals[i];
             }
         }
-        // the next pass's clearing touches the counters alone, and its barrier comes before its scatter
+        __syncthreads();   // the next pass clears its masks over the keys
     }
 #pragma unroll
     for (uint32_t k = 0; k < kItems; ++k) {
@@ -378,14 +415,7 @@ __global__ void __launch_bounds__(kSortThreads)
 }
 template <typename K, uint32_t kValues>
 constexpr size_t smallSortSmem() {
-    return kSortTileKeys * (sizeof(K) + (kValues == kNoValues ? 0 : 4)) + (size_t)kWarps * kMaxRadix * 4;
-}
-
-// A pass's dynamic shared memory: its keys and its chains' digit counters.
-template <typename K, uint32_t kBits, uint32_t kPerThread>
-constexpr size_t onesweepSmem() {
-    return (size_t)kSortThreads * kPerThread * sizeof(K) +
-           (size_t)kWarps * (kBits == 8 && kPerThread >= 16 ? 2 : 1) * ((size_t)1 << kBits) * 4;
+    return smallKeysSmem<K, kValues>() + (size_t)kWarps * kMaxRadix * 4;
 }
 
 template <typename K, uint32_t kValues, uint32_t kBits, uint32_t kPerThread>
