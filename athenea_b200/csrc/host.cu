@@ -26,10 +26,11 @@ struct ath_raster {
     int sms = 148;
     bool tight = false;   // after release_scratch: grow to the need exactly
     uint32_t slotCapacity = 0, pairCapacity = 0, tileCapacity = 0, instanceCapacity = 0;
-    DeviceBuffer recs, rects, masks, keys, offsets, instances;
+    DeviceBuffer recs, spans, keys, instances;
     DeviceBuffer depthKeys[2], depthSlots[2];   // the depth sort's
     DeviceBuffer pairs[2], sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
-    DeviceBuffer inspectSplats;   // ath_raster_frame_buffers' slots, a pair each (its keys: the spare pair buffer)
+    // ath_raster_frame_buffers' own: slots, a pair each (its keys: the spare pair buffer); rects and first pairs, a slot each
+    DeviceBuffer inspectSplats, inspectRects, inspectOffsets;
     DeviceBuffer zeroed;         // what a frame starts at zero, cleared at once (FrameZeroed): its words first
     uint2* ranges = nullptr;     // the last frame's, there
     PinnedBuffer wordsHost;      // kFrameWords: a frame that waits (its handle's first, or timed) reads them here
@@ -350,7 +351,7 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     cudaDeviceSynchronize();
     r->tight = true;
     r->slotCapacity = r->pairCapacity = r->tileCapacity = r->instanceCapacity = 0;
-    for (DeviceBuffer* b : {&r->recs, &r->rects, &r->masks, &r->keys, &r->offsets, &r->instances,
+    for (DeviceBuffer* b : {&r->recs, &r->spans, &r->keys, &r->instances, &r->inspectRects, &r->inspectOffsets,
                             &r->depthKeys[0], &r->depthKeys[1], &r->depthSlots[0], &r->depthSlots[1], &r->pairs[0],
                             &r->pairs[1], &r->inspectSplats, &r->sortScratch, &r->zeroed, &r->finalT, &r->lastContrib, &r->live, &r->grads})
         b->release();
@@ -417,10 +418,8 @@ ath_status reserveSlots(ath_raster* r, uint32_t slots) {   // reserveSplats (Til
     if (slots <= r->slotCapacity && r->recs.bytes) return ATH_OK;
     const uint32_t n = r->tight ? slots : grow(r->slotCapacity, slots);
     cudaError_t err = r->recs.reserve((size_t)n * 48);
-    if (err == cudaSuccess) err = r->rects.reserve((size_t)n * 8);
+    if (err == cudaSuccess) err = r->spans.reserve((size_t)n * 16);
     if (err == cudaSuccess) err = r->keys.reserve((size_t)n * 4);
-    if (err == cudaSuccess) err = r->offsets.reserve((size_t)n * 4);
-    if (err == cudaSuccess) err = r->masks.reserve((size_t)n * 8);
     for (int k = 0; k < 2; ++k) {
         if (err == cudaSuccess) err = r->depthKeys[k].reserve((size_t)n * 4);
         if (err == cudaSuccess) err = r->depthSlots[k].reserve((size_t)n * 4);
@@ -449,10 +448,9 @@ ath_status reservePairs(ath_raster* r, uint32_t pairs, uint32_t bits) {   // res
 // What a frame of `slots` splats and `tiles` tiles starts at zero, one after another in
 // ath_raster::zeroed, so that one clearing serves them all.
 struct FrameZeroed {
-    size_t words = 0, projectFlags, emitFlags, depthHist, depthFlags, ranges, bytes;   // byte offsets
+    size_t words = 0, emitFlags, depthHist, depthFlags, ranges, bytes;   // byte offsets
     FrameZeroed(uint32_t slots, uint32_t tiles) {
-        projectFlags = (kFrameWords * sizeof(uint32_t) + 255) / 256 * 256;
-        emitFlags = projectFlags + (size_t)projectBlocks(std::max(slots, 1u)) * 8;
+        emitFlags = (kFrameWords * sizeof(uint32_t) + 255) / 256 * 256;
         depthHist = emitFlags + (size_t)projectBlocks(std::max(slots, 1u)) * 8;
         depthFlags = depthHist + kSortHistBytes;
         ranges = depthFlags + sortFlagWords(slots, kDepthBits) * 8;
@@ -491,7 +489,7 @@ ath_status checkFrame(const ath_settings& s, const ath_targets& targets) {
 
 // The status bits of a frame's words as a status: the frame is not valid when any is set.
 ath_status frameStatusOf(const uint32_t* w) {
-    const uint32_t bits = w[kWordStatus] | w[kWordSticky];
+    const uint32_t bits = w[kWordSticky];
     if (bits & kStatusLookbackTimeout)
         return fail(ATH_E_TIMEOUT, "a look-back wait gave up (bounded spin); the frame is not valid");
     if (bits & kStatusPairOverflow)
@@ -565,7 +563,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     const bool sizing = r->pairCapacity == 0 || !r->pairs[0].bytes;   // no capacity yet: read the total once
     auto mark = [&](int k) { if (timed) cudaEventRecord(r->marks[k], stream); };
 
-    // --- project, with the tiles-touched scan fused in --------------------
+    // --- project ----------------------------------------------------------
     mark(0);
     cudaError_t err = cudaMemsetAsync(zero, 0, zeroed.bytes, stream);
     if (err == cudaSuccess && instanceCount > 1)
@@ -573,10 +571,8 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                               stream);
     if (err == cudaSuccess)
         err = launchProject(F, staged[0], static_cast<const InstanceConst*>(r->instances.ptr), instanceCount, slots, layout,
-                            s.count_splats != 0, static_cast<float4*>(r->recs.ptr), static_cast<uint2*>(r->rects.ptr),
-                            static_cast<unsigned long long*>(r->masks.ptr), static_cast<uint32_t*>(r->keys.ptr),
-                            static_cast<uint32_t*>(r->offsets.ptr), reinterpret_cast<uint64_t*>(zero + zeroed.projectFlags),
-                            words, stream);
+                            s.count_splats != 0, static_cast<float4*>(r->recs.ptr), static_cast<uint4*>(r->spans.ptr),
+                            static_cast<uint32_t*>(r->keys.ptr), words, stream);
     mark(1);
     bool haveTotals = false;
     if (sizing && err == cudaSuccess) {
@@ -584,8 +580,6 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
         err = cudaMemcpyAsync(wordsHost, words, kFrameWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
         if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
         if (err != cudaSuccess) return failCuda(err, "projecting the splats");
-        if (wordsHost[kWordStatus] & kStatusLookbackTimeout)
-            return fail(ATH_E_TIMEOUT, "a look-back wait gave up (bounded spin); the frame is not valid");
         const uint64_t pairs64 = pairsOf(wordsHost);
         if (pairs64 > 0xFFFFFFFFull) return fail(ATH_E_UNSUPPORTED, "more than 2^32 (tile, splat) pairs in one frame");
         // room for the next frames to vary without outgrowing it (a seventh over)
@@ -613,9 +607,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     mark(3);
     if (err == cudaSuccess)
         err = launchEmit(F, slots, depthSlots[0], static_cast<const float4*>(r->recs.ptr),
-                         static_cast<const uint2*>(r->rects.ptr), static_cast<const unsigned long long*>(r->masks.ptr),
-                         keys, static_cast<const uint32_t*>(r->offsets.ptr),
-                         reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
+                         static_cast<const uint4*>(r->spans.ptr), reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
     mark(4);
     if (err == cudaSuccess && capacity > kSortTileKeys)   // a sort in one block needs none of it
         err = cudaMemsetAsync(hist, 0, kSortHistBytes + sortFlagWords(capacity, bits) * 8, stream);
@@ -893,15 +885,30 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
         err = launchInspectPairs(static_cast<const uint64_t*>(r->pairs[r->lastSorted].ptr), pairs,
                                  static_cast<const uint32_t*>(r->keys.ptr), r->lastSlots, pairKeys,
                                  static_cast<uint32_t*>(r->inspectSplats.ptr), nullptr);
+    // the slots' rects and first pairs, through look-back words of this call's own
+    const size_t blocks = projectBlocks(std::max(r->lastSlots, 1u));
+    DeviceBuffer lookback;
+    if (err == cudaSuccess) err = r->inspectRects.reserve((size_t)std::max(r->lastSlots, 1u) * 8);
+    if (err == cudaSuccess) err = r->inspectOffsets.reserve((size_t)std::max(r->lastSlots, 1u) * 4);
+    if (err == cudaSuccess) err = lookback.reserve(blocks * 8 + 8);
+    if (err == cudaSuccess) err = cudaMemsetAsync(lookback.ptr, 0, blocks * 8 + 8, nullptr);
+    uint32_t* const ticketAndStatus = reinterpret_cast<uint32_t*>(static_cast<uint64_t*>(lookback.ptr) + blocks);
+    if (err == cudaSuccess)
+        err = launchInspectSlots(static_cast<const uint4*>(r->spans.ptr), r->lastSlots, static_cast<uint64_t*>(lookback.ptr),
+                                 ticketAndStatus, static_cast<uint2*>(r->inspectRects.ptr),
+                                 static_cast<uint32_t*>(r->inspectOffsets.ptr), nullptr);
+    uint32_t status[2] = {0, 0};
+    if (err == cudaSuccess) err = cudaMemcpyAsync(status, ticketAndStatus, sizeof(status), cudaMemcpyDeviceToHost, nullptr);
     if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
     if (err != cudaSuccess) return failCuda(err, "reading the frame's pairs");
+    if (status[1]) return fail(ATH_E_TIMEOUT, "a look-back wait gave up (bounded spin); the buffers were not read");
     out->slots = r->lastSlots;
     out->pairs = pairs;
     out->tiles = r->lastTiles;
     out->records = static_cast<const float*>(r->recs.ptr);
-    out->rects = static_cast<const uint32_t*>(r->rects.ptr);
+    out->rects = static_cast<const uint32_t*>(r->inspectRects.ptr);
     out->keys = static_cast<const uint32_t*>(r->keys.ptr);
-    out->offsets = static_cast<const uint32_t*>(r->offsets.ptr);
+    out->offsets = static_cast<const uint32_t*>(r->inspectOffsets.ptr);
     out->pair_keys = pairKeys;
     out->pair_splats = static_cast<const uint32_t*>(r->inspectSplats.ptr);
     out->ranges = reinterpret_cast<const uint32_t*>(r->ranges);

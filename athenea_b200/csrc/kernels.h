@@ -18,22 +18,25 @@ FrameConst frameConstFor(const ath_projection& p, const ath_settings& s);
 InstanceConst instanceConstFor(const ath_projection& p, const ath_settings& s, const ath_instance& in, uint32_t base);
 
 // project.cu
-uint32_t projectBlocks(uint32_t slots);   // also the look-back words of the projection, and of the emit
-// masks: a 64-bit word a slot, the tiles of its rect it touches (rects of at most 64 tiles).
+uint32_t projectBlocks(uint32_t slots);   // also the look-back words of the emit
+// spans: 16 bytes a slot, its rect and the tiles of it that it touches (project.cu).
 // inst: the instances in device memory; a single one is passed by value, `one`, and needs none.
 cudaError_t launchProject(const FrameConst& F, const InstanceConst& one, const InstanceConst* inst, uint32_t nInst, uint32_t slots,
-                          uint32_t layout, bool countCulls, float4* recs, uint2* rects, unsigned long long* masks,
-                          uint32_t* keys, uint32_t* offsets, uint64_t* flags, uint32_t* words, cudaStream_t stream);
+                          uint32_t layout, bool countCulls, float4* recs, uint4* spans, uint32_t* keys, uint32_t* words,
+                          cudaStream_t stream);
 // The pairs (tile << 32 | slot) of the slots in `order` (the depth sort's). Writes the pairs the
 // buffers hold, min(pairs, capacity), into words[kWordPairsKept], and raises kStatusPairOverflow in
 // words[kWordSticky] past the capacity. flags: projectBlocks(slots) words, zeroed by the caller.
 cudaError_t launchEmit(const FrameConst& F, uint32_t slots, const uint32_t* order, const float4* recs,
-                       const uint2* rects, const unsigned long long* masks, const uint32_t* keys,
-                       const uint32_t* offsets, uint64_t* flags, uint32_t* words, uint64_t capacity, uint64_t* pairs,
+                       const uint4* spans, uint64_t* flags, uint32_t* words, uint64_t capacity, uint64_t* pairs,
                        cudaStream_t stream);
 // Ranges over the sorted pairs, *pairsDevice of them, at most `pairs`.
 cudaError_t launchRanges(uint32_t pairs, const uint32_t* pairsDevice, uint32_t tiles, const uint64_t* sorted,
                          uint2* ranges, uint32_t* status, cudaStream_t stream);
+// The slots' rects and first pairs, for inspection. flags (projectBlocks(slots) words) and
+// ticketAndStatus (two): zeroed by the caller.
+cudaError_t launchInspectSlots(const uint4* spans, uint32_t slots, uint64_t* flags, uint32_t* ticketAndStatus,
+                               uint2* rects, uint32_t* offsets, cudaStream_t stream);
 // The sorted pairs as (tile << 24 | depth key) and slot, for inspection.
 cudaError_t launchInspectPairs(const uint64_t* pairs, uint32_t count, const uint32_t* keys, uint32_t slots,
                                uint64_t* pairKeys, uint32_t* pairSplats, cudaStream_t stream);

@@ -136,38 +136,44 @@ __device__ __forceinline__ uint32_t warpInclusive(uint32_t v) {
     return v;
 }
 
-// The tiles a splat touches, found by its warp: bit k for tile k of its rect, row-major,
-// kept for a rect of at most kMaskTiles tiles; a larger one's tiles are tested again
-// where its pairs are written.
+// What the emit reads of a slot, 16 bytes, so that its walk in depth order touches one
+// sector a splat: the rect (x0 | y0 << 16, x1 | y1 << 16) and the tiles of it the splat
+// touches, bit k of (z, w) for tile k, row-major. A rect of more than kMaskTiles tiles has
+// their number in z, and its tiles are tested again where its pairs are written. A culled
+// slot is all zeros.
 constexpr uint32_t kMaskTiles = 64;
+__device__ __forceinline__ void spanShape(uint4 s, uint32_t& cols, uint32_t& area, uint32_t& touched) {
+    cols = (s.y & 0xFFFFu) - (s.x & 0xFFFFu) + 1;
+    area = cols * ((s.y >> 16) - (s.x >> 16) + 1);
+    touched = area > kMaskTiles ? s.z : __popc(s.z) + __popc(s.w);
+}
 
 // One thread a slot: projectSplat<0>, its record, rect and key. The tiles are tested by
 // warps: the candidates of a warp's 32 footprints (each footprint's screen rect, row-major)
 // are one list, lane l taking entry 32 c + l, so a warp's work is the sum of its rects,
-// where a thread a footprint took 32 times the largest. 1.5M splats at
-// 1920x1080 406 -> 201 us, 6M at 3840x2160 4.52 -> 1.22 ms.
+// where a thread a footprint took 32 times the largest. The warps of a block wait for each
+// other nowhere (but where a frame counts): the last to end adds the block's sums. 1.5M
+// splats at 1920x1080: 406 us, by lists 201, without a scan among the blocks 154; 6M at
+// 3840x2160: 4.52 ms, 1.23, 1.07.
 // kOne: a single instance, its constants among the kernel's.
 template <uint32_t L, bool kOne>
 __global__ void __launch_bounds__(kProjectThreads)
     projectKernel(const FrameConst F, const __grid_constant__ InstanceConst one, const InstanceConst* __restrict__ inst,
                   uint32_t nInst, uint32_t slots,
-                  uint32_t countCulls, float4* __restrict__ recs, uint2* __restrict__ rects,
-                  unsigned long long* __restrict__ masks, uint32_t* __restrict__ keys, uint32_t* __restrict__ offsets,
-                  uint64_t* __restrict__ flags, uint32_t* __restrict__ words) {
-    __shared__ uint32_t sTicket;
-    __shared__ uint32_t sWarp[kProjectThreads / 32];
-    __shared__ uint64_t sPrefix;
+                  uint32_t countCulls, float4* __restrict__ recs, uint4* __restrict__ spans,
+                  uint32_t* __restrict__ keys, uint32_t* __restrict__ words) {
+    __shared__ unsigned long long sPairs;
+    __shared__ uint32_t sKept, sEnded;
     __shared__ uint32_t sCulled[8];
     __shared__ uint32_t sCloud[2 * kMaxClouds];   // count_splats: (visible, pairs) a cloud, this block's share
     __shared__ float4 sFoot[kProjectThreads];     // cx cy ca cb
     __shared__ float2 sFootRest[kProjectThreads]; // cc cutoff
     __shared__ uint4 sRect[kProjectThreads];      // rx0 ry0 cols
-    if (threadIdx.x == 0) sTicket = atomicAdd(&words[kWordTicket], 1u);
+    if (threadIdx.x == 0) sPairs = 0, sKept = sEnded = 0;
     if (threadIdx.x < 8) sCulled[threadIdx.x] = 0;
     if (countCulls && threadIdx.x < 2 * kMaxClouds) sCloud[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t b = sTicket;
-    const uint32_t slot = b * kProjectThreads + threadIdx.x;
+    const uint32_t slot = blockIdx.x * kProjectThreads + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t area = 0, key = kCulledKey, cloud = 0;
     uint2 rect = make_uint2(0, 0);
@@ -271,10 +277,8 @@ __global__ void __launch_bounds__(kProjectThreads)
     }
     if (slot < slots) {
         keys[slot] = key;
-        if (kept) {
-            rects[slot] = rect;
-            masks[slot] = mask;
-        }
+        const uint2 bits = area > kMaskTiles ? make_uint2(touched, 0) : make_uint2((uint32_t)mask, (uint32_t)(mask >> 32));
+        spans[slot] = kept ? make_uint4(rect.x, rect.y, bits.x, bits.y) : make_uint4(0, 0, 0, 0);
         if (countCulls && !kept) atomicAdd(&sCulled[key & 7u], 1u);
         // splatCountersCloud's rows (TileRasterizer.cpp:1335-1346): the first 64 clouds one by one
         if (countCulls && kept && cloud < kMaxClouds) {
@@ -282,40 +286,29 @@ __global__ void __launch_bounds__(kProjectThreads)
             atomicAdd(&sCloud[2 * cloud + 1], touched);
         }
     }
-    // block-wide exclusive scan of `touched`
-    const uint32_t incl = warpInclusive(touched);
-    if (lane == 31) sWarp[warp] = incl;
-    const uint32_t keptCount = __syncthreads_count(kept);
-    uint32_t warpBase = 0, blockTotal = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kProjectThreads / 32; ++w) {
-        const uint32_t v = sWarp[w];
-        warpBase += w < warp ? v : 0u;
-        blockTotal += v;
-    }
-    if (warp == 0) {
-        const uint64_t prefix = lookbackExclusive(flags, b, blockTotal, &words[kWordStatus]);
-        if (lane == 0) {
-            sPrefix = prefix;
-            if (keptCount) atomicAdd(&words[kWordVisible], keptCount);
-            if (b == gridDim.x - 1) {
-                const uint64_t total = prefix + blockTotal;
-                words[kWordPairsLo] = (uint32_t)total;
-                words[kWordPairsHi] = (uint32_t)(total >> 32);
+    // the block's sums, added by the last of its warps to get here
+    const uint32_t warpKept = __popc(__ballot_sync(0xFFFFFFFFu, kept));
+    const uint32_t warpPairs = __reduce_add_sync(0xFFFFFFFFu, touched);
+    if (lane == 0) {
+        if (warpKept) {
+            atomicAdd(&sPairs, (unsigned long long)warpPairs);
+            atomicAdd(&sKept, warpKept);
+        }
+        __threadfence_block();
+        if (atomicAdd(&sEnded, 1u) == kProjectThreads / 32 - 1) {
+            __threadfence_block();
+            if (const uint32_t all = atomicAdd(&sKept, 0u)) {
+                atomicAdd(&words[kWordVisible], all);
+                atomicAdd(reinterpret_cast<unsigned long long*>(&words[kWordPairsLo]), atomicAdd(&sPairs, 0ull));
             }
         }
     }
-    if (countCulls) {
-        uint32_t most = touched;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
-        if (lane == 0 && most) atomicMax(&words[kWordMaxTiles], most);
-    }
+    if (!countCulls) return;
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, touched);
+    if (lane == 0 && most) atomicMax(&words[kWordMaxTiles], most);
     __syncthreads();
-    if (countCulls && threadIdx.x < 7 && sCulled[threadIdx.x]) atomicAdd(&words[kWordCulled + threadIdx.x], sCulled[threadIdx.x]);
-    if (countCulls && threadIdx.x < 2 * kMaxClouds && sCloud[threadIdx.x])
-        atomicAdd(&words[kWordClouds + threadIdx.x], sCloud[threadIdx.x]);
-    if (slot < slots) offsets[slot] = (uint32_t)(sPrefix + (incl - touched) + warpBase);
+    if (threadIdx.x < 7 && sCulled[threadIdx.x]) atomicAdd(&words[kWordCulled + threadIdx.x], sCulled[threadIdx.x]);
+    if (threadIdx.x < 2 * kMaxClouds && sCloud[threadIdx.x]) atomicAdd(&words[kWordClouds + threadIdx.x], sCloud[threadIdx.x]);
 }
 
 // Bit `k` (counted from the least) of the set bits of a 64-bit word.
@@ -343,12 +336,13 @@ __device__ __forceinline__ uint32_t setBit(uint32_t lo, uint32_t hi, uint32_t k)
 // touched tile, row-major over the splat's rect. A stable sort by tile then leaves each
 // tile its splats in (depth key, slot) order (splat/frame.slang:17-20). A warp writes its
 // 32 splats' pairs as one list, lane l pair 32 c + l, from the masks of the tiles they
-// touch; where the splats' pairs start comes from a look-back over the blocks.
+// touch; where the splats' pairs start comes from a look-back over the blocks. Bound by
+// the splats' records, a sector each in depth order, and the pairs' writes. With rects,
+// masks, keys and offsets apart: 1.5M splats 102 us, so 92; 6M 692, so 621.
 __global__ void __launch_bounds__(kProjectThreads)
     emitKernel(const FrameConst F, uint32_t slots, const uint32_t* __restrict__ order, const float4* __restrict__ recs,
-               const uint2* __restrict__ rects, const unsigned long long* __restrict__ masks,
-               const uint32_t* __restrict__ keys, const uint32_t* __restrict__ offsets, uint64_t* __restrict__ flags,
-               uint32_t* __restrict__ words, uint64_t capacity, uint64_t* __restrict__ pairs) {
+               const uint4* __restrict__ spans, uint64_t* __restrict__ flags, uint32_t* __restrict__ words,
+               uint64_t capacity, uint64_t* __restrict__ pairs) {
     __shared__ uint32_t sTicket;
     __shared__ uint32_t sWarp[kProjectThreads / 32];
     __shared__ uint64_t sPrefix;
@@ -363,19 +357,13 @@ __global__ void __launch_bounds__(kProjectThreads)
         words[kWordPairsKept] = (uint32_t)min(all, capacity);
         if (all > capacity) atomicOr(&words[kWordSticky], kStatusPairOverflow);
     }
-    uint32_t slot = 0, touched = 0, cols = 1, area = 0;
-    uint2 rect = make_uint2(0, 0);
-    unsigned long long mask = 0;
+    uint32_t slot = 0, touched, cols, area;
+    uint4 span = make_uint4(0, 0, 0, 0);
     if (i < slots) {
         slot = order[i];
-        if (slot < slots && keys[slot] < kCulledKey) {
-            touched = (slot + 1 < slots ? offsets[slot + 1] : (uint32_t)all) - offsets[slot];
-            rect = rects[slot];
-            mask = masks[slot];
-            cols = (rect.y & 0xFFFFu) - (rect.x & 0xFFFFu) + 1;
-            area = cols * ((rect.y >> 16) - (rect.x >> 16) + 1);
-        }
+        if (slot < slots) span = spans[slot];
     }
+    spanShape(span, cols, area, touched);
     const uint32_t incl = warpInclusive(touched), excl = incl - touched;
     if (lane == 31) sWarp[warp] = incl;
     __syncthreads();
@@ -394,7 +382,7 @@ __global__ void __launch_bounds__(kProjectThreads)
     const uint64_t base = sPrefix + warpBase;
     const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     const bool large = area > kMaskTiles;
-    const uint32_t rect0 = rect.x, maskLo = (uint32_t)mask, maskHi = (uint32_t)(mask >> 32);
+    const uint32_t rect0 = span.x, maskLo = span.z, maskHi = span.w;
     const uint32_t tagged = slot, shape = cols | (large ? 1u << 31 : 0u);
     for (uint32_t q0 = 0; q0 < total; q0 += 32) {
         const uint32_t q = q0 + lane;
@@ -430,6 +418,40 @@ __global__ void __launch_bounds__(kProjectThreads)
             written += __popc(hits);
         }
     }
+}
+
+// The slots' rects, and the exclusive scan of the tiles they touch, for inspection.
+__global__ void __launch_bounds__(kProjectThreads)
+    inspectSlotsKernel(const uint4* __restrict__ spans, uint32_t slots, uint64_t* __restrict__ flags,
+                       uint32_t* __restrict__ ticketAndStatus, uint2* __restrict__ rects, uint32_t* __restrict__ offsets) {
+    __shared__ uint32_t sTicket;
+    __shared__ uint32_t sWarp[kProjectThreads / 32];
+    __shared__ uint64_t sPrefix;
+    if (threadIdx.x == 0) sTicket = atomicAdd(&ticketAndStatus[0], 1u);
+    __syncthreads();
+    const uint32_t b = sTicket, slot = b * kProjectThreads + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint4 span = slot < slots ? spans[slot] : make_uint4(0, 0, 0, 0);
+    uint32_t cols, area, touched;
+    spanShape(span, cols, area, touched);
+    const uint32_t incl = warpInclusive(touched);
+    if (lane == 31) sWarp[warp] = incl;
+    __syncthreads();
+    uint32_t warpBase = 0, blockTotal = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kProjectThreads / 32; ++w) {
+        const uint32_t v = sWarp[w];
+        warpBase += w < warp ? v : 0u;
+        blockTotal += v;
+    }
+    if (warp == 0) {
+        const uint64_t prefix = lookbackExclusive(flags, b, blockTotal, &ticketAndStatus[1]);
+        if (lane == 0) sPrefix = prefix;
+    }
+    __syncthreads();
+    if (slot >= slots) return;
+    rects[slot] = make_uint2(span.x, span.y);
+    offsets[slot] = (uint32_t)(sPrefix + (incl - touched) + warpBase);
 }
 
 // The sorted pairs as frame.slang's two sorts have them, for inspection: (tile << 24 |
@@ -491,13 +513,13 @@ __global__ void __launch_bounds__(256)
 }   // namespace
 
 cudaError_t launchProject(const FrameConst& F, const InstanceConst& one, const InstanceConst* inst, uint32_t nInst, uint32_t slots,
-                          uint32_t layout, bool countCulls, float4* recs, uint2* rects, unsigned long long* masks,
-                          uint32_t* keys, uint32_t* offsets, uint64_t* flags, uint32_t* words, cudaStream_t stream) {
+                          uint32_t layout, bool countCulls, float4* recs, uint4* spans, uint32_t* keys, uint32_t* words,
+                          cudaStream_t stream) {
     if (slots == 0) return cudaSuccess;
     const uint32_t cc = countCulls ? 1u : 0u;
 #define ATH_PROJECT(L_, O_)                                                                                        \
     projectKernel<L_, O_><<<projectBlocks(slots), kProjectThreads, 0, stream>>>(F, one, inst, nInst, slots, cc, recs, \
-                                                                               rects, masks, keys, offsets, flags, words)
+                                                                               spans, keys, words)
     if (layout == kLayoutPacked && nInst == 1) ATH_PROJECT(kLayoutPacked, true);
     else if (layout == kLayoutPacked) ATH_PROJECT(kLayoutPacked, false);
     else ATH_PROJECT(kLayoutParams, true);
@@ -508,11 +530,17 @@ cudaError_t launchProject(const FrameConst& F, const InstanceConst& one, const I
 uint32_t projectBlocks(uint32_t slots) { return (slots + kProjectThreads - 1) / kProjectThreads; }
 
 cudaError_t launchEmit(const FrameConst& F, uint32_t slots, const uint32_t* order, const float4* recs,
-                       const uint2* rects, const unsigned long long* masks, const uint32_t* keys,
-                       const uint32_t* offsets, uint64_t* flags, uint32_t* words, uint64_t capacity, uint64_t* pairs,
+                       const uint4* spans, uint64_t* flags, uint32_t* words, uint64_t capacity, uint64_t* pairs,
                        cudaStream_t stream) {
     emitKernel<<<std::max(1u, projectBlocks(slots)), kProjectThreads, 0, stream>>>(
-        F, slots, order, recs, rects, masks, keys, offsets, flags, words, capacity, pairs);
+        F, slots, order, recs, spans, flags, words, capacity, pairs);
+    return cudaGetLastError();
+}
+
+cudaError_t launchInspectSlots(const uint4* spans, uint32_t slots, uint64_t* flags, uint32_t* ticketAndStatus,
+                               uint2* rects, uint32_t* offsets, cudaStream_t stream) {
+    if (slots == 0) return cudaSuccess;
+    inspectSlotsKernel<<<projectBlocks(slots), kProjectThreads, 0, stream>>>(spans, slots, flags, ticketAndStatus, rects, offsets);
     return cudaGetLastError();
 }
 

@@ -63,11 +63,9 @@ struct InstanceConst {
 // counts), so nothing waits for them.
 constexpr uint32_t kMaxClouds = 64;   // SplatCounters::kMaxClouds (TileRasterizer.h:376)
 enum FrameWord : uint32_t {
-    kWordTicket = 0,        // the projection's block ticket
-    kWordVisible = 1,       // splats kept
-    kWordStatus = 2,        // kStatus* bits of the projection's scan
-    kWordPairsLo = 3,       // pairs (the sum of tiles touched), 64-bit
-    kWordPairsHi = 4,
+    kWordVisible = 0,       // splats kept
+    kWordPairsLo = 2,       // pairs (the sum of tiles touched), 64-bit and aligned so
+    kWordPairsHi = 3,
     kWordMaxTiles = 5,
     kWordCulled = 6,        // 7 words: culled by reason (count_splats)
     kWordPairsKept = 13,    // the pairs the buffers hold: min(pairs, capacity), what the sort sorts
