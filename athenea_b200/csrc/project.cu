@@ -338,8 +338,8 @@ __device__ __forceinline__ uint32_t setBit(uint32_t lo, uint32_t hi, uint32_t k)
 // 32 splats' pairs as one list, lane l pair 32 c + l, from the masks of the tiles they
 // touch; where the splats' pairs start comes from a look-back over the blocks. Bound by
 // the splats' records, a sector each in depth order, and the pairs' writes. With rects,
-// masks, keys and offsets apart: 1.5M splats 102 us, so 92; 6M 692, so 621.
-__global__ void __launch_bounds__(kProjectThreads)
+// masks, keys and offsets apart: 1.5M splats 102 us, so 73; 6M 692, so 515.
+__global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by five blocks an SM 91 and 619 us
     emitKernel(const FrameConst F, uint32_t slots, const uint32_t* __restrict__ order, const float4* __restrict__ recs,
                const uint4* __restrict__ spans, uint64_t* __restrict__ flags, uint32_t* __restrict__ words,
                uint64_t capacity, uint64_t* __restrict__ pairs) {
