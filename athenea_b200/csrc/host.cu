@@ -519,8 +519,8 @@ TrainingState trainingState(const ath_raster* r) {
                          static_cast<uint32_t*>(r->live.ptr), r->trainingOnePixel};
 }
 
-// One frame: project (scan fused), emit, sort, ranges, blend, with nothing read
-// back in between. The pairs are sized from a capacity: a handle's first frame
+// One frame: project, sort the splats by depth, emit, sort the pairs by tile, ranges,
+// blend, with nothing read back in between. The pairs are sized from a capacity: a handle's first frame
 // (and its first after release_scratch) reads the pair total back once and sizes
 // them exactly, as the reference does every frame (TileRasterizer.cpp:1093-1102);
 // later frames use the capacity the earlier ones needed. A frame whose pairs
@@ -529,7 +529,7 @@ TrainingState trainingState(const ath_raster* r) {
 // the pair count from the device. At its end the frame's words are copied to
 // pinned memory behind an event (its status, for ath_raster_check), and, when it
 // counts, to the counters' ring. `staged` is the instance table in host memory
-// (pinned staging). `training` also keeps, per pixel, the final transmittance
+// (pageable: copied before the call returns). `training` also keeps, per pixel, the final transmittance
 // and the last record blended, for the backward.
 ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, uint32_t instanceCount,
                      uint32_t slots, uint32_t layout, const ath_settings& s, ath_targets* targets,

@@ -1,10 +1,11 @@
 // Stage (a): per-Gaussian projection -- splat/splat_project.slang:497-785 and
 // :1080-1129 (projectSplat<0>, the plain entry splatProjectPlain) -- with the
-// exclusive scan of the tiles each splat touches fused in (the reference runs
-// PrefixSum::apply over them afterwards, TileRasterizer.cpp:1088-1089).
+// tiles each splat touches.
 // Stage (b): the pairs, (tile, slot), in depth order (splat/splat_emit.slang:17-50 over
-// the depth sort's slots, as the reference), whose stable sort by tile (sort.cu) gives each
-// tile its splats front to back; and the tiles' ranges (splat/splat_ranges.slang:11-25).
+// the depth sort's slots, as the reference; the scan of their counts, which the reference
+// runs as PrefixSum::apply, TileRasterizer.cpp:1088-1089, is fused in), whose stable sort by
+// tile (sort.cu) gives each tile its splats front to back; and the tiles' ranges
+// (splat/splat_ranges.slang:11-25).
 //
 // Built with --fmad=false: see splat_math.cuh.
 #include <algorithm>

@@ -148,7 +148,7 @@ constexpr size_t onesweepSmem() {
     return rankSmem<K, kBits, kPerThread>() + ((size_t)rankChains<kBits, kPerThread>() << kBits) * 4;
 }
 
-// kBits: the pass's digit width, 8 or 9 (kRadixT digits, one thread each in the
+// kBits: the pass's digit width, 8 or 9 (its digits one thread each in the
 // digit phase; a 9-bit pass ranks in one chain, so that its counters fit beside the keys).
 // The values take the keys' shared memory once the keys are out, each thread keeping its
 // items' places in the tile and its outputs' destinations in registers: with values as
