@@ -242,11 +242,21 @@ __global__ void __launch_bounds__(256)
             some = some || v.x != 0.0f || v.y != 0.0f;
         }
     }
-    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, some);
-    uint32_t first = 0;
-    if (lane == 0 && ballot) first = atomicAdd(listed, (uint32_t)__popc(ballot));
-    first = __shfl_sync(0xFFFFFFFFu, first, 0);
-    if (some) list[first + __popc(ballot & ((1u << lane) - 1u))] = slot;
+    // a block's places by one addition: one a warp, all to one word, was most of the
+    // kernel (500k Gaussians: 14 us, so 7)
+    __shared__ uint32_t sCount[8], sFirst;
+    const uint32_t warp = threadIdx.x >> 5, ballot = __ballot_sync(0xFFFFFFFFu, some);
+    if (lane == 0) sCount[warp] = __popc(ballot);
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; ++w) {
+        before += w < warp ? sCount[w] : 0u;
+        all += sCount[w];
+    }
+    if (threadIdx.x == 0 && all) sFirst = atomicAdd(listed, all);
+    __syncthreads();
+    if (some) list[sFirst + before + __popc(ballot & ((1u << lane) - 1u))] = slot;
 }
 
 // The projection's adjoint, one thread a listed Gaussian: dL/d(record) -> dL/d(parameters),
@@ -255,7 +265,7 @@ __global__ void __launch_bounds__(256)
 // place, and the warp adds the rows to the gradients a row at a time: every access covers
 // whole sectors, where a lane at its own row touched a line a load.
 // Over every slot in order, each thread its own rows: 500k Gaussians at 1280x720, degree 3,
-// 308 us; the list 14 and this 49.
+// 308 us; the list 7 and this 49.
 constexpr uint32_t kRowsAtOnce = 8;   // of rows that are not whole pieces
 
 __global__ void __launch_bounds__(128)
