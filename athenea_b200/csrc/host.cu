@@ -415,8 +415,9 @@ extern "C" ath_status ath_raster_latest_counters(ath_raster* r, ath_splat_counte
 namespace {
 
 ath_status reserveSlots(ath_raster* r, uint32_t slots) {   // reserveSplats (TileRasterizer.cpp:193-226)
-    if (slots <= r->slotCapacity && r->recs.bytes) return ATH_OK;
+    if (slots <= r->slotCapacity) return ATH_OK;
     const uint32_t n = r->tight ? slots : grow(r->slotCapacity, slots);
+    r->slotCapacity = 0;   // no slots until every array has them: an array that grows gives up its old memory first
     cudaError_t err = r->recs.reserve((size_t)n * 48);
     if (err == cudaSuccess) err = r->spans.reserve((size_t)n * 16);
     if (err == cudaSuccess) err = r->keys.reserve((size_t)n * 4);
@@ -432,8 +433,9 @@ ath_status reserveSlots(ath_raster* r, uint32_t slots) {   // reserveSplats (Til
 const size_t kSortHistBytes = sortHistWords() * sizeof(uint32_t);
 
 ath_status reservePairs(ath_raster* r, uint32_t pairs, uint32_t bits) {   // reservePairs (:228-247)
-    if (pairs > r->pairCapacity || !r->pairs[0].bytes) {
+    if (pairs > r->pairCapacity) {
         const uint32_t n = r->tight ? pairs : grow(r->pairCapacity, pairs);
+        r->pairCapacity = 0;   // as the slots
         cudaError_t err = cudaSuccess;
         for (int k = 0; k < 2 && err == cudaSuccess; ++k) err = r->pairs[k].reserve((size_t)n * 8);
         if (err != cudaSuccess) return failCuda(err, "reserving the pairs");
@@ -560,7 +562,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     uint32_t* words = reinterpret_cast<uint32_t*>(zero + zeroed.words);
     uint32_t* wordsHost = static_cast<uint32_t*>(r->wordsHost.ptr);
     const bool timed = s.time_stages != 0;
-    const bool sizing = r->pairCapacity == 0 || !r->pairs[0].bytes;   // no capacity yet: read the total once
+    const bool sizing = r->pairCapacity == 0;   // no capacity yet: read the total once
     auto mark = [&](int k) { if (timed) cudaEventRecord(r->marks[k], stream); };
 
     // --- project ----------------------------------------------------------

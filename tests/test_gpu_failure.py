@@ -3,6 +3,8 @@ reference's ATHENEA_GPU_BUDGET, modules/gpu/src/Device.cpp:434-449) turning an
 allocation into OutOfMemory on the host side, and the library's bounded
 device-side wait running out on a flag nothing sets, with the context usable
 after both."""
+import functools
+
 import numpy as np
 import pytest
 import torch
@@ -13,12 +15,13 @@ from tests.fixtures import ENC_BUILDER, CloudBuilder, product_encoding
 pytestmark = pytest.mark.gpu
 
 
-def _cloud():
+@functools.lru_cache
+def _cloud(count=200, size=0.05):
     b = CloudBuilder()
     rng = np.random.default_rng(5)
-    for _ in range(200):
+    for _ in range(count):
         x, y, z = rng.uniform(-1, 1, 3)
-        b.add(x, y, z, 0.8, 0.05, 0.05, 0.05, (1, 0, 0, 0), tuple(rng.uniform(0, 1, 3)))
+        b.add(x, y, z, 0.8, size, size, size, (1, 0, 0, 0), tuple(rng.uniform(0, 1, 3)))
     recs = torch.from_numpy(b.records().reshape(-1)).cuda()
     return A.CloudLoader.upload(recs, product_encoding(ENC_BUILDER), 3)
 
@@ -51,6 +54,33 @@ def test_a_budget_turns_scratch_into_out_of_memory_and_release_gives_it_back(nat
         assert budget == 0 and held_after > 0
         raster.release_scratch()
         assert A.memory_held()[0] < held_after
+    finally:
+        A.set_memory_budget(0)
+
+
+# The budget admits a part of what a larger frame of the handle asks for, so that some of its buffers have grown when
+# one cannot: the next frame, small enough for what the handle had, asks for all of them again.
+@pytest.mark.parametrize("part", [0.02, 0.2, 0.5, 0.6, 0.75, 0.9])
+def test_a_growth_that_fails_part_way_leaves_a_handle_that_draws(native, part):
+    import gc
+    small, large = _cloud(), _cloud(60_000, 0.02)
+    want = _frame(A.TileRasterizer.create(), small)
+    raster, other = A.TileRasterizer.create(), A.TileRasterizer.create()
+    np.testing.assert_array_equal(_frame(raster, small), want)
+    gc.collect()
+    before = A.memory_held()[0]
+    whole = _frame(other, large, 640, 480)
+    need = A.memory_held()[0] - before
+    del other
+    gc.collect()
+    try:
+        A.set_memory_budget(A.memory_held()[0] + int(part * need))
+        with pytest.raises(A.AtheneaError) as e:
+            _frame(raster, large, 640, 480)
+        assert e.value.code == 9                    # OutOfMemory
+        A.set_memory_budget(0)
+        np.testing.assert_array_equal(_frame(raster, small), want)
+        np.testing.assert_array_equal(_frame(raster, large, 640, 480), whole)
     finally:
         A.set_memory_budget(0)
 
