@@ -537,6 +537,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                      uint32_t slots, uint32_t layout, const ath_settings& s, ath_targets* targets,
                      ath_frame_stats* stats, cudaStream_t stream, bool training, const ath_targets* under = nullptr) {
     const auto frameStart = std::chrono::steady_clock::now();
+    r->ranges = nullptr;   // until this frame is whole, nothing to inspect: growing gives up what the last one left
     const uint32_t tiles = F.tilesX * F.tilesY;
     const uint32_t bits = F.tileBits;   // the pairs sort by tile alone, their splats in depth order already
     ath_status st = reserveSlots(r, std::max(slots, 1u));
@@ -874,7 +875,7 @@ extern "C" ath_status ath_l2_loss(const float* colour, const float* target, uint
 
 extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers* out) {
     if (!r || !out) return fail(ATH_E_INVALID_ARGUMENT, "ath_raster_frame_buffers: null argument");
-    if (!r->recs.ptr || !r->frameRecorded) return fail(ATH_E_NOT_FOUND, "no frame has been drawn since the scratch was made");
+    if (!r->ranges) return fail(ATH_E_NOT_FOUND, "the handle holds no frame: none drawn since its scratch was made, or the last one failed");
     DeviceGuard guard(r->device);
     // inspection: waits for the frame, whose pair count only the device knew
     if (const cudaError_t err = cudaEventSynchronize(r->frameDone); err != cudaSuccess)

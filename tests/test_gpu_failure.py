@@ -11,6 +11,7 @@ import torch
 
 import athenea_b200 as A
 from tests.fixtures import ENC_BUILDER, CloudBuilder, product_encoding
+from tests.gpu_helpers import frame_buffers
 
 pytestmark = pytest.mark.gpu
 
@@ -83,6 +84,26 @@ def test_a_growth_that_fails_part_way_leaves_a_handle_that_draws(native, part):
         np.testing.assert_array_equal(_frame(raster, large, 640, 480), whole)
     finally:
         A.set_memory_budget(0)
+
+
+def test_a_failed_frame_leaves_nothing_to_inspect(native):
+    small, large = _cloud(), _cloud(60_000, 0.02)
+    raster = A.TileRasterizer.create()
+    _frame(raster, small)
+    want = frame_buffers(raster)
+    try:
+        A.set_memory_budget(1)
+        with pytest.raises(A.AtheneaError) as e:
+            _frame(raster, large, 640, 480)
+        assert e.value.code == 9                    # OutOfMemory
+        with pytest.raises(A.AtheneaError) as e:
+            frame_buffers(raster)
+        assert e.value.code == 2                    # NotFound
+    finally:
+        A.set_memory_budget(0)
+    _frame(raster, small)
+    for name, value in frame_buffers(raster).items():
+        np.testing.assert_array_equal(value, want[name], err_msg=name)
 
 
 def test_a_wait_on_a_flag_nothing_sets_gives_up_with_timeout(native):
