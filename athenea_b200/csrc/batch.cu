@@ -1225,15 +1225,15 @@ ath_status sizePairs(ath_batch* b, const ath_mixed_params& P, cudaStream_t strea
     b->planWide = wide;
     b->depthBits = wide ? 24u : depthBits;
     b->expBase = wide ? 0u : expBase;
-    if (want > b->capacity || !b->pairs[0].ptr || (wide && !b->values[0].ptr)) {
-        const uint64_t room = std::max<uint64_t>(want, b->capacity);
-        for (int k = 0; k < 2; ++k) {
-            if ((err = b->pairs[k].reserve((size_t)room * 8)) != cudaSuccess) return failCuda(err, "reserving the pairs");
-            if (wide && (err = b->values[k].reserve((size_t)room * 4)) != cudaSuccess)
-                return failCuda(err, "reserving the pairs' Gaussians");
-        }
-        b->capacity = room;
+    // every buffer by its own size: a wide plan after a packed one that grew the pairs finds
+    // its values short of the capacity
+    const uint64_t room = std::max<uint64_t>(want, b->capacity);
+    for (int k = 0; k < 2; ++k) {
+        if ((err = b->pairs[k].reserve((size_t)room * 8)) != cudaSuccess) return failCuda(err, "reserving the pairs");
+        if (wide && (err = b->values[k].reserve((size_t)room * 4)) != cudaSuccess)
+            return failCuda(err, "reserving the pairs' Gaussians");
     }
+    b->capacity = room;
     const uint32_t bits = b->depthBits + b->tileBits;
     err = b->sortFlags.reserve(sortFlagWords((uint32_t)b->capacity, bits, b->planWide) * 8);
     if (err != cudaSuccess) return failCuda(err, "reserving the sort's look-back words");

@@ -144,3 +144,21 @@ def test_the_pair_form_switched_between_steps_draws_the_same_image():
             np.testing.assert_array_equal(img, first[0], err_msg=f"key mode {mode}")
             assert stats["pairs"] == first[1]
             assert abs(loss.item() - first[2]) <= 1e-5 * first[2]
+
+
+def test_wide_pairs_after_a_packed_step_that_grew_draw_as_a_fresh_trainer():
+    """The wide form's own arrays follow the pairs' capacity, whichever form grew it: a wide step on a small cloud,
+    a packed one on a larger, then a wide one on the larger."""
+    _, M = _scene(60_000, 26)
+    views = _views()
+    gen = torch.Generator().manual_seed(26)
+    targets = [torch.rand((W * H, 3), generator=gen).cuda() for _, W, H in views]
+    b = BatchTrainer()
+    for mode, n in ((2, 500), (1, 60_000), (2, 60_000)):
+        part = MixedParams(M.means[:n], M.scales[:n], M.quats[:n], M.sh_low[:n], M.sh_high[:n], M.sh_scale[:n], 3)
+        b.set_key_mode(mode)
+        _, colour, loss, _, stats = _batched(part, views, targets, trainer=b)
+        _, fresh, fresh_loss, _, fresh_stats = _batched(part, views, targets)
+        np.testing.assert_array_equal(colour.cpu().numpy(), fresh.cpu().numpy(), err_msg=f"mode {mode}, {n} Gaussians")
+        assert stats["pairs"] == fresh_stats["pairs"] and stats["kept"] == fresh_stats["kept"]
+        assert abs(loss.item() - fresh_loss.item()) <= 1e-5 * fresh_loss.item()
