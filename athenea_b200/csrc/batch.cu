@@ -1225,8 +1225,8 @@ ath_status sizePairs(ath_batch* b, const ath_mixed_params& P, cudaStream_t strea
     b->planWide = wide;
     b->depthBits = wide ? 24u : depthBits;
     b->expBase = wide ? 0u : expBase;
-    // every buffer by its own size: a wide plan after a packed one that grew the pairs finds
-    // its values short of the capacity
+    // every buffer by its own size: a wide plan after a packed one that grew the pairs, or a
+    // growth that failed between them, finds some short of the capacity
     const uint64_t room = std::max<uint64_t>(want, b->capacity);
     for (int k = 0; k < 2; ++k) {
         if ((err = b->pairs[k].reserve((size_t)room * 8)) != cudaSuccess) return failCuda(err, "reserving the pairs");
@@ -1384,9 +1384,11 @@ ath_status runStep(ath_batch* b, const ath_mixed_params* params, const float* ta
     // the buffers a view, a tile or a Gaussian holds: grown whenever the cloud, the
     // views or the tile size changed (set_views and set_tuning mark a resize)
     if (P.count != b->count || b->resize) {
-        if ((st = reserveBatch(b, P.count)) != ATH_OK) return st;
+        // first, for a growth that fails gives up old memory that captured steps use: the next
+        // step, whatever its size, sizes and captures again
         b->resize = true;
         dropGraph(b);
+        if ((st = reserveBatch(b, P.count)) != ATH_OK) return st;
     }
     placeCloud(b, P.object_to_world);
     cudaError_t err = cudaMemcpyAsync(b->viewsDev.ptr, b->views.data(), b->views.size() * sizeof(BatchView),

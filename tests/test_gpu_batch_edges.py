@@ -162,3 +162,36 @@ def test_wide_pairs_after_a_packed_step_that_grew_draw_as_a_fresh_trainer():
         np.testing.assert_array_equal(colour.cpu().numpy(), fresh.cpu().numpy(), err_msg=f"mode {mode}, {n} Gaussians")
         assert stats["pairs"] == fresh_stats["pairs"] and stats["kept"] == fresh_stats["kept"]
         assert abs(loss.item() - fresh_loss.item()) <= 1e-5 * fresh_loss.item()
+
+
+# as for a frame's growth (test_gpu_failure.py): a part of what the larger step asks for fits, then the same steps again
+@pytest.mark.parametrize("part_of_need", [0.02, 0.2, 0.4, 0.6, 0.75, 0.9])
+def test_a_batch_growth_that_fails_part_way_leaves_a_trainer_that_steps(part_of_need):
+    import gc
+    _, M = _scene(60_000, 27)
+    views = _views()
+    gen = torch.Generator().manual_seed(27)
+    targets = [torch.rand((W * H, 3), generator=gen).cuda() for _, W, H in views]
+    part = lambda n: MixedParams(M.means[:n], M.scales[:n], M.quats[:n], M.sh_low[:n], M.sh_high[:n],  # noqa: E731
+                                 M.sh_scale[:n], 3)
+    small, small_image = part(500), None
+    gc.collect()
+    before = A.memory_held()[0]
+    other, whole, *_ = _batched(M, views, targets)
+    need = A.memory_held()[0] - before
+    del other
+    gc.collect()
+    b = BatchTrainer()
+    _, small_image, *_ = _batched(small, views, targets, trainer=b)
+    has = A.memory_held()[0] - before
+    try:
+        A.set_memory_budget(before + has + int(part_of_need * (need - has)))
+        with pytest.raises(A.AtheneaError) as e:
+            _batched(M, views, targets, trainer=b)
+        assert e.value.code == 9                    # OutOfMemory
+        A.set_memory_budget(0)
+        for cloud, want in ((small, small_image), (M, whole)):
+            _, image, *_ = _batched(cloud, views, targets, trainer=b)
+            np.testing.assert_array_equal(image.cpu().numpy(), want.cpu().numpy())
+    finally:
+        A.set_memory_budget(0)
