@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
     const Px<kPx> yc = both<kPx>((float)py + 0.5f);
     Px<kPx> xc, T, dR, dG, dB, sd, rest, dDepth;
     uint32_t last[kPx], most = 0;
+    bool wild = false;   // a gradient that is not finite, or whose products may not be
 #pragma unroll
     for (int p = 0; p < kPx; ++p) {
         const uint32_t px = boxX + Box<kPx>::laneX(lane) + 4u * (uint32_t)p;
@@ -86,7 +87,8 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         xc.v[p] = (float)px + 0.5f;
         const float left = inside ? training.finalT[at] : 1.0f;
         last[p] = inside ? min(training.lastContrib[at], range.y - range.x) : 0u;
-        const float4 dC = inside ? dLdColour[at] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        // a pixel that blended nothing gives nothing, whatever its gradient holds
+        const float4 dC = last[p] ? dLdColour[at] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         T.v[p] = left;
         dR.v[p] = dC.x;
         dG.v[p] = dC.y;
@@ -98,17 +100,20 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         // channel's 1 - T + T bg_a, and the depth's division by the coverage
         rest.v[p] = dC.w * left * (1.0f - F.bg[3]);
         dDepth.v[p] = 0.0f;
-        if (kDepth && inside) {
+        if (kDepth && last[p]) {
             const float cov = 1.0f - left, dD = dLdDepth[at];
             if (cov > 1e-6f && dD != 0.0f) {
                 dDepth.v[p] = dD / cov;
                 rest.v[p] -= dDepth.v[p] * depthOut[at] * left;
             }
         }
+        const float size = ((fabsf(dC.x) + fabsf(dC.y)) + fabsf(dC.z)) + ((fabsf(sd.v[p]) + fabsf(rest.v[p])) + fabsf(dDepth.v[p]));
+        wild = wild || !(size < kWalkLimit);
         most = max(most, last[p]);
     }
     const uint32_t sumRecord = lane / kValues, sumValue = lane % kValues;   // the column this lane sums
     const float rowMid = (float)boxY + 0.5f * (float)Box<kPx>::kHeight;      // the box's middle row
+    wild = __any_sync(0xFFFFFFFFu, wild);
     const int32_t chunks = (int32_t)((__reduce_max_sync(0xFFFFFFFFu, most) + 31u) >> 5);
     const uint32_t* liveOf = training.live + ((size_t)(range.x >> 5) + tile) * Box<kPx>::kCount + warp;
     for (int32_t hi = chunks - 1; hi >= 0; hi -= 32) {
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 sh.records[lane].set(recs[(size_t)s * 3 + 0], recs[(size_t)s * 3 + 1], recs[(size_t)s * 3 + 2], s, rel + 1u);
             }
             __syncwarp();
-            const bool odd = __any_sync(0xFFFFFFFFu, lane < count && sh.records[lane].odd != 0u);
+            const bool odd = wild || __any_sync(0xFFFFFFFFu, lane < count && sh.records[lane].odd != 0u);
             auto walk = [&](auto oddHere) {
             constexpr bool kOdd = decltype(oddHere)::value;
             for (uint32_t q0 = 0; q0 < count; q0 += kRecords) {
@@ -164,17 +169,25 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     Px<kPx> Tb = T * inv;
                     Tb = fused(fused(om * both<kPx>(-1.0f), Tb, T), inv, Tb);
                     const Px<kPx> w = Tb * alpha;
-                    Px<kPx> cd = fused(Rec::px(R.bl), dB, fused(Rec::px(R.g), dG, Rec::px(R.r) * dR));
-                    if (kDepth) cd = fused(Rec::px(R.z), dDepth, cd);
+                    // where a colour or a gradient may not be finite, alpha 0 does not keep the pixels
+                    // that did not blend the record out of its sums: their terms are left out
+                    Px<kPx> vR = dR, vG = dG, vB = dB, vDepth = dDepth, vRest = rest;
+                    if (kOdd) {
+#pragma unroll
+                        for (int p = 0; p < kPx; ++p)
+                            if (!on[p]) vR.v[p] = vG.v[p] = vB.v[p] = vDepth.v[p] = vRest.v[p] = 0.0f;
+                    }
+                    Px<kPx> cd = fused(Rec::px(R.bl), vB, fused(Rec::px(R.g), vG, Rec::px(R.r) * vR));
+                    if (kDepth) cd = fused(Rec::px(R.z), vDepth, cd);
                     Px<kPx> u = fused(sd, both<kPx>(-1.0f), cd);
-                    if (kOdd && R.odd) {   // a colour that is not finite stays out of the pixels that did not blend it
+                    if (kOdd) {
 #pragma unroll
                         for (int p = 0; p < kPx; ++p)
                             if (!on[p]) u.v[p] = 0.0f;
                     }
                     // alpha dL/dalpha: the opacity times dL/dopacity, and -2 dL/dpower, where alpha is
                     // neither clamped nor of an opacity over 1
-                    Px<kPx> aDA = fused(alpha * inv, rest, w * u);
+                    Px<kPx> aDA = fused(alpha * inv, vRest, w * u);
                     sd = fused(alpha, u, sd);
                     T = Tb;
 #pragma unroll
@@ -185,10 +198,10 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     column[0 * kColumnStride] = sum(aDA);
                     column[1 * kColumnStride] = sum(x1);
                     column[2 * kColumnStride] = sum(x2);
-                    column[3 * kColumnStride] = sum(w * dR);
-                    column[4 * kColumnStride] = sum(w * dG);
-                    column[5 * kColumnStride] = sum(w * dB);
-                    if (kDepth) column[6 * kColumnStride] = sum(w * dDepth);
+                    column[3 * kColumnStride] = sum(w * vR);
+                    column[4 * kColumnStride] = sum(w * vG);
+                    column[5 * kColumnStride] = sum(w * vB);
+                    if (kDepth) column[6 * kColumnStride] = sum(w * vDepth);
                 }
                 __syncwarp();
                 // dL/dpower is -1/2 alpha dL/dalpha; its moments over (dx, dy) give the centre's and

@@ -159,6 +159,10 @@ __device__ __forceinline__ bool reachesBox(float4 screen, float4 conic, float x0
     return !(least > limit);
 }
 
+// Colours and gradients below this have finite products, so that a factor of 0 takes a
+// pixel's term out of a sum; past it the walks choose the pixels one by one.
+constexpr float kWalkLimit = 1e18f;
+
 // ---- a record as a warp's walk holds it ------------------------------------------
 // Values the packed arithmetic takes are stored once a pixel of the lane, so that a
 // broadcast load gives the pair.
@@ -170,7 +174,7 @@ struct alignas(16) WalkRecord {
     float r[kPx], g[kPx];
     float bl[kPx], z[kPx];
     float cutoff;
-    uint32_t odd;                  // 1: an opacity over 1 or a colour that is not finite
+    uint32_t odd;                  // 1: an opacity over 1, or a colour that is not finite or past kWalkLimit
     uint32_t slot, place;          // the record's slot; its place in the tile's list
 
     __device__ __forceinline__ void set(float4 screen, float4 conic, float4 colour, uint32_t atSlot, uint32_t atPlace) {
@@ -183,7 +187,7 @@ struct alignas(16) WalkRecord {
         }
         cutoff = screen.w;
         const float sum = ((fabsf(colour.x) + fabsf(colour.y)) + fabsf(colour.z)) + fabsf(screen.z);
-        odd = opacity <= 1.0f && sum < 3.0e38f ? 0u : 1u;
+        odd = opacity <= 1.0f && sum < kWalkLimit ? 0u : 1u;
         slot = atSlot;
         place = atPlace;
     }

@@ -223,3 +223,64 @@ def test_autograd_function_matches_the_fused_loss(raster):
     for leaf, ours in zip(leaves, (grads.means, grads.scales, grads.quats, grads.sh)):
         a, b = leaf.grad.cpu().numpy(), ours.cpu().numpy()
         assert np.abs(a - b).max() <= 1e-4 * (np.abs(b).max() + 1e-12)
+
+
+def _records_and_gradients(raster, proj, P, W, H, dl, dz):
+    """dL/d(record) a slot and dL/dparameters a Gaussian of one frame."""
+    import ctypes as C
+
+    from athenea_b200 import _native as N
+    from tests import gpu_helpers as G
+    t = A.RenderTargets.make(W, H)
+    raster.render_params(proj, P, A.RenderSettings(width=W, height=H), t)
+    grads = P.zeros_like()
+    raster.backward(dl(t), grads, None if dz is None else dz(t))
+    torch.cuda.synchronize()
+    b = N.FrameBuffers()
+    N.check(N.lib().ath_raster_frame_buffers(raster._h, C.byref(b)))
+    rows = np.concatenate([getattr(grads, n).cpu().numpy().reshape(P.count, -1) for n in ("means", "scales", "quats", "sh")], 1)
+    return G.fetch(b.grads, (b.slots, 10), np.float32), rows, t
+
+
+# boxes of one pixel a lane and of two (from 2368 tiles on 148 SMs)
+@pytest.mark.parametrize("size", [(320, 200), (1184, 528)])
+@pytest.mark.parametrize("depth", [False, True])
+def test_a_gradient_that_is_not_finite_stays_with_its_pixels_gaussians(raster, size, depth):
+    """An infinite dL/dalpha where nothing is drawn (a division by the coverage gives it) reaches nothing; a NaN or an
+    infinity at one pixel reaches the Gaussians that the pixel blends."""
+    W, H = size
+    P = _params_gpu(scenes.params(20_000, True, 31, 3))
+    proj = _frame(W, H)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    clean = torch.rand((W * H, 4), generator=gen, device="cuda")
+    cleanz = torch.rand(W * H, generator=gen, device="cuda")
+    covered = _records_and_gradients(raster, proj, P, W, H, lambda t: clean, None)[2].colour[:, 3]
+    thin = torch.nonzero((covered > 0.05) & (covered < 0.6))[:, 0]   # a few Gaussians each
+    bad = thin[:: max(1, thin.numel() // 7)][:7]
+    assert bad.numel() == 7 and int((covered == 0).sum()) > 1000
+    clean[bad], cleanz[bad] = 0.0, 0.0
+    base, want, _ = _records_and_gradients(raster, proj, P, W, H, lambda t: clean, (lambda t: cleanz) if depth else None)
+    one = torch.zeros_like(clean)
+    one[bad] = 1.0
+    blends = np.any(_records_and_gradients(raster, proj, P, W, H, lambda t: one, None)[0][:, 6:9] != 0, axis=1)
+    assert 0 < blends.sum() < 0.5 * (base != 0).any(1).sum()
+
+    def poisoned(t):
+        dl = clean.clone()
+        dl[t.colour[:, 3] == 0] = float("inf")
+        dl[bad[0]], dl[bad[1], 3], dl[bad[2], 1] = float("nan"), float("inf"), -float("inf")
+        if not depth:
+            dl[bad[3:]] = 3e38
+        return dl
+
+    def poisonedz(t):
+        dz = cleanz.clone()
+        dz[t.colour[:, 3] == 0] = float("nan")
+        dz[bad[3:]] = float("nan")
+        return dz
+
+    got, rows, _ = _records_and_gradients(raster, proj, P, W, H, poisoned, poisonedz if depth else None)
+    assert not np.isfinite(got[blends]).all(axis=1).all()
+    for a, b in ((got[~blends], base[~blends]), (rows[~blends], want[~blends])):
+        assert np.isfinite(a).all()
+        np.testing.assert_allclose(a, b, rtol=1e-3, atol=1e-5 * np.abs(b).max())   # the order of the atomic sums
