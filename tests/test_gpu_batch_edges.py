@@ -195,3 +195,34 @@ def test_a_batch_growth_that_fails_part_way_leaves_a_trainer_that_steps(part_of_
             np.testing.assert_array_equal(image.cpu().numpy(), want.cpu().numpy())
     finally:
         A.set_memory_budget(0)
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+def test_a_target_that_is_not_finite_stays_with_its_pixels_gaussians(tile):
+    """A target without values where nothing is drawn reaches no Gaussian, one at a drawn pixel the Gaussians that the
+    pixel blends."""
+    _, M = _scene(20_000, 28)
+    views = _views(2)
+    pixels = [W * H for _, W, H in views]
+    gen = torch.Generator().manual_seed(28)
+    clean = [torch.rand((n, 3), generator=gen).cuda() for n in pixels]
+    _, colour, *_ = _batched(M, views, clean, tile)
+    alpha = colour[:pixels[0], 3]
+    thin = torch.nonzero((alpha > 0.05) & (alpha < 0.6))[:, 0]   # a few Gaussians each
+    bad = thin[:: max(1, thin.numel() // 5)][:5]
+    assert bad.numel() == 5 and int((colour[:, 3] == 0).sum()) > 500
+    rows = lambda g: torch.cat([getattr(g, n).reshape(M.count, -1) for n in ("means", "scales", "quats", "sh")], 1)  # noqa: E731
+    own = [c.clone() for c in colour[:, :3].split(pixels)]
+    own[0][bad] += 0.25
+    blends = (rows(_batched(M, views, own, tile)[3]) != 0).any(1)
+    clean[0][bad] = colour[bad, :3]   # these pixels give no gradient
+    want = rows(_batched(M, views, clean, tile)[3])
+    assert 0 < int(blends.sum()) < 0.5 * int((want != 0).any(1).sum())
+    poisoned = [c.clone() for c in clean]
+    for p, c in zip(poisoned, colour.split(pixels)):
+        p[c[:, 3] == 0] = float("nan")
+    poisoned[0][bad[0]], poisoned[0][bad[1], 1], poisoned[0][bad[2:]] = float("nan"), float("inf"), 3e38
+    got = rows(_batched(M, views, poisoned, tile)[3])
+    assert not bool(torch.isfinite(got[blends]).all())
+    assert bool(torch.isfinite(got[~blends]).all())
+    torch.testing.assert_close(got[~blends], want[~blends], rtol=1e-3, atol=1e-5 * float(want.abs().max()))
