@@ -50,7 +50,7 @@ __device__ __forceinline__ float reciprocal(float x) {
 // through shared memory by atomics: 0.28 ms for 500k Gaussians at 1280x720 (0.71), 75 us
 // for 20k at 333x251 (201).
 template <int kPx, bool kDepth>
-__global__ void __launch_bounds__(Box<kPx>::kThreads)
+__global__ void __launch_bounds__(Box<kPx>::kThreads)   // what shared memory and no spill allow
     blendBackwardKernel(const FrameConst F, uint32_t pairs, uint32_t slots, const uint2* __restrict__ ranges,
                         const uint64_t* __restrict__ sorted, const float4* __restrict__ recs,
                         const TrainingState training, const float4* __restrict__ dLdColour,
@@ -112,7 +112,6 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
         most = max(most, last[p]);
     }
     const uint32_t sumRecord = lane / kValues, sumValue = lane % kValues;   // the column this lane sums
-    const float rowMid = (float)boxY + 0.5f * (float)Box<kPx>::kHeight;      // the box's middle row
     wild = __any_sync(0xFFFFFFFFu, wild);
     const int32_t chunks = (int32_t)((__reduce_max_sync(0xFFFFFFFFu, most) + 31u) >> 5);
     const uint32_t* liveOf = training.live + ((size_t)(range.x >> 5) + tile) * Box<kPx>::kCount + warp;
@@ -208,11 +207,10 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                 // the conic's gradients, the centre's x and y both in the lane of the moment dx
                 const bool mine = lane < batch * kValues;
                 RowSums v{0.0f, 0.0f, 0.0f};
-                if (mine) v = rowSums<(int)Box<kPx>::kHeight>(sh.sums + lane * kColumnStride);
                 const WalkRecord<kPx>& R = sh.records[q0 + min(sumRecord, batch - 1u)];
-                const float dy = rowMid + R.ny[0];
-                const float overRows = __fmaf_rn(dy, v.sum, v.first);   // dy, or dx dy
-                const float my = __shfl_up_sync(0xFFFFFFFFu, overRows, 1);
+                if (mine)
+                    v = rowSums<(int)Box<kPx>::kHeight>(sh.sums + lane * kColumnStride, (float)boxY + 0.5f, R.ny[0]);
+                const float my = __shfl_up_sync(0xFFFFFFFFu, v.first, 1);   // of the moment dx: sum dy
                 if (mine) {
                     float* words = grads + (size_t)R.slot * kGradWords;
                     auto add = [&](uint32_t word, float value) {
@@ -220,11 +218,11 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)
                     };
                     if (sumValue == 0) {
                         add(kGradAlpha, v.sum / R.alpha[0]);
-                        add(kGradC, -0.5f * __fmaf_rn(dy, __fmaf_rn(dy, v.sum, 2.0f * v.first), v.second));
+                        add(kGradC, -0.5f * v.second);
                     } else if (sumValue == 1) {
                         add(kGradCx, __fmaf_rn(R.a[0], v.sum, 0.5f * R.b2[0] * my));
                         add(kGradCy, __fmaf_rn(0.5f * R.b2[0], v.sum, R.c[0] * my));
-                        add(kGradB2, -overRows);
+                        add(kGradB2, -v.first);
                     } else {
                         add(sumValue == 2 ? (uint32_t)kGradA : (uint32_t)kGradR + sumValue - 3u,
                             sumValue == 2 ? -0.5f * v.sum : v.sum);

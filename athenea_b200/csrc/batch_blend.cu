@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
         __syncthreads();   // the block's warps are done with the staged records, whose memory the adjoint takes
         Adjoint& sA = reinterpret_cast<Adjoint*>(sRaw)[warp];
         const Px<2> xc{{pxc[0], pxc[1]}}, yc = both<2>(pyc);
-        const float rowMid = tileY0 + (float)((warp / kAcross) * kBox) + 0.5f * (float)kBox;   // the box's middle row
+        const float boxRow = tileY0 + (float)((warp / kAcross) * kBox) + 0.5f;   // the box's first row
         Px<2> light{{Tr[0], Tr[1]}};   // the pixels' transmittance, from the last record back
         const uint32_t warpLast = __reduce_max_sync(0xFFFFFFFFu, max(last[0], last[1]));
         const uint32_t nChunks = (warpLast + 31u) >> 5;
@@ -438,8 +438,7 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                     // (all its pixels clamped) are not added.
                     if (lane < batch * kSumValues) {
                         const Gathered& G = sA.records[q0 + sumRecord];
-                        const RowSums v = rowSums<8>(sA.sums + lane * kColumnStride);
-                        const float dy = rowMid + G.ny[0];   // of the box's middle row
+                        const RowSums v = rowSums<8>(sA.sums + lane * kColumnStride, boxRow, G.ny[0]);
                         float* words = grads + (size_t)sA.rec[q0 + sumRecord] * kGradWords;
                         // an opacity over 1 takes no geometry or opacity gradient (its kernel has no moments)
                         const bool some = v.sum != 0.0f || v.first != 0.0f || v.second != 0.0f;
@@ -447,9 +446,8 @@ __global__ void __launch_bounds__(S * S / 2, S == 32 ? 2 : S == 16 ? (kTrain ? 8
                             // words: moments t, dy, t t, t dy, dy dy; the opacity's; the colour's
                             atomicAdd(words + (sumValue == 0 ? 5u : sumValue == 1 ? 0u : sumValue == 2 ? 2u : 3u + sumValue),
                                       v.sum);
-                            if (sumValue < 2) atomicAdd(words + (sumValue == 0 ? 1u : 3u), __fmaf_rn(dy, v.sum, v.first));
-                            if (sumValue == 0)
-                                atomicAdd(words + 4, __fmaf_rn(dy, __fmaf_rn(dy, v.sum, 2.0f * v.first), v.second));
+                            if (sumValue < 2) atomicAdd(words + (sumValue == 0 ? 1u : 3u), v.first);
+                            if (sumValue == 0) atomicAdd(words + 4, v.second);
                         }
                     }
                     __syncwarp();   // the next records' values overwrite the columns
