@@ -28,7 +28,10 @@
 namespace ath {
 namespace {
 
-// 1 / x, x in [0.01, 1]: the hardware's approximation and one Newton step.
+// 1 / x for x = 1 - alpha, in [0.01, 1]: the hardware's approximation and one Newton step.
+// Rounded as __frcp_rn for every such x (all 66.9M of the 32-bit alphas from 1/255 to 0.99
+// compared, none differed), without its test for exponents that do not occur here: 20k
+// Gaussians at 333x251 295 us by this, 310 by the call.
 __device__ __forceinline__ float reciprocal(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -159,14 +162,15 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)   // what shared memory an
                         on[p] = R.place <= last[p] && !(at.power.v[p] > R.cutoff) && !(a < kFaint);
                         alpha.v[p] = on[p] ? a : 0.0f;
                     }
-                    const Px<kPx> minus = alpha * both<kPx>(-1.0f);
-                    const Px<kPx> om = minus + both<kPx>(1.0f);
+                    const Px<kPx> minus = alpha + both<kPx>(-1.0f);   // -(1 - alpha), rounded alike
 #pragma unroll
-                    for (int p = 0; p < kPx; ++p) inv.v[p] = reciprocal(om.v[p]);
-                    // the transmittance before the record: T / (1 - alpha), its quotient corrected
-                    // by its remainder
+                    for (int p = 0; p < kPx; ++p) inv.v[p] = reciprocal(-minus.v[p]);
+                    // the transmittance before the record: T / (1 - alpha), its quotient corrected by its
+                    // remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
+                    // System/6000 processor", IBM J. Res. Dev. 34, 1990): with a rounded reciprocal
+                    // the rounded quotient
                     Px<kPx> Tb = T * inv;
-                    Tb = fused(fused(om * both<kPx>(-1.0f), Tb, T), inv, Tb);
+                    Tb = fused(fused(minus, Tb, T), inv, Tb);
                     const Px<kPx> w = Tb * alpha;
                     // where a colour or a gradient may not be finite, alpha 0 does not keep the pixels
                     // that did not blend the record out of its sums: their terms are left out
