@@ -51,6 +51,7 @@ struct SortPlan {
     uint32_t passes;
     uint32_t width[kMaxPasses];
     uint32_t shift[kMaxPasses];   // from firstBit
+    uint32_t mask[kMaxPasses];    // a digit's bits that take part
 };
 
 template <typename K>
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (uint32_t p = 0; p < kMaxPasses; ++p) {
             if (p >= plan.passes) break;
-            const uint32_t shift = firstBit + plan.shift[p], mask = (1u << plan.width[p]) - 1u;
+            const uint32_t shift = firstBit + plan.shift[p], mask = plan.mask[p];
             uint32_t run = (uint32_t)(key[0] >> shift) & mask, length = 1;
 #pragma unroll
             for (uint32_t k = 1; k < kRun; ++k) {
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(kSortThreads)
         if constexpr (kValues == kIndexValues) val[k] = i;
     }
     for (uint32_t p = 0; p < plan.passes; ++p) {
-        const uint32_t radix = 1u << plan.width[p], digitMask = radix - 1u, shift = firstBit + plan.shift[p];
+        const uint32_t radix = 1u << plan.width[p], digitMask = plan.mask[p], shift = firstBit + plan.shift[p];
         for (uint32_t j = tid; j < kWarps * radix / 4; j += kSortThreads) {
             reinterpret_cast<uint4*>(sWarpCnt)[j] = make_uint4(0, 0, 0, 0);
             reinterpret_cast<uint4*>(sMasks)[j] = make_uint4(0, 0, 0, 0);
@@ -466,6 +467,8 @@ SortPlan planSort(uint32_t bits) {
     for (uint32_t k = 0; k < p.passes && k < kMaxPasses; ++k) {
         p.width[k] = k < wide ? 9u : 8u;
         p.shift[k] = at;
+        // the last digit's bits past the sort's take no part
+        p.mask[k] = (1u << (bits - at < p.width[k] ? bits - at : p.width[k])) - 1u;
         at += p.width[k];
     }
     return p;
@@ -557,7 +560,7 @@ cudaError_t runSort(uint32_t n, const uint32_t* nDevice, const uint32_t* epochDe
     histogramKernel<K><<<min((n + 255) / 256, (uint32_t)sms * 4), 256, 0, stream>>>(in, n, nDevice, firstBit, plan, hist);
     for (uint32_t p = 0; p < plan.passes; ++p) {
         pass(p, plan, keys, tiles, firstBit + plan.shift[p], hist + p * kMaxRadix, flags, tickets + p,
-             (1u << plan.width[p]) - 1u);
+             plan.mask[p]);
         flags += (size_t)tiles << plan.width[p];
     }
     return cudaGetLastError();

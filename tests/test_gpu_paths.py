@@ -60,7 +60,7 @@ def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(native, raster)
 
 # one block up to 8192; 2048-key tiles up to 606,208; then tiles of 6144 (pairs)
 @pytest.mark.parametrize("count", [2, 511, 513, 8191, 8192, 8193, 10_240, 606_208, 606_209, 700_001])
-@pytest.mark.parametrize("bits", [1, 9, 24, 45, 64])
+@pytest.mark.parametrize("bits", [1, 9, 12, 24, 37, 38, 45, 64])
 def test_sorts_are_stable_at_every_tile_size(native, count, bits):
     gen = torch.Generator(device="cuda").manual_seed(count + bits)
     keys = (torch.randint(0, 1 << 32, (count,), generator=gen, device="cuda") << 32) | \
@@ -74,7 +74,7 @@ def test_sorts_are_stable_at_every_tile_size(native, count, bits):
                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)))
     N.check(N.lib().ath_sorter_check(sorter.handle))
     host = keys.cpu().numpy().view(np.uint64)
-    order = np.argsort(host & np.uint64((1 << max(bits, 8)) - 1), kind="stable")   # a pass takes a whole digit
+    order = np.argsort(host & np.uint64((1 << bits) - 1), kind="stable")   # the low bits alone
     np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), order.astype(np.uint32))
     np.testing.assert_array_equal(k.cpu().numpy().view(np.uint64), host[order])
 
