@@ -14,6 +14,7 @@
 // with --fmad=false), so it skips the same records, and divides the
 // transmittance back out record by record.
 #include <algorithm>
+#include <utility>
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -371,16 +372,24 @@ __global__ void __launch_bounds__(128)
 
 // L = mean over pixels and r g b of (colour - target)^2: its value (added into
 // *loss) and dL/dcolour (float4 a pixel, alpha 0). The threads' shares are summed in 64
-// bits over a cluster of blocks, one 32-bit addition into *loss a cluster: one a block of
-// 256 pixels, thousands an image, each rounded *loss, up to 2e-6 of it in all.
+// bits over a cluster of blocks, one 32-bit addition into *loss a cluster, 148 at most: one
+// a block of 256 pixels, thousands an image, each rounded *loss, 3e-6 of it in all at
+// 1920x1080 (so 3e-7), though without clusters the blocks drift apart less where the target
+// comes from memory. The grid fills every SM once, which takes 32 registers a thread, and
+// a block writes its sum into the first block's shared memory, a barrier's first half at the
+// start standing for that block's being there. 333x251: 2.6 us a block at a time, 3.3 so
+// (4.0 by 40 registers and two barriers at the end); 1280x720 8.5, 9.8 (11.3), 7.9, 7.0 (9.1)
+// where the target is in the L2; 1920x1080 16.0, 17.1 (18.7); 3840x2160 58, 72 (70).
 constexpr uint32_t kLossThreads = 256, kLossCluster = 8, kLossBlocks = 148 * kLossCluster;
 
-__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads)
+__global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThreads, 2048 / kLossThreads)
     l2LossKernel(const float4* __restrict__ colour, const float* __restrict__ target, uint32_t pixels, float scale,
                  float4* __restrict__ dLdColour, float* __restrict__ loss) {
-    __shared__ double sPart[kLossThreads / 32], sBlock;
+    __shared__ double sPart[kLossThreads / 32], sBlocks[kLossCluster];
+    const auto cluster = cooperative_groups::this_cluster();
+    auto started = cluster.barrier_arrive();
     float share = 0.0f;
-#pragma unroll 4
+#pragma unroll 1
     for (uint64_t p = blockIdx.x * kLossThreads + threadIdx.x; p < pixels; p += (uint64_t)gridDim.x * kLossThreads) {
         const float4 c = colour[p];
         const float er = c.x - target[p * 3 + 0], eg = c.y - target[p * 3 + 1], eb = c.z - target[p * 3 + 2];
@@ -396,16 +405,16 @@ __global__ void __cluster_dims__(kLossCluster, 1, 1) __launch_bounds__(kLossThre
         sum = 0.0;
 #pragma unroll
         for (uint32_t w = 0; w < kLossThreads / 32; ++w) sum += sPart[w];
-        sBlock = sum;
     }
-    const auto cluster = cooperative_groups::this_cluster();
+    cluster.barrier_wait(std::move(started));   // every block runs: its shared memory is there
+    if (threadIdx.x == 0) *cluster.map_shared_rank(sBlocks + cluster.block_rank(), 0) = sum;
     cluster.sync();
     if (threadIdx.x == 0 && cluster.block_rank() == 0) {
         sum = 0.0;
-        for (uint32_t b = 0; b < kLossCluster; ++b) sum += *cluster.map_shared_rank(&sBlock, b);
+#pragma unroll
+        for (uint32_t b = 0; b < kLossCluster; ++b) sum += sBlocks[b];
         if (sum != 0.0) atomicAdd(loss, (float)sum);
     }
-    cluster.sync();   // the others' shared memory is read until here
 }
 
 }   // namespace

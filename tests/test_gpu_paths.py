@@ -153,3 +153,19 @@ def test_gradients_do_not_depend_on_the_rows_layout(native, stride, shift):
     for name in ("means", "scales", "quats"):
         a, b = getattr(grads, name), getattr(want, name)
         assert torch.allclose(a, b, rtol=1e-3, atol=1e-5 * float(b.abs().max())), name
+
+
+# less than a block, a block and a cluster of blocks with remainders, and past one pixel a thread of the whole grid
+@pytest.mark.parametrize("pixels", [1, 255, 257, 2048, 2049, 303_104, 303_105, 921_600])
+def test_the_l2_loss_at_every_size(native, pixels):
+    """148 additions of 32 bits at most into the loss: 3e-7 of it where they round at random, 1e-6 allowed."""
+    gen = torch.Generator(device="cuda").manual_seed(pixels)
+    colour = torch.rand((pixels, 4), generator=gen, device="cuda")
+    target = torch.rand((pixels, 3), generator=gen, device="cuda")
+    dl, loss = torch.full_like(colour, 7.0), torch.full((1,), 0.5, device="cuda")
+    A.l2_loss(colour, target, dl, loss)
+    error = colour[:, :3].double() - target.double()
+    want = 0.5 + float(error.square().mean())
+    assert abs(loss.item() - want) <= 1e-6 * want
+    assert float((dl[:, :3].double() - 2.0 * error / (3.0 * pixels)).abs().max()) <= 1e-6 / (3.0 * pixels)
+    assert not bool(dl[:, 3].any())
