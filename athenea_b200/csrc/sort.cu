@@ -154,9 +154,11 @@ constexpr size_t onesweepSmem() {
 // The values take the keys' shared memory once the keys are out, each thread keeping its
 // items' places in the tile and its outputs' destinations in registers: with values as
 // without, two blocks an SM (values beside the keys, 128 KB, left one). 8M pairs of
-// 40 bits: 605 -> 549 us with the masks below.
+// 40 bits: 605 -> 549 us with the masks below. 64-bit keys with values in 8192-key tiles, the
+// static sort's, are at most 128 tiles for more SMs: one block an SM, and no spill (1M pairs
+// of 40 bits 136 -> 119 us, 20k 108 -> 92).
 template <typename K, uint32_t kValues, uint32_t kBits, uint32_t kPerThread>
-__global__ void __launch_bounds__(kSortThreads, 2)
+__global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNoValues && kPerThread == kItems ? 1 : 2)
     onesweepKernel(const K* __restrict__ keysIn, const uint32_t* __restrict__ valsIn, K* __restrict__ keysOut,
                    uint32_t* __restrict__ valsOut, uint32_t n, uint32_t shift, uint32_t digitMask,
                    const uint32_t* __restrict__ globalHist, uint64_t* __restrict__ flags, uint32_t* __restrict__ ticket,
