@@ -26,9 +26,15 @@ struct ath_raster {
     int sms = 148;
     bool tight = false;   // after release_scratch: grow to the need exactly
     uint32_t slotCapacity = 0, pairCapacity = 0, tileCapacity = 0, instanceCapacity = 0;
-    DeviceBuffer recs, spans, keys, instances;
-    DeviceBuffer depthKeys[2], depthSlots[2];   // the depth sort's
-    DeviceBuffer pairs[2], sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
+    // A slot's arrays, one after another in one allocation (a handle's first frame is mostly
+    // allocations), each null until it holds slotCapacity slots.
+    struct SlotArrays {
+        float4* recs = nullptr;
+        uint4* spans = nullptr;
+        uint32_t *keys = nullptr, *depthKeys[2] = {}, *depthSlots[2] = {};   // the last four the depth sort's
+    } slot;
+    uint64_t* pairs[2] = {};   // halves of pairMemory, pairCapacity pairs each
+    DeviceBuffer slotMemory, pairMemory, instances, sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
     // ath_raster_frame_buffers' own: slots, a pair each (its keys: the spare pair buffer); rects and first pairs, a slot each
     DeviceBuffer inspectSplats, inspectRects, inspectOffsets;
     DeviceBuffer zeroed;         // what a frame starts at zero, cleared at once (FrameZeroed): its words first
@@ -312,7 +318,6 @@ extern "C" ath_status ath_raster_create(ath_raster** out) {
     cudaError_t err = cudaGetDevice(&r->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, r->device);
     if (err == cudaSuccess) err = sortPrepare(kSortsKeys | kSortsDepths);
-    if (err == cudaSuccess) err = r->zeroed.reserve(kFrameWords * sizeof(uint32_t));
     if (err == cudaSuccess) err = r->wordsHost.reserve(kFrameWords * sizeof(uint32_t));
     if (err == cudaSuccess) err = r->statusHost.reserve(kFrameWords * sizeof(uint32_t));
     for (int k = 0; k < ath_raster::kCountDepth && err == cudaSuccess; ++k) {
@@ -320,7 +325,6 @@ extern "C" ath_status ath_raster_create(ath_raster** out) {
         if (err == cudaSuccess) err = cudaEventCreateWithFlags(&r->countDone[k], cudaEventDisableTiming);
     }
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&r->frameDone, cudaEventDisableTiming);
-    if (err == cudaSuccess) err = cudaMemset(r->zeroed.ptr, 0, kFrameWords * sizeof(uint32_t));
     for (int k = 0; k < 8 && err == cudaSuccess; ++k) err = cudaEventCreate(&r->marks[k]);
     if (err != cudaSuccess) {
         ath_status s = failCuda(err, "ath_raster_create");
@@ -351,9 +355,10 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     cudaDeviceSynchronize();
     r->tight = true;
     r->slotCapacity = r->pairCapacity = r->tileCapacity = r->instanceCapacity = 0;
-    for (DeviceBuffer* b : {&r->recs, &r->spans, &r->keys, &r->instances, &r->inspectRects, &r->inspectOffsets,
-                            &r->depthKeys[0], &r->depthKeys[1], &r->depthSlots[0], &r->depthSlots[1], &r->pairs[0],
-                            &r->pairs[1], &r->inspectSplats, &r->sortScratch, &r->zeroed, &r->finalT, &r->lastContrib, &r->live, &r->grads})
+    r->slot = {};
+    r->pairs[0] = r->pairs[1] = nullptr;
+    for (DeviceBuffer* b : {&r->slotMemory, &r->pairMemory, &r->instances, &r->inspectRects, &r->inspectOffsets,
+                            &r->inspectSplats, &r->sortScratch, &r->zeroed, &r->finalT, &r->lastContrib, &r->live, &r->grads})
         b->release();
     r->trainingValid = false;
     r->frameRecorded = false;
@@ -417,15 +422,22 @@ namespace {
 ath_status reserveSlots(ath_raster* r, uint32_t slots) {   // reserveSplats (TileRasterizer.cpp:193-226)
     if (slots <= r->slotCapacity) return ATH_OK;
     const uint32_t n = r->tight ? slots : grow(r->slotCapacity, slots);
-    r->slotCapacity = 0;   // no slots until every array has them: an array that grows gives up its old memory first
-    cudaError_t err = r->recs.reserve((size_t)n * 48);
-    if (err == cudaSuccess) err = r->spans.reserve((size_t)n * 16);
-    if (err == cudaSuccess) err = r->keys.reserve((size_t)n * 4);
-    for (int k = 0; k < 2; ++k) {
-        if (err == cudaSuccess) err = r->depthKeys[k].reserve((size_t)n * 4);
-        if (err == cudaSuccess) err = r->depthSlots[k].reserve((size_t)n * 4);
-    }
-    if (err != cudaSuccess) return failCuda(err, "reserving the splats' scratch");
+    r->slotCapacity = 0;   // no slots until there is memory for them: growing gives up the old memory first
+    r->slot = {};
+    size_t bytes = 0;
+    auto place = [&](size_t each) {
+        const size_t at = bytes;
+        bytes = (bytes + each * n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t recs = place(48), spans = place(16), keys = place(4);
+    const size_t depth[4] = {place(4), place(4), place(4), place(4)};
+    if (const cudaError_t err = r->slotMemory.reserve(bytes); err != cudaSuccess)
+        return failCuda(err, "reserving the splats' scratch");
+    char* const base = static_cast<char*>(r->slotMemory.ptr);
+    auto words = [&](size_t at) { return reinterpret_cast<uint32_t*>(base + at); };
+    r->slot = {reinterpret_cast<float4*>(base + recs), reinterpret_cast<uint4*>(base + spans), words(keys),
+               {words(depth[0]), words(depth[1])}, {words(depth[2]), words(depth[3])}};
     r->slotCapacity = n;
     return ATH_OK;
 }
@@ -436,11 +448,14 @@ ath_status reservePairs(ath_raster* r, uint32_t pairs, uint32_t bits) {   // res
     if (pairs > r->pairCapacity) {
         const uint32_t n = r->tight ? pairs : grow(r->pairCapacity, pairs);
         r->pairCapacity = 0;   // as the slots
-        cudaError_t err = cudaSuccess;
-        for (int k = 0; k < 2 && err == cudaSuccess; ++k) err = r->pairs[k].reserve((size_t)n * 8);
-        if (err != cudaSuccess) return failCuda(err, "reserving the pairs");
+        r->pairs[0] = r->pairs[1] = nullptr;
+        const size_t half = ((size_t)n * 8 + 255) / 256 * 256;
+        if (const cudaError_t err = r->pairMemory.reserve(2 * half); err != cudaSuccess)
+            return failCuda(err, "reserving the pairs");
+        for (int k = 0; k < 2; ++k) r->pairs[k] = reinterpret_cast<uint64_t*>(static_cast<char*>(r->pairMemory.ptr) + k * half);
         r->pairCapacity = n;
     }
+    if (r->pairCapacity <= kSortTileKeys) return ATH_OK;   // a sort in one block needs none
     const size_t bytes = kSortHistBytes + sortFlagWords(r->pairCapacity, bits) * 8;
     if (cudaError_t err = r->sortScratch.reserve(bytes); err != cudaSuccess)
         return failCuda(err, "reserving the sort's scratch");
@@ -574,8 +589,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
                               stream);
     if (err == cudaSuccess)
         err = launchProject(F, staged[0], static_cast<const InstanceConst*>(r->instances.ptr), instanceCount, slots, layout,
-                            s.count_splats != 0, static_cast<float4*>(r->recs.ptr), static_cast<uint4*>(r->spans.ptr),
-                            static_cast<uint32_t*>(r->keys.ptr), words, stream);
+                            s.count_splats != 0, r->slot.recs, r->slot.spans, r->slot.keys, words, stream);
     mark(1);
     bool haveTotals = false;
     if (sizing && err == cudaSuccess) {
@@ -597,20 +611,17 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     // --- depth sort, emit, tile sort, ranges (the pair count on the device) --
     const uint32_t capacity = r->pairCapacity;
     uint32_t* kept = words + kWordPairsKept;
-    uint32_t* keys = static_cast<uint32_t*>(r->keys.ptr);
-    uint32_t* hist = static_cast<uint32_t*>(r->sortScratch.ptr);
-    uint64_t* flags = reinterpret_cast<uint64_t*>(static_cast<char*>(r->sortScratch.ptr) + kSortHistBytes);
-    uint32_t* depthKeys[2] = {static_cast<uint32_t*>(r->depthKeys[0].ptr), static_cast<uint32_t*>(r->depthKeys[1].ptr)};
-    uint32_t* depthSlots[2] = {static_cast<uint32_t*>(r->depthSlots[0].ptr),
-                               static_cast<uint32_t*>(r->depthSlots[1].ptr)};
-    uint64_t* pairs[2] = {static_cast<uint64_t*>(r->pairs[0].ptr), static_cast<uint64_t*>(r->pairs[1].ptr)};
-    err = launchSortDepths(keys, depthKeys, depthSlots, slots, reinterpret_cast<uint32_t*>(zero + zeroed.depthHist),
+    uint32_t* hist = static_cast<uint32_t*>(r->sortScratch.ptr);   // null, and not used, for a sort in one block
+    uint64_t* flags = hist ? reinterpret_cast<uint64_t*>(static_cast<char*>(r->sortScratch.ptr) + kSortHistBytes) : nullptr;
+    uint64_t** pairs = r->pairs;
+    err = launchSortDepths(r->slot.keys, r->slot.depthKeys, r->slot.depthSlots, slots,
+                           reinterpret_cast<uint32_t*>(zero + zeroed.depthHist),
                            reinterpret_cast<uint64_t*>(zero + zeroed.depthFlags), words + kWordDepthTickets,
                            words + kWordSticky, stream);
     mark(3);
     if (err == cudaSuccess)
-        err = launchEmit(F, slots, depthSlots[0], static_cast<const float4*>(r->recs.ptr),
-                         static_cast<const uint4*>(r->spans.ptr), reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
+        err = launchEmit(F, slots, r->slot.depthSlots[0], r->slot.recs, r->slot.spans,
+                         reinterpret_cast<uint64_t*>(zero + zeroed.emitFlags), words, capacity, pairs[0], stream);
     mark(4);
     if (err == cudaSuccess && capacity > kSortTileKeys)   // a sort in one block needs none of it
         err = cudaMemsetAsync(hist, 0, kSortHistBytes + sortFlagWords(capacity, bits) * 8, stream);
@@ -633,9 +644,8 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     }
     if (err == cudaSuccess)
         err = launchBlend(F, capacity, slots, ranges, pairs[sorted],
-                          static_cast<const float4*>(r->recs.ptr), reinterpret_cast<float4*>(targets->colour),
-                          targets->depth, reinterpret_cast<float4*>(targets->position), training ? &keep : nullptr,
-                          r->sms, words + kWordSticky, stream, contrib,
+                          r->slot.recs, reinterpret_cast<float4*>(targets->colour), targets->depth,
+                          reinterpret_cast<float4*>(targets->position), training ? &keep : nullptr, r->sms, words + kWordSticky, stream, contrib,
                           under ? Under{under->colour, under->depth} : Under{}, matte);
     mark(6);
     // --- the frame's words: its counters into the ring; its status behind an event
@@ -690,8 +700,9 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
 }
 
 ath_status reserveInstances(ath_raster* r, uint32_t instanceCount) {
-    if (instanceCount > r->instanceCapacity || !r->instances.bytes) {
+    if (instanceCount > 1 && instanceCount > r->instanceCapacity) {   // a single one goes with its kernel
         const uint32_t n = std::max(instanceCount, 4u);
+        r->instanceCapacity = 0;
         cudaError_t err = r->instances.reserve((size_t)n * sizeof(InstanceConst));
         if (err != cudaSuccess) return failCuda(err, "reserving the instance table");
         r->instanceCapacity = n;
@@ -827,13 +838,12 @@ extern "C" ath_status ath_raster_backward(ath_raster* r, const float* dlDcolour,
     uint32_t* words = static_cast<uint32_t*>(r->zeroed.ptr);
     if (err == cudaSuccess)
         err = launchBlendBackward(F, r->pairCapacity, slots, r->ranges,
-                                  static_cast<const uint64_t*>(r->pairs[r->lastSorted].ptr),
-                                  static_cast<const float4*>(r->recs.ptr), trainingState(r),
+                                  r->pairs[r->lastSorted], r->slot.recs, trainingState(r),
                                   reinterpret_cast<const float4*>(dlDcolour), dlDdepth, r->trainingDepth,
                                   static_cast<float*>(r->grads.ptr), words + kWordSticky, stream);
     if (err == cudaSuccess)
-        err = launchProjectBackward(F, I, static_cast<const uint32_t*>(r->keys.ptr), static_cast<const float*>(r->grads.ptr),
-                                    static_cast<uint32_t*>(r->depthKeys[0].ptr),   // spare after the depth sort
+        err = launchProjectBackward(F, I, r->slot.keys, static_cast<const float*>(r->grads.ptr),
+                                    r->slot.depthKeys[0],   // spare after the depth sort
                                     reinterpret_cast<uint32_t*>(static_cast<char*>(r->grads.ptr) + gradBytes),
                                     reinterpret_cast<float4*>(grads->means), reinterpret_cast<float4*>(grads->scales),
                                     reinterpret_cast<float4*>(grads->quats), grads->sh, r->sms, stream);
@@ -883,10 +893,9 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     // the pairs with their depth keys, in the pair buffer the sort left spare
     const uint32_t pairs = static_cast<const uint32_t*>(r->statusHost.ptr)[kWordPairsKept];
     cudaError_t err = r->inspectSplats.reserve((size_t)std::max(pairs, 1u) * 4);
-    uint64_t* pairKeys = static_cast<uint64_t*>(r->pairs[r->lastSorted ^ 1u].ptr);
+    uint64_t* pairKeys = r->pairs[r->lastSorted ^ 1u];
     if (err == cudaSuccess)
-        err = launchInspectPairs(static_cast<const uint64_t*>(r->pairs[r->lastSorted].ptr), pairs,
-                                 static_cast<const uint32_t*>(r->keys.ptr), r->lastSlots, pairKeys,
+        err = launchInspectPairs(r->pairs[r->lastSorted], pairs, r->slot.keys, r->lastSlots, pairKeys,
                                  static_cast<uint32_t*>(r->inspectSplats.ptr), nullptr);
     // the slots' rects and first pairs, through look-back words of this call's own
     const size_t blocks = projectBlocks(std::max(r->lastSlots, 1u));
@@ -897,7 +906,7 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     if (err == cudaSuccess) err = cudaMemsetAsync(lookback.ptr, 0, blocks * 8 + 8, nullptr);
     uint32_t* const ticketAndStatus = reinterpret_cast<uint32_t*>(static_cast<uint64_t*>(lookback.ptr) + blocks);
     if (err == cudaSuccess)
-        err = launchInspectSlots(static_cast<const uint4*>(r->spans.ptr), r->lastSlots, static_cast<uint64_t*>(lookback.ptr),
+        err = launchInspectSlots(r->slot.spans, r->lastSlots, static_cast<uint64_t*>(lookback.ptr),
                                  ticketAndStatus, static_cast<uint2*>(r->inspectRects.ptr),
                                  static_cast<uint32_t*>(r->inspectOffsets.ptr), nullptr);
     uint32_t status[2] = {0, 0};
@@ -908,9 +917,9 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     out->slots = r->lastSlots;
     out->pairs = pairs;
     out->tiles = r->lastTiles;
-    out->records = static_cast<const float*>(r->recs.ptr);
+    out->records = reinterpret_cast<const float*>(r->slot.recs);
     out->rects = static_cast<const uint32_t*>(r->inspectRects.ptr);
-    out->keys = static_cast<const uint32_t*>(r->keys.ptr);
+    out->keys = r->slot.keys;
     out->offsets = static_cast<const uint32_t*>(r->inspectOffsets.ptr);
     out->pair_keys = pairKeys;
     out->pair_splats = static_cast<const uint32_t*>(r->inspectSplats.ptr);
