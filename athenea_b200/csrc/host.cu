@@ -35,8 +35,7 @@ struct ath_raster {
     } slot;
     uint64_t* pairs[2] = {};   // halves of pairMemory, pairCapacity pairs each
     DeviceBuffer slotMemory, pairMemory, instances, sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
-    // ath_raster_frame_buffers' own: slots, a pair each (its keys: the spare pair buffer); rects and first pairs, a slot each
-    DeviceBuffer inspectSplats, inspectRects, inspectOffsets;
+    DeviceBuffer inspect;        // ath_raster_frame_buffers' own: a slot a pair; the slots' rects and first pairs
     DeviceBuffer zeroed;         // what a frame starts at zero, cleared at once (FrameZeroed): its words first
     uint2* ranges = nullptr;     // the last frame's, there
     PinnedBuffer wordsHost;      // kFrameWords: a frame that waits (its handle's first, or timed) reads them here
@@ -357,8 +356,8 @@ extern "C" ath_status ath_raster_release_scratch(ath_raster* r) {
     r->slotCapacity = r->pairCapacity = r->tileCapacity = r->instanceCapacity = 0;
     r->slot = {};
     r->pairs[0] = r->pairs[1] = nullptr;
-    for (DeviceBuffer* b : {&r->slotMemory, &r->pairMemory, &r->instances, &r->inspectRects, &r->inspectOffsets,
-                            &r->inspectSplats, &r->sortScratch, &r->zeroed, &r->finalT, &r->lastContrib, &r->live, &r->grads})
+    for (DeviceBuffer* b : {&r->slotMemory, &r->pairMemory, &r->instances, &r->inspect, &r->sortScratch, &r->zeroed,
+                            &r->finalT, &r->lastContrib, &r->live, &r->grads})
         b->release();
     r->trainingValid = false;
     r->frameRecorded = false;
@@ -890,39 +889,41 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     // inspection: waits for the frame, whose pair count only the device knew
     if (const cudaError_t err = cudaEventSynchronize(r->frameDone); err != cudaSuccess)
         return failCuda(err, "waiting for the frame");
-    // the pairs with their depth keys, in the pair buffer the sort left spare
+    // one allocation for what the handle's frames can ask: a slot each of the pairs, the slots'
+    // rects and first pairs, and the look-back words of the latter's scan
     const uint32_t pairs = static_cast<const uint32_t*>(r->statusHost.ptr)[kWordPairsKept];
-    cudaError_t err = r->inspectSplats.reserve((size_t)std::max(pairs, 1u) * 4);
-    uint64_t* pairKeys = r->pairs[r->lastSorted ^ 1u];
-    if (err == cudaSuccess)
-        err = launchInspectPairs(r->pairs[r->lastSorted], pairs, r->slot.keys, r->lastSlots, pairKeys,
-                                 static_cast<uint32_t*>(r->inspectSplats.ptr), nullptr);
-    // the slots' rects and first pairs, through look-back words of this call's own
+    const size_t rectsAt = ((size_t)r->pairCapacity * 4 + 255) / 256 * 256, offsetsAt = rectsAt + (size_t)r->slotCapacity * 8;
+    const size_t scanAt = (offsetsAt + (size_t)r->slotCapacity * 4 + 255) / 256 * 256;
     const size_t blocks = projectBlocks(std::max(r->lastSlots, 1u));
-    DeviceBuffer lookback;
-    if (err == cudaSuccess) err = r->inspectRects.reserve((size_t)std::max(r->lastSlots, 1u) * 8);
-    if (err == cudaSuccess) err = r->inspectOffsets.reserve((size_t)std::max(r->lastSlots, 1u) * 4);
-    if (err == cudaSuccess) err = lookback.reserve(blocks * 8 + 8);
-    if (err == cudaSuccess) err = cudaMemsetAsync(lookback.ptr, 0, blocks * 8 + 8, nullptr);
-    uint32_t* const ticketAndStatus = reinterpret_cast<uint32_t*>(static_cast<uint64_t*>(lookback.ptr) + blocks);
+    cudaError_t err = r->inspect.reserve(scanAt + ((size_t)projectBlocks(r->slotCapacity) + 1) * 8);
+    char* const inspect = static_cast<char*>(r->inspect.ptr);
+    uint32_t* const pairSplats = reinterpret_cast<uint32_t*>(inspect);
+    uint2* const rects = reinterpret_cast<uint2*>(inspect + rectsAt);
+    uint32_t* const offsets = reinterpret_cast<uint32_t*>(inspect + offsetsAt);
+    uint64_t* const lookback = reinterpret_cast<uint64_t*>(inspect + scanAt);
+    uint32_t* const ticketAndStatus = reinterpret_cast<uint32_t*>(lookback + blocks);
+    uint64_t* const pairKeys = r->pairs[r->lastSorted ^ 1u];   // the pair buffer the sort left spare
+    // the frame is done: a stream that no other work waits for, or is waited for by
+    const cudaStream_t stream = cudaStreamPerThread;
+    if (err == cudaSuccess) err = cudaMemsetAsync(lookback, 0, blocks * 8 + 8, stream);
     if (err == cudaSuccess)
-        err = launchInspectSlots(r->slot.spans, r->lastSlots, static_cast<uint64_t*>(lookback.ptr),
-                                 ticketAndStatus, static_cast<uint2*>(r->inspectRects.ptr),
-                                 static_cast<uint32_t*>(r->inspectOffsets.ptr), nullptr);
+        err = launchInspectPairs(r->pairs[r->lastSorted], pairs, r->slot.keys, r->lastSlots, pairKeys, pairSplats, stream);
+    if (err == cudaSuccess)
+        err = launchInspectSlots(r->slot.spans, r->lastSlots, lookback, ticketAndStatus, rects, offsets, stream);
     uint32_t status[2] = {0, 0};
-    if (err == cudaSuccess) err = cudaMemcpyAsync(status, ticketAndStatus, sizeof(status), cudaMemcpyDeviceToHost, nullptr);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(status, ticketAndStatus, sizeof(status), cudaMemcpyDeviceToHost, stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) return failCuda(err, "reading the frame's pairs");
     if (status[1]) return fail(ATH_E_TIMEOUT, "a look-back wait gave up (bounded spin); the buffers were not read");
     out->slots = r->lastSlots;
     out->pairs = pairs;
     out->tiles = r->lastTiles;
     out->records = reinterpret_cast<const float*>(r->slot.recs);
-    out->rects = static_cast<const uint32_t*>(r->inspectRects.ptr);
+    out->rects = reinterpret_cast<const uint32_t*>(rects);
     out->keys = r->slot.keys;
-    out->offsets = static_cast<const uint32_t*>(r->inspectOffsets.ptr);
+    out->offsets = offsets;
     out->pair_keys = pairKeys;
-    out->pair_splats = static_cast<const uint32_t*>(r->inspectSplats.ptr);
+    out->pair_splats = pairSplats;
     out->ranges = reinterpret_cast<const uint32_t*>(r->ranges);
     out->grads = static_cast<const float*>(r->grads.ptr);
     return ATH_OK;
