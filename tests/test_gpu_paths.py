@@ -12,7 +12,8 @@ import athenea_b200 as A
 from athenea_b200 import _native as N
 from athenea_b200 import scenes
 from perf import cases
-from tests.fixtures import random_cloud
+from tests.fixtures import CloudBuilder, random_cloud
+from tests.gpu_helpers import frame_buffers, oracle_projection, upload
 from tests.test_gpu_parity import _compare, _decode, _settings
 
 pytestmark = pytest.mark.gpu
@@ -26,36 +27,67 @@ def raster(native):
 # On 148 SMs a frame takes boxes of one pixel a lane below 4736 tiles: (1184, 1008) is the last of them here,
 # (1184, 1024) is past it; (1279, 719) leaves part of a box in both directions; (16, 16) is one tile, (3, 5) less than a box
 @pytest.mark.parametrize("size", [(3, 5), (16, 16), (250, 190), (1279, 719), (1184, 1008), (1184, 1024)])
+@pytest.mark.parametrize("threshold", [0, 1])
 @pytest.mark.parametrize("opacity", [1.0, 6.0])
-def test_frames_equal_the_restatement_to_the_bit(oracle, native, raster, size, opacity):
+def test_frames_equal_the_restatement_to_the_bit(oracle, native, raster, size, opacity, threshold):
     """Footprints from a pixel to the whole image (rects of more than 64 tiles), with opacities over 1 (the harder
-    kernel) by an edit, over a background."""
+    kernel) by an edit, over a background, the depth layer in both modes."""
     W, H = size
     packed = _decode(oracle, random_cloud(900, 17 + W, min_size=0.002, max_size=1.5))
     cam = A.pinhole_for_vertical_fov((0.3, 0.2, 4.0), (0, 0, 0), W, H, 60.0)
-    s = _settings(W, H, background=(0.1, 0.3, 0.2, 0.4), depth_mode=int(W % 2))
+    s = _settings(W, H, background=(0.1, 0.3, 0.2, 0.4), depth_mode=threshold)
     edit = A.SplatEdit(active=True, mode=2, size=(1.0, 2.0, 2.0), opacity=opacity) if opacity != 1.0 else None
     got, want = _compare(oracle, None, raster, [packed], [np.eye(4)], cam.projection_for(W, H), s, edit=edit)
     np.testing.assert_array_equal(got["colour"], want["colour"])
     np.testing.assert_array_equal(got["depth"], want["depth"])
 
 
-def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(native, raster):
-    """A frame's pairs around the 8192 a block sorts by itself: the same image with the capacity a hundred pairs
-    need and with that of a frame before it that needed many."""
-    W, H = 160, 120
+# boxes of one pixel a lane and of two
+@pytest.mark.parametrize("size", [(1184, 1008), (1185, 1025)])
+@pytest.mark.parametrize("threshold", [0, 1])
+def test_frames_over_a_layer_equal_the_restatement_to_the_bit(oracle, native, size, threshold):
+    W, H = size
+    packed = _decode(oracle, random_cloud(900, 5, min_size=0.002, max_size=1.5))
+    cam = A.pinhole_for_vertical_fov((0.3, 0.2, 4.0), (0, 0, 0), W, H, 60.0).projection_for(W, H)
+    s = _settings(W, H, background=(0.1, 0.3, 0.2, 0.4), depth_mode=threshold)
+    drawn = oracle.render([(*packed, np.eye(4), 0)], oracle_projection(oracle, cam), W, H, bg=s.background, depth_mode=threshold)
+    gen = torch.Generator().manual_seed(W)
+    depth = 2.0 + torch.rand(W * H, generator=gen) * 5.0   # among the splats, from 2 to 6.5
+    depth[torch.rand(W * H, generator=gen) < 0.2] = 0.0
+    under, t = A.RenderTargets.make(W, H), A.RenderTargets.make(W, H)
+    under.colour.copy_(torch.rand((W * H, 4), generator=gen).cuda())
+    under.depth.copy_(depth.cuda())
+    A.TileRasterizer.create().render(cam, [A.SplatInstance(upload(packed))], s, t, under=under)
+    want = oracle.blend_over(drawn["frame"], drawn["binned"], drawn["proj"], under.colour.cpu().numpy(), depth.numpy())
+    np.testing.assert_array_equal(t.colour.cpu().numpy(), want["colour"])
+    np.testing.assert_array_equal(t.depth.cpu().numpy(), want["depth"])
+
+
+def test_the_last_capacity_of_one_block_sorts_and_the_next_agree(oracle, native):
+    """After release_scratch a frame's pairs have room for a seventh more than they are: 7168 pairs for 8192, which one
+    block sorts, 7169 for 8193, which tiles do. The same frame by both, each splat inside a tile of its own."""
+    W, H = 160, 128
     cam = A.pinhole_for_vertical_fov((0, 0, 3), (0, 0, 0), W, H, 60.0).projection_for(W, H)
-    small, large = [cases._records(cases._gaussians(n, True, 1, 5)) for n in (3000, 60_000)]
-    small, large = [A.CloudLoader.upload(*r) for r in (small, large)]
-    images = []
-    for first in (None, large):
-        r = A.TileRasterizer.create()
-        t = A.RenderTargets.make(W, H)
-        if first is not None:
-            r.render(cam, [A.SplatInstance(first)], A.RenderSettings(width=W, height=H), t)
-        r.render(cam, [A.SplatInstance(small)], A.RenderSettings(width=W, height=H), t)
-        images.append((t.colour.cpu(), t.depth.cpu()))
-    assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
+    rng, b = np.random.default_rng(8), CloudBuilder()
+    for _ in range(7169):
+        z = rng.uniform(-0.3, 0.3)
+        at = 16 * rng.integers(0, (W // 16, H // 16)) + 8 + rng.uniform(-3, 3, 2) - (W / 2, H / 2)
+        x, y = at * (3.0 - z) / cam.focal_x
+        b.add(x, y, z, 0.05, 1e-3, 1e-3, 1e-3, (1, 0, 0, 0), rng.uniform(0, 1, 3))
+    more = _decode(oracle, b)
+    less = tuple(a[:7168] for a in more[:3]) + more[3:]
+    found = []
+    for first, pairs in ((less, 7168), (more, 7169)):
+        r, t = A.TileRasterizer.create(), A.RenderTargets.make(W, H)
+        r.release_scratch()
+        settings = A.RenderSettings(width=W, height=H, antialias=False)
+        assert r.render(cam, [A.SplatInstance(upload(first))], settings, t).pairs == pairs
+        r.render(cam, [A.SplatInstance(upload(less))], settings, t)
+        found.append((t.colour.cpu().numpy(), t.depth.cpu().numpy(), frame_buffers(r)))
+    for k in range(2):
+        np.testing.assert_array_equal(found[0][k], found[1][k])
+    for name in ("pair_keys", "pair_splats", "ranges"):
+        np.testing.assert_array_equal(found[0][2][name], found[1][2][name], err_msg=name)
 
 
 # one block up to 8192; 2048-key tiles up to 606,208; then tiles of 6144 (pairs)
