@@ -118,6 +118,23 @@ __device__ __forceinline__ void rectTile(uint32_t local, uint32_t cols, uint32_t
     c = local - r * cols;
 }
 
+// A lane's tiles of a rect `cols` wide, 32 apart in its row-major order.
+struct RectWalk {
+    uint32_t cols, col, row, stepCol, stepRow;
+    __device__ __forceinline__ RectWalk(uint32_t width, uint32_t lane) : cols(width) {
+        rectTile(lane, cols, col, row);
+        rectTile(32, cols, stepCol, stepRow);
+    }
+    __device__ __forceinline__ void next() {
+        col += stepCol;
+        row += stepRow;
+        if (col >= cols) {
+            col -= cols;
+            ++row;
+        }
+    }
+};
+
 // The least lane k whose inclusive sum `incl` passes q (q below the warp's total).
 __device__ __forceinline__ uint32_t ownerOf(uint32_t incl, uint32_t q) {
     uint32_t lo = 0;
@@ -143,6 +160,11 @@ __device__ __forceinline__ uint32_t warpInclusive(uint32_t v) {
 // their number in z, and its tiles are tested again where its pairs are written. A culled
 // slot is all zeros.
 constexpr uint32_t kMaskTiles = 64;
+// A rect of more than kListTiles tiles the projection counts by itself, kLargeRun tiles a lane
+// at once: the list's search and loads, one after another a tile, are a large rect's whole time,
+// for its warp is alone with it. Below, rects of all sizes share the list's lanes without a gap.
+// 3000 splats over most of 1920x1080: 3.63 ms by the list, so 1.03 (a thread a footprint 1.66).
+constexpr uint32_t kListTiles = 512, kLargeRun = 4;
 __device__ __forceinline__ void spanShape(uint4 s, uint32_t& cols, uint32_t& area, uint32_t& touched) {
     cols = (s.y & 0xFFFFu) - (s.x & 0xFFFFu) + 1;
     area = cols * ((s.y >> 16) - (s.x >> 16) + 1);
@@ -152,13 +174,13 @@ __device__ __forceinline__ void spanShape(uint4 s, uint32_t& cols, uint32_t& are
 // One thread a slot: projectSplat<0>, its record, rect and key. The tiles are tested by
 // warps: the candidates of a warp's 32 footprints (each footprint's screen rect, row-major)
 // are one list, lane l taking entry 32 c + l, so a warp's work is the sum of its rects,
-// where a thread a footprint took 32 times the largest. The warps of a block wait for each
+// where a thread a footprint took 32 times the largest (rects of hundreds of tiles apart: kListTiles). The warps of a block wait for each
 // other nowhere (but where a frame counts): the last to end adds the block's sums. 1.5M
 // splats at 1920x1080: 406 us, by lists 201, without a scan among the blocks 154; 6M at
 // 3840x2160: 4.52 ms, 1.23, 1.07.
 // kOne: a single instance, its constants among the kernel's.
 template <uint32_t L, bool kOne>
-__global__ void __launch_bounds__(kProjectThreads)
+__global__ void __launch_bounds__(kProjectThreads, 5)   // as its main path fits without a spill
     projectKernel(const FrameConst F, const __grid_constant__ InstanceConst one, const InstanceConst* __restrict__ inst,
                   uint32_t nInst, uint32_t slots,
                   uint32_t countCulls, float4* __restrict__ recs, uint4* __restrict__ spans,
@@ -169,7 +191,7 @@ __global__ void __launch_bounds__(kProjectThreads)
     __shared__ uint32_t sCloud[2 * kMaxClouds];   // count_splats: (visible, pairs) a cloud, this block's share
     __shared__ float4 sFoot[kProjectThreads];     // cx cy ca cb
     __shared__ float2 sFootRest[kProjectThreads]; // cc cutoff
-    __shared__ uint4 sRect[kProjectThreads];      // rx0 ry0 cols
+    __shared__ uint4 sRect[kProjectThreads];      // rx0 ry0 cols rows
     if (threadIdx.x == 0) sPairs = 0, sKept = sEnded = 0;
     if (threadIdx.x < 8) sCulled[threadIdx.x] = 0;
     if (countCulls && threadIdx.x < 2 * kMaxClouds) sCloud[threadIdx.x] = 0;
@@ -201,7 +223,7 @@ __global__ void __launch_bounds__(kProjectThreads)
                 rect = make_uint2(rx0 | (ry0 << 16), rx1 | (ry1 << 16));
                 sFoot[threadIdx.x] = make_float4(G.cx, G.cy, G.ca, G.cb);
                 sFootRest[threadIdx.x] = make_float2(G.cc, G.cutoff);
-                sRect[threadIdx.x] = make_uint4(rx0, ry0, rx1 - rx0 + 1, 0);
+                sRect[threadIdx.x] = make_uint4(rx0, ry0, rx1 - rx0 + 1, ry1 - ry0 + 1);
                 recs[(size_t)slot * 3 + 0] = make_float4(G.cx, G.cy, G.tz, G.cutoff);
                 recs[(size_t)slot * 3 + 1] = make_float4(G.ca, G.cb, G.cc, G.alpha);
             }
@@ -211,7 +233,8 @@ __global__ void __launch_bounds__(kProjectThreads)
     uint32_t touched = 0;
     unsigned long long mask = 0;
     {
-        const uint32_t incl = warpInclusive(area), excl = incl - area;
+        const uint32_t listed = area > kListTiles ? 0u : area;
+        const uint32_t incl = warpInclusive(listed), excl = incl - listed;
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
         __syncwarp();
         for (uint32_t q0 = 0; q0 < total; q0 += 32) {
@@ -237,6 +260,32 @@ __global__ void __launch_bounds__(kProjectThreads)
                 if (lo - excl < kMaskTiles) mask |= (unsigned long long)own << (lo - excl);
             }
         }
+    }
+    for (uint32_t left = __ballot_sync(0xFFFFFFFFu, area > kListTiles); left; left &= left - 1u) {
+        const uint32_t owner = (uint32_t)__ffs((int)left) - 1u, k = warp * 32 + owner;
+        const float4 f = sFoot[k];
+        const float2 rest = sFootRest[k];
+        const uint4 r = sRect[k];
+        RectWalk at(r.z, lane);
+        uint32_t mine = 0;
+        for (uint32_t q0 = lane; q0 < r.z * r.w; q0 += 32 * kLargeRun) {
+            uint32_t near = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < kLargeRun; ++j, at.next()) {
+                const TileBox t(F.width, F.height, f.x, f.y, r.x + at.col, r.y + at.row);
+                const int estimate = powerEstimate(f.z, f.w, rest.x, rest.y, t.lox, t.loy, t.hix, t.hiy);
+                const bool here = q0 + 32 * j < r.z * r.w;
+                mine += here && estimate > 0 ? 1u : 0u;
+                near |= here && estimate == 0 ? 1u << j : 0u;
+            }
+            for (; near; near &= near - 1u) {
+                uint32_t col, row;
+                rectTile(q0 + 32 * ((uint32_t)__ffs((int)near) - 1u), r.z, col, row);
+                mine += tileTouched(F.width, F.height, f.x, f.y, f.z, f.w, rest.x, rest.y, r.x + col, r.y + row) ? 1u : 0u;
+            }
+        }
+        const uint32_t found = __reduce_add_sync(0xFFFFFFFFu, mine);
+        if (lane == owner) touched = found;
     }
     if (area && touched == 0) key = kCulledKey | kCullNoTile;
     const bool kept = touched != 0;
@@ -339,7 +388,7 @@ __device__ __forceinline__ uint32_t setBit(uint32_t lo, uint32_t hi, uint32_t k)
 // 32 splats' pairs as one list, lane l pair 32 c + l, from the masks of the tiles they
 // touch; where the splats' pairs start comes from a look-back over the blocks. Bound by
 // the splats' records, a sector each in depth order, and the pairs' writes. With rects,
-// masks, keys and offsets apart: 1.5M splats 102 us, so 73; 6M 692, so 515.
+// masks, keys and offsets apart 1.5M splats took 102 us, so 73; 6M 692, so 498.
 __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by five blocks an SM 91 and 619 us
     emitKernel(const FrameConst F, uint32_t slots, const uint32_t* __restrict__ order, const float4* __restrict__ recs,
                const uint4* __restrict__ spans, uint64_t* __restrict__ flags, uint32_t* __restrict__ words,
@@ -381,27 +430,35 @@ __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by 
     }
     __syncthreads();
     const uint64_t base = sPrefix + warpBase;
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
     const bool large = area > kMaskTiles;
+    const uint32_t anyLarge = __ballot_sync(0xFFFFFFFFu, large);
     const uint32_t rect0 = span.x, maskLo = span.z, maskHi = span.w;
-    const uint32_t tagged = slot, shape = cols | (large ? 1u << 31 : 0u);
+    // the list leaves out rects too large for a mask, whose pairs lie between the others' (walking past
+    // them there was a third of the kernel where splats cover the image: 4.0 ms for 3000, so 2.8)
+    uint32_t listIncl = incl, gap = 0;
+    if (anyLarge) {
+        listIncl = warpInclusive(large ? 0u : touched);
+        gap = incl - listIncl;
+    }
+    const uint32_t listExcl = listIncl - (large ? 0u : touched), total = __shfl_sync(0xFFFFFFFFu, listIncl, 31);
     for (uint32_t q0 = 0; q0 < total; q0 += 32) {
         const uint32_t q = q0 + lane;
-        const uint32_t owner = ownerOf(incl, min(q, total - 1u));
-        const uint32_t k = q - __shfl_sync(0xFFFFFFFFu, excl, owner);
-        const uint32_t oRect = __shfl_sync(0xFFFFFFFFu, rect0, owner), oShape = __shfl_sync(0xFFFFFFFFu, shape, owner);
+        const uint32_t owner = ownerOf(listIncl, min(q, total - 1u));
+        const uint32_t k = q - __shfl_sync(0xFFFFFFFFu, listExcl, owner);
+        const uint32_t oRect = __shfl_sync(0xFFFFFFFFu, rect0, owner), oCols = __shfl_sync(0xFFFFFFFFu, cols, owner);
         const uint32_t oLo = __shfl_sync(0xFFFFFFFFu, maskLo, owner), oHi = __shfl_sync(0xFFFFFFFFu, maskHi, owner);
-        const uint32_t oSlot = __shfl_sync(0xFFFFFFFFu, tagged, owner);
-        if (q >= total || (oShape >> 31)) continue;
+        const uint32_t oSlot = __shfl_sync(0xFFFFFFFFu, slot, owner);
+        const uint32_t skipped = anyLarge ? __shfl_sync(0xFFFFFFFFu, gap, owner) : 0u;
+        if (q >= total) continue;
         uint32_t col, row;
-        rectTile(setBit(oLo, oHi, k), oShape, col, row);
+        rectTile(setBit(oLo, oHi, k), oCols, col, row);
         const uint32_t tile = ((oRect >> 16) + row) * F.tilesX + (oRect & 0xFFFFu) + col;
-        const uint64_t at = base + q;
+        const uint64_t at = base + skipped + q;
         if (at < capacity) pairs[at] = ((uint64_t)tile << 32) | oSlot;
     }
     // rects too large for a mask: the warp tests their tiles again, one splat after another
-    for (uint32_t left = __ballot_sync(0xFFFFFFFFu, large); left; left &= left - 1u) {
-        const uint32_t owner = (uint32_t)__ffs(left) - 1u;
+    for (uint32_t left = anyLarge; left; left &= left - 1u) {
+        const uint32_t owner = (uint32_t)__ffs((int)left) - 1u;
         const uint32_t oSlot = __shfl_sync(0xFFFFFFFFu, slot, owner), oRect = __shfl_sync(0xFFFFFFFFu, rect0, owner);
         const uint32_t oCols = __shfl_sync(0xFFFFFFFFu, cols, owner), oArea = __shfl_sync(0xFFFFFFFFu, area, owner);
         const uint32_t expected = __shfl_sync(0xFFFFFFFFu, touched, owner);

@@ -168,14 +168,36 @@ __device__ __forceinline__ bool powerWithin(float a, float b, float c, float cut
     return minPowerOverBox(a, b, c, lox, loy, hix, hiy) <= cutoff;
 }
 
+// A tile's pixel centres about a footprint's centre: the box that its test is over.
+struct TileBox {
+    float lox, loy, hix, hiy;
+    __device__ __forceinline__ TileBox(uint32_t width, uint32_t height, float cx, float cy, uint32_t tx, uint32_t ty) {
+        lox = ((float)(tx * kTile) + 0.5f) - cx;
+        loy = ((float)(ty * kTile) + 0.5f) - cy;
+        hix = ((float)(min((tx + 1) * kTile, width) - 1) + 0.5f) - cx;
+        hiy = ((float)(min((ty + 1) * kTile, height) - 1) + 0.5f) - cy;
+    }
+};
+
 // frame.slang:374-379: does tile (tx, ty) hold a pixel centre inside the footprint?
 __device__ __forceinline__ bool tileTouched(uint32_t width, uint32_t height, float cx, float cy, float ca, float cb,
                                             float cc, float cutoff, uint32_t tx, uint32_t ty) {
-    const float fx = (float)(tx * kTile) + 0.5f;
-    const float fy = (float)(ty * kTile) + 0.5f;
-    const float lx = (float)(min((tx + 1) * kTile, width) - 1) + 0.5f;
-    const float ly = (float)(min((ty + 1) * kTile, height) - 1) + 0.5f;
-    return powerWithin(ca, cb, cc, cutoff, fx - cx, fy - cy, lx - cx, ly - cy);
+    const TileBox t(width, height, cx, cy, tx, ty);
+    return powerWithin(ca, cb, cc, cutoff, t.lox, t.loy, t.hix, t.hiy);
+}
+
+// powerWithin's estimate without branches, for several at once: 1 within, -1 not, 0 where the exact minimum decides.
+__device__ __forceinline__ int powerEstimate(float a, float b, float c, float cutoff, float lox, float loy, float hix,
+                                             float hiy) {
+    const float X = fmaxf(fabsf(lox), fabsf(hix)), Y = fmaxf(fabsf(loy), fabsf(hiy)), b2 = 2.0f * b;
+    const float margin = 4e-6f * __fmaf_rn(a * X, X, __fmaf_rn(fabsf(b2) * X, Y, (c * Y) * Y));
+    const float ex = clampf(0.0f, lox, hix), ey = clampf(0.0f, loy, hiy);
+    const float y = clampf(__fdividef(-b * ex, c), loy, hiy), x = clampf(__fdividef(-b * ey, a), lox, hix);
+    const float onX = ex != 0.0f ? __fmaf_rn(a * ex, ex, y * __fmaf_rn(c, y, b2 * ex)) : 3.4e38f;
+    const float onY = ey != 0.0f ? __fmaf_rn(c * ey, ey, x * __fmaf_rn(a, x, b2 * ey)) : 3.4e38f;
+    const float over = fminf(onX, onY) - cutoff;
+    const bool sure = a > 1e-12f && c > 1e-12f && (ex != 0.0f || ey != 0.0f);
+    return !sure ? 0 : over > margin ? -1 : over < -margin ? 1 : 0;
 }
 
 // common/color.slang:7-10
