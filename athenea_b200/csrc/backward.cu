@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256)
         }
     }
     // a block's places by one addition: one a warp, all to one word, was most of the
-    // kernel (500k Gaussians: 14 us, so 7)
+    // kernel (500k Gaussians: 14 us, now 7)
     __shared__ uint32_t sCount[8], sFirst;
     const uint32_t warp = threadIdx.x >> 5, ballot = __ballot_sync(0xFFFFFFFFu, some);
     if (lane == 0) sCount[warp] = __popc(ballot);
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(128)
 // *loss) and dL/dcolour (float4 a pixel, alpha 0). The threads' shares are summed in 64
 // bits over a cluster of blocks, one 32-bit addition into *loss a cluster, 148 at most: one
 // a block of 256 pixels, thousands an image, each rounded *loss, 3e-6 of it in all at
-// 1920x1080 (so 3e-7), though without clusters the blocks drift apart less where the target
+// 1920x1080 (3e-7 now), though without clusters the blocks drift apart less where the target
 // comes from memory. The grid fills every SM once, which takes 32 registers a thread, and
 // a block writes its sum into the first block's shared memory, a barrier's first half at the
 // start standing for that block's being there. 333x251: 2.6 us a block at a time, 3.3 so

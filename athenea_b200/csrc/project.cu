@@ -163,7 +163,7 @@ constexpr uint32_t kMaskTiles = 64;
 // A rect of more than kListTiles tiles the projection counts by itself, kLargeRun tiles a lane
 // at once: the list's search and loads, one after another a tile, are a large rect's whole time,
 // for its warp is alone with it. Below, rects of all sizes share the list's lanes without a gap.
-// 3000 splats over most of 1920x1080: 3.63 ms by the list, so 1.03 (a thread a footprint 1.66).
+// 3000 splats over most of 1920x1080: 3.63 ms by the list, 1.03 now (a thread a footprint 1.66).
 constexpr uint32_t kListTiles = 512, kLargeRun = 4;
 __device__ __forceinline__ void spanShape(uint4 s, uint32_t& cols, uint32_t& area, uint32_t& touched) {
     cols = (s.y & 0xFFFFu) - (s.x & 0xFFFFu) + 1;
@@ -388,7 +388,7 @@ __device__ __forceinline__ uint32_t setBit(uint32_t lo, uint32_t hi, uint32_t k)
 // 32 splats' pairs as one list, lane l pair 32 c + l, from the masks of the tiles they
 // touch; where the splats' pairs start comes from a look-back over the blocks. Bound by
 // the splats' records, a sector each in depth order, and the pairs' writes. With rects,
-// masks, keys and offsets apart 1.5M splats took 102 us, so 73; 6M 692, so 498.
+// masks, keys and offsets apart 1.5M splats took 102 us, now 73; 6M 692, now 498.
 __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by five blocks an SM 91 and 619 us
     emitKernel(const FrameConst F, uint32_t slots, const uint32_t* __restrict__ order, const float4* __restrict__ recs,
                const uint4* __restrict__ spans, uint64_t* __restrict__ flags, uint32_t* __restrict__ words,
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by 
     const uint32_t anyLarge = __ballot_sync(0xFFFFFFFFu, large);
     const uint32_t rect0 = span.x, maskLo = span.z, maskHi = span.w;
     // the list leaves out rects too large for a mask, whose pairs lie between the others' (walking past
-    // them there was a third of the kernel where splats cover the image: 4.0 ms for 3000, so 2.8)
+    // them there was a third of the kernel where splats cover the image: 4.0 ms for 3000, now 2.8)
     uint32_t listIncl = incl, gap = 0;
     if (anyLarge) {
         listIncl = warpInclusive(large ? 0u : touched);

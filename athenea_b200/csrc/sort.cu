@@ -48,7 +48,7 @@ __device__ __forceinline__ uint32_t digitSlot(uint32_t d) { return d ^ ((d >> 5)
 
 // A sort's passes over bits [firstBit, firstBit + bits): `wide` digits of nine bits, then
 // eights. Worked out where it is asked for: with arrays among a kernel's constants, looked up
-// by pass, the one-block sort of 5k depths took 16.9 us, so 12.8.
+// by pass, the one-block sort of 5k depths took 16.9 us, now 12.8.
 struct SortPlan {
     uint32_t passes, bits, wide;
     __host__ __device__ uint32_t width(uint32_t p) const { return p < wide ? 9u : 8u; }
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256)
     // A thread takes a run of eight keys, all in flight before their counts, and counts equal
     // digits that follow each other at once: the high digits of pairs written splat by splat are
     // alike, and lanes that count the same digit wait for each other. 6M
-    // splats' pairs at 3840x2160: 249 us, so 157; 8M random keys 33, so 30.
+    // splats' pairs at 3840x2160: 249 us, now 157; 8M random keys 33, now 30.
     constexpr uint32_t kRun = 8, kVector = 16 / sizeof(K);
     const bool aligned = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0;
     const uint64_t threads = (uint64_t)gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x;
@@ -203,7 +203,9 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
     // lane l being the (k*32 + l)-th; walking k then l is input order, so the
     // ranks are stable. A key's peers, the warp's keys of its digit, are the bits their lanes
     // set in the digit's mask: __match_any_sync takes some 240 cycles of an SM's quarter where
-    // 32 digits differ, and was most of a pass; the masks take 35 there, 130 where all agree.
+    // 32 digits differ, and was most of a pass; the masks take 35 there, 130 where all agree. (A
+    // warp's ranking by masks of lanes is the warp-level multisplit of S. Ashkiani et al., "GPU
+    // Multisplit", PPoPP 2016, which makes them by ballots.)
     const uint32_t mine = base + warp * 32 * kPerThread + lane;
     K key[kPerThread];
     uint32_t rank[kPerThread];
@@ -339,8 +341,9 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
 // A whole sort of at most kSortTileKeys keys in one block: the passes of `plan` one after
 // another, the keys (and values) carried in registers and reordered through shared memory.
 // A small sort's passes are latency alone, each some 6 us as a kernel; in one block they
-// need no histograms, look-back, tickets or clearing either. A frame of 5k splats: 144 -> 127 us. Every key is
-// read before the first is written, so the output may be the input.
+// need no histograms, look-back, tickets or clearing either. A frame of 5k splats: 144 -> 140 us
+// (128 now: the masks below, and SortPlan). Every key is read before the first is written, so the
+// output may be the input.
 template <typename K, uint32_t kValues>
 __host__ __device__ constexpr size_t smallKeysSmem() { return kSortTileKeys * (sizeof(K) + (kValues == kNoValues ? 0 : 4)); }
 template <typename K, uint32_t kValues>
@@ -567,7 +570,7 @@ cudaError_t runSort(uint32_t n, const uint32_t* nDevice, const uint32_t* epochDe
 // keys/vals[0] hold the input; the sorted result lands in keys/vals[sortResultIndex(n, bits)]
 // (n as given here, also where nDevice holds the count). vals may be null (keys only). The passes
 // sort bits [firstBit, firstBit + bits) of the keys, eight or nine at a time
-// (planSort). hist: kMaxPasses * kSortHistStride words, flags: sortFlagWords
+// (planSort). hist: kMaxPasses * kMaxRadix words, flags: sortFlagWords
 // words, tickets: one word a pass; all three start at zero (`clear`: what of them is
 // zeroed here). tileKeys: kSortTileKeys for callers whose flags hold no more than that
 // takes; 0 by the count.

@@ -148,9 +148,9 @@ __device__ __forceinline__ float minPowerOverBox(float a, float b, float c, floa
 // minPowerOverBox(...) <= cutoff, decided by an estimate where that is certain: the least
 // power over the edges that face the centre (the form is positive up to its entries'
 // rounding, so no other edge holds less), with approximate divisions. It is off from
-// minPowerOverBox's by at most some ten roundings of the largest term the power has over the
-// box; past four times that the answer stands, else minPowerOverBox gives it. Its four exact
-// divisions were over a third of a tile's test.
+// minPowerOverBox's by at most some ten roundings (of 2^-24 each) of the largest term the power has
+// over the box; 4e-6 of that term is 67 of them, and past it the answer stands, else
+// minPowerOverBox gives it. Its four exact divisions were over a third of a tile's test.
 __device__ __forceinline__ bool powerWithin(float a, float b, float c, float cutoff, float lox, float loy, float hix,
                                             float hiy) {
     if (lox <= 0.0f && hix >= 0.0f && loy <= 0.0f && hiy >= 0.0f) return 0.0f <= cutoff;

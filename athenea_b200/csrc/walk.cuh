@@ -66,9 +66,9 @@ struct Box {
 // one pixel a lane: half the work a warp, twice the warps, where warps are too few to
 // hide each other's latency and the longest lists' boxes end last. A training pass, whose
 // adjoint reads and tests each record once a box, does so up to 64 boxes an SM, a frame up to 128.
-// By one and by two: frames of 100k splats at 960x540 (55 an SM) 233 and 262 us, of 1.5M at
-// 1280x720 (97) 743 and 755, at 1920x1080 (221) 876 and 870; passes over 500k Gaussians at
-// 960x540 763 and 793 us, at 1280x720 885 and 856.
+// By one and by two: frames of 100k splats at 960x540 (55 an SM) 218 and 246 us, of 1.5M at
+// 1280x720 (97) 613 and 626, at 1920x1080 (221) 818 and 813; passes over 500k Gaussians at
+// 960x540 708 and 729 us, at 1280x720 828 and 789.
 inline bool onePixelBoxes(uint32_t tiles, uint32_t sms, bool training) {
     return tiles * Box<2>::kCount < sms * (training ? 64u : 128u);
 }

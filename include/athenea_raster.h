@@ -219,7 +219,9 @@ ath_status ath_settings_default(ath_settings* out);
 ath_status ath_raster_create(ath_raster** out);
 /* ~TileRasterizer: frees the scratch; the handle is gone. */
 void ath_raster_destroy(ath_raster* r);
-/* TileRasterizer::releaseScratch (TileRasterizer.h:482; TileRasterizer.cpp:178-191). */
+/* TileRasterizer::releaseScratch (TileRasterizer.h:482; TileRasterizer.cpp:178-191). Waits for the
+ * device. Also gives back what ath_decode_records keeps for the calling thread; another thread's
+ * stays, in ath_memory_held too, until that thread calls this or ends. */
 ath_status ath_raster_release_scratch(ath_raster* r);
 
 /* TileRasterizer::render(const Projection&, span<const SplatInstance>,
@@ -490,7 +492,10 @@ ath_status ath_raster_check(ath_raster* r, ath_frame_stats* out);
 
 /* The last frame's intermediate buffers, for inspection (what the reference's
  * tests read through its Buffer handles). Device pointers owned by the
- * rasteriser, valid until its next render or release_scratch:
+ * rasteriser, valid until its next render or release_scratch. Waits for the frame; some of them are
+ * made by the call, in device memory that the handle keeps from its first (4 bytes a pair and 12 a
+ * slot: ATH_E_OUT_OF_MEMORY where it cannot be had). ATH_E_NOT_FOUND: no frame yet, or the last one
+ * failed, whose buffers may be gone.
  *   records    12 floats a slot: screen (centre xy, view z, cutoff), conic (a b c, alpha),
  *              colour (rgb, 0) -- splat/frame.slang:269-281's ProjRecord without the surfel
  *              word; written for kept slots only
@@ -526,10 +531,10 @@ void ath_sorter_destroy(ath_sorter* s);
 
 /* RadixSort::sort(batch, SortBuffers, count, keyBits): sorts the first `count`
  * (key, value) pairs stably by the low `key_bits` bits (1..64) of the key,
- * eight bits a pass. keys/values hold the input and receive the result; the
+ * eight or nine bits a pass; the bits above take no part. keys/values hold the input and receive the result; the
  * scratch pair (as SortBuffers' scratchKeys/scratchValues) holds count
- * entries each. An odd number of passes ends with a copy back. Enqueued on
- * `stream`, not waited for, and nothing is read back: what the sorts raise is
+ * entries each. An odd number of passes ends with a copy back (up to 8192 pairs
+ * sort in place). Enqueued on `stream`, not waited for, and nothing is read back: what the sorts raise is
  * kept for ath_sorter_check. */
 ath_status ath_sorter_sort(ath_sorter* s, uint64_t* keys, uint32_t* values, uint64_t* scratch_keys,
                            uint32_t* scratch_values, uint32_t count, uint32_t key_bits, void* stream);
@@ -565,7 +570,8 @@ ath_status ath_sort_pairs_static_status(void* stream);
  * wxyz rotation, SH DC, rest colour-outer). `records` is device memory,
  * `count` records of `stride` floats; field indices as named. The valid
  * records are written compacted, in file order, to positions/shape/sh (room
- * for `count` splats); *kept receives how many (a device-to-host read). */
+ * for `count` splats); *kept receives how many (a device-to-host read). Up to
+ * 1 MiB of device scratch stays with the calling thread for its next call. */
 typedef struct {
     uint32_t stride;
     uint32_t x, y, z, opacity, scale0, scale1, scale2, rot_w, rot_x, rot_y, rot_z, dc0, dc1, dc2;
