@@ -613,7 +613,7 @@ ath_status drawFrame(ath_raster* r, const FrameConst& F, InstanceConst* staged, 
     uint32_t* hist = static_cast<uint32_t*>(r->sortScratch.ptr);   // null, and not used, for a sort in one block
     uint64_t* flags = hist ? reinterpret_cast<uint64_t*>(static_cast<char*>(r->sortScratch.ptr) + kSortHistBytes) : nullptr;
     uint64_t** pairs = r->pairs;
-    err = launchSortDepths(r->slot.keys, r->slot.depthKeys, r->slot.depthSlots, slots,
+    err = launchSortDepths(r->slot.keys, r->slot.depthKeys, r->slot.depthSlots, slots, words + kWordVisible,
                            reinterpret_cast<uint32_t*>(zero + zeroed.depthHist),
                            reinterpret_cast<uint64_t*>(zero + zeroed.depthFlags), words + kWordDepthTickets,
                            words + kWordSticky, stream);

@@ -24,7 +24,8 @@ uint32_t projectBlocks(uint32_t slots);   // also the look-back words of the emi
 cudaError_t launchProject(const FrameConst& F, const InstanceConst& one, const InstanceConst* inst, uint32_t nInst, uint32_t slots,
                           uint32_t layout, bool countCulls, float4* recs, uint4* spans, uint32_t* keys, uint32_t* words,
                           cudaStream_t stream);
-// The pairs (tile << 32 | slot) of the slots in `order` (the depth sort's). Writes the pairs the
+// The pairs (tile << 32 | slot) of the visible slots in `order` (the depth sort's; words[kWordVisible] of
+// them, at most `slots`). Writes the pairs the
 // buffers hold, min(pairs, capacity), into words[kWordPairsKept], and raises kStatusPairOverflow in
 // words[kWordSticky] past the capacity. flags: projectBlocks(slots) words, zeroed by the caller.
 cudaError_t launchEmit(const FrameConst& F, uint32_t slots, const uint32_t* order, const float4* recs,
@@ -65,12 +66,13 @@ cudaError_t launchSortDevice(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, c
                              uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream,
                              SortClear clear = kClearAll, uint32_t tileKeys = 0);
 
-// A frame's splats front to back: the slots sorted stably by the low 24 bits of `keys` (left as
-// they are), into slots[0]; sortKeys and slots: room for n each. Culled slots (keys of
-// kCulledKey and a reason) come first. hist (three passes' worth), flags and tickets: zeroed by
-// the caller.
-cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n, uint32_t* hist,
-                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream);
+// A frame's visible splats front to back: the slots sorted stably by the low 24 bits of `keys` (left
+// as they are), into slots[0], *visible of them (the culled ones, keys of kCulledKey and a reason,
+// are left out; past the visible ones slots[0] holds nothing of use). sortKeys and slots: room for n
+// each. hist (three passes' worth), flags and tickets: zeroed by the caller.
+cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n,
+                             const uint32_t* visible, uint32_t* hist, uint64_t* flags, uint32_t* tickets, uint32_t* status,
+                             cudaStream_t stream);
 constexpr uint32_t kDepthBits = 24;
 
 // blend.cu

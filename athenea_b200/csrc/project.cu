@@ -396,9 +396,11 @@ __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by 
     __shared__ uint32_t sTicket;
     __shared__ uint32_t sWarp[kProjectThreads / 32];
     __shared__ uint64_t sPrefix;
+    const uint32_t visible = min(slots, words[kWordVisible]);
     if (threadIdx.x == 0) sTicket = atomicAdd(&words[kWordEmitTicket], 1u);
     __syncthreads();
     const uint32_t b = sTicket;
+    if (b != 0 && b * kProjectThreads >= visible) return;   // past the visible slots: no block waits for this one
     const uint32_t i = b * kProjectThreads + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint64_t all = (uint64_t)words[kWordPairsLo] | ((uint64_t)words[kWordPairsHi] << 32);
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(kProjectThreads, 8)   // it waits, mostly: by 
     }
     uint32_t slot = 0, touched, cols, area;
     uint4 span = make_uint4(0, 0, 0, 0);
-    if (i < slots) {
+    if (i < visible) {
         slot = order[i];
         if (slot < slots) span = spans[slot];
     }

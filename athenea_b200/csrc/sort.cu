@@ -14,6 +14,7 @@
 
 #include "kernels.h"
 #include "raster_types.cuh"
+#include "splat_math.cuh"
 
 namespace ath {
 namespace {
@@ -94,20 +95,29 @@ __global__ void __launch_bounds__(256)
         for (uint32_t p = 0; p < kMaxPasses; ++p) {
             if (p >= plan.passes) break;
             const uint32_t shift = firstBit + plan.shift(p), mask = plan.mask(p);
-            uint32_t run = (uint32_t)(key[0] >> shift) & mask, length = 1;
+            // a frame's depths: a culled slot's key counts as no digit (a run with some of them counted by
+            // a second copy of this costs more, 12 us for 1.5M slots: lanes differ; this 8.8, without 7.3)
+            auto digitOf = [&](K k) {
+                const uint32_t d = (uint32_t)(k >> shift) & mask;
+                return sizeof(K) == 4 && k >= (K)kCulledKey ? kMaxRadix : d;
+            };
+            auto add = [&](uint32_t d, uint32_t times) {
+                if (sizeof(K) == 8 || d < kMaxRadix) atomicAdd(&sHist[p * kMaxRadix + digitSlot(d)], times);
+            };
+            uint32_t run = digitOf(key[0]), length = 1;
 #pragma unroll
             for (uint32_t k = 1; k < kRun; ++k) {
                 if (k >= count) break;
-                const uint32_t d = (uint32_t)(key[k] >> shift) & mask;
+                const uint32_t d = digitOf(key[k]);
                 if (d == run) {
                     ++length;
                 } else {
-                    atomicAdd(&sHist[p * kMaxRadix + digitSlot(run)], length);
+                    add(run, length);
                     run = d;
                     length = 1;
                 }
             }
-            atomicAdd(&sHist[p * kMaxRadix + digitSlot(run)], length);
+            add(run, length);
         }
     }
     __syncthreads();
@@ -171,12 +181,15 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
     constexpr uint32_t kCounters = rankChains<kBits, kPerThread>(), kChains = kCounters / kWarps;
     constexpr uint32_t kChainItems = kPerThread / kChains;
     constexpr uint32_t kTileKeys = kSortThreads * kPerThread;
+    // The first pass of a frame's depths leaves culled slots out: the passes after it, and the emit,
+    // take the visible ones alone.
+    constexpr bool kDrop = kValues == kIndexValues;
     extern __shared__ __align__(16) unsigned char smem[];
     K* sKeys = reinterpret_cast<K*>(smem);
     uint32_t* sVals = reinterpret_cast<uint32_t*>(smem);
     uint32_t* sMasks = reinterpret_cast<uint32_t*>(smem);   // kCounters x kRadix, while the keys are ranked
     uint32_t* sWarpCnt = reinterpret_cast<uint32_t*>(smem + rankSmem<K, kBits, kPerThread>());   // kCounters x kRadix
-    __shared__ uint32_t sTile;
+    __shared__ uint32_t sTile, sKept;
     __shared__ uint32_t sStart[kRadix];
     __shared__ uint32_t sAdjust[kRadix];
     __shared__ uint32_t sScan[kWarps];
@@ -210,7 +223,8 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
     K key[kPerThread];
     uint32_t rank[kPerThread];
 #pragma unroll
-    for (uint32_t k = 0; k < kPerThread; ++k) key[k] = mine + k * 32 < n ? keysIn[mine + k * 32] : (K)0;
+    for (uint32_t k = 0; k < kPerThread; ++k) key[k] = mine + k * 32 < n ? keysIn[mine + k * 32] : (K)(kDrop ? kCulledKey : 0u);
+    auto takes = [&](uint32_t k) { return kDrop ? key[k] < (K)kCulledKey : mine + k * 32 < n; };
 #pragma unroll
     for (uint32_t i = 0; i < kChainItems; ++i) {
         uint32_t at[kChains], peers[kChains], before[kChains];
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
 #pragma unroll
         for (uint32_t c = 0; c < kChains; ++c) {
             const uint32_t k = c * kChainItems + i;
-            valid[c] = mine + k * 32 < n;
+            valid[c] = takes(k);
             at[c] = (warp * kChains + c) * kRadix + digitSlot((uint32_t)((key[k] >> shift) & digitMask));
             if (valid[c]) atomicOr(&sMasks[at[c]], 1u << lane);
         }
@@ -289,6 +303,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
         sStart[digitSlot(t)] = start;
         sAdjust[digitSlot(t)] = exclusive - start;
     }
+    if (kDrop && tid == kRadix - 1) sKept = start + count;
     __syncthreads();
 
     // Scatter into shared memory in the tile's sorted order, then out.
@@ -296,7 +311,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
 #pragma unroll
     for (uint32_t k = 0; k < kPerThread; ++k) {
         uint32_t s = 0;
-        if (mine + k * 32 < n) {
+        if (takes(k)) {
             const uint32_t at = digitSlot((uint32_t)((key[k] >> shift) & digitMask));
             s = sStart[at] + sWarpCnt[(warp * kChains + k / kChainItems) * kRadix + at] + rank[k];
             sKeys[s] = key[k];
@@ -304,7 +319,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
         place[k / 2] = k & 1u ? place[k / 2] | (s << 16) : s;
     }
     __syncthreads();
-    const uint32_t tileN = min(kTileKeys, n - base);
+    const uint32_t tileN = kDrop ? sKept : min(kTileKeys, n - base);
     uint32_t to[kValues == kNoValues ? 1 : kPerThread];
 #pragma unroll
     for (uint32_t k = 0; k < kPerThread; ++k) {
@@ -330,7 +345,7 @@ __global__ void __launch_bounds__(kSortThreads, sizeof(K) == 8 && kValues != kNo
         __syncthreads();
 #pragma unroll
         for (uint32_t k = 0; k < kPerThread; ++k)
-            if (mine + k * 32 < n) sVals[(place[k / 2] >> (16 * (k & 1u))) & 0xFFFFu] = val[k];
+            if (takes(k)) sVals[(place[k / 2] >> (16 * (k & 1u))) & 0xFFFFu] = val[k];
         __syncthreads();
 #pragma unroll
         for (uint32_t k = 0; k < kPerThread; ++k)
@@ -371,6 +386,7 @@ __global__ void __launch_bounds__(kSortThreads)
         const uint32_t i = mine + k * 32;
         const bool valid = k < perThread && i < n;
         key[k] = valid ? keysIn[i] : (K)0;
+        if (kValues == kIndexValues && key[k] >= (K)kCulledKey) key[k] = (K)((1u << kDepthBits) - 1u);   // past any depth: last
         if constexpr (kValues == kReadValues) val[k] = valid ? valsIn[i] : 0u;
         if constexpr (kValues == kIndexValues) val[k] = i;
     }
@@ -615,16 +631,17 @@ cudaError_t launchSort(uint64_t* keys[2], uint32_t* vals[2], uint32_t n, uint32_
     return launchSortDevice(keys, vals, n, nullptr, nullptr, 0, bits, hist, flags, tickets, status, stream, clear, tileKeys);
 }
 
-cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n, uint32_t* hist,
-                             uint64_t* flags, uint32_t* tickets, uint32_t* status, cudaStream_t stream) {
+cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32_t* slots[2], uint32_t n,
+                             const uint32_t* visible, uint32_t* hist, uint64_t* flags, uint32_t* tickets, uint32_t* status,
+                             cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     if (n <= kSortTileKeys) {
         smallSortKernel<uint32_t, kIndexValues><<<1, kSortThreads, smallSortSmem<uint32_t, kIndexValues>(), stream>>>(
             keys, nullptr, nullptr, slots[0], n, nullptr, 0, planSort(kDepthBits));
         return cudaGetLastError();
     }
-    // three 8-bit passes: keys -> [0] -> [1] -> [0], the first carrying its keys' places, the
-    // last writing the slots alone
+    // three 8-bit passes: keys -> [0] -> [1] -> [0], the first carrying its keys' places and leaving
+    // the culled ones out, the last writing the slots alone
     auto pass = [&](uint32_t p, const SortPlan& plan, uint32_t tileKeys, uint32_t tiles, uint32_t shift, const uint32_t* h,
                     uint64_t* f, uint32_t* ticket, uint32_t mask) {
         const uint32_t out = p & 1u, in = out ^ 1u;
@@ -634,7 +651,7 @@ cudaError_t launchSortDepths(const uint32_t* keys, uint32_t* sortKeys[2], uint32
                                                   status, nullptr, nullptr, mask, stream);
         else
             launchPass<uint32_t, kReadValues, 8>(tileKeys, tiles, sortKeys[in], slots[in], ko, slots[out], n, shift, h, f,
-                                                 ticket, status, nullptr, nullptr, mask, stream);
+                                                 ticket, status, visible, nullptr, mask, stream);
     };
     static_assert(kDepthBits == 24, "three 8-bit passes");
     return runSort<uint32_t>(n, nullptr, nullptr, 0, kDepthBits, 0, kClearNone, hist, flags, tickets, stream, keys, false, pass);

@@ -201,3 +201,31 @@ def test_the_l2_loss_at_every_size(native, pixels):
     assert abs(loss.item() - want) <= 1e-6 * want
     assert float((dl[:, :3].double() - 2.0 * error / (3.0 * pixels)).abs().max()) <= 1e-6 / (3.0 * pixels)
     assert not bool(dl[:, 3].any())
+
+
+# depth sorts in one block, in small tiles and in large ones; none, one and some of the slots in sight
+@pytest.mark.parametrize("slots", [5000, 20_011, 700_003])
+@pytest.mark.parametrize("seen", [0, 1, 257, 4000])
+def test_a_cloud_mostly_out_of_sight_draws_as_what_is_in_sight(native, slots, seen):
+    p = scenes.params(seen + 1, True, 21, 3)
+    few = A.Params(*[torch.from_numpy(np.ascontiguousarray(p[k][:seen])).cuda() for k in ("means", "scales", "quats", "sh")], 3)
+    gen = torch.Generator(device="cuda").manual_seed(slots)
+    at = torch.randperm(slots, generator=gen, device="cuda")[:seen].sort().values   # in order: ties in depth keep it
+    means = torch.zeros((slots, 4), device="cuda")
+    means[:, 2] = 10.0   # behind the camera
+    scales, quats = torch.full_like(means, -4.0), torch.ones_like(means)
+    sh = torch.zeros((slots, few.sh.shape[1]), device="cuda")
+    for whole, part in ((means, few.means), (scales, few.scales), (quats, few.quats), (sh, few.sh)):
+        whole[at] = part
+    W, H = 320, 200
+    cam = A.pinhole_for_vertical_fov((0, 0, 3), (0, 0, 0), W, H, 60.0).projection_for(W, H)
+    images, slot_of = [], []
+    for cloud in (A.Params(means, scales, quats, sh, 3), few):
+        r, t = A.TileRasterizer.create(), A.RenderTargets.make(W, H)
+        for _ in range(2):   # sized by its own pairs, then as any later frame
+            stats = r.render_params(cam, cloud, A.RenderSettings(width=W, height=H), t)
+        images.append((t.colour.cpu(), t.depth.cpu()))
+        slot_of.append(torch.from_numpy(frame_buffers(r)["pair_splats"].astype(np.int64)))
+        assert stats.visible <= seen
+    assert torch.equal(images[0][0], images[1][0]) and torch.equal(images[0][1], images[1][1])
+    assert torch.equal(slot_of[0], at.cpu()[slot_of[1]])
