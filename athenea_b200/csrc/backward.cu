@@ -236,8 +236,16 @@ __global__ void __launch_bounds__(Box<kPx>::kThreads)   // what shared memory an
                 __syncwarp();   // the next records overwrite the columns
             }
             };
-            if (odd) walk(std::true_type());
-            else walk(std::false_type());
+            if (odd) {
+                walk(std::true_type());
+                // a pixel that blended a colour past the limit has it behind the records in front
+                bool past = false;
+#pragma unroll
+                for (int p = 0; p < kPx; ++p) past = past || !(fabsf(sd.v[p]) < kWalkLimit);
+                wild = wild || __any_sync(0xFFFFFFFFu, past);
+            } else {
+                walk(std::false_type());
+            }
         }
     }
 }

@@ -284,3 +284,28 @@ def test_a_gradient_that_is_not_finite_stays_with_its_pixels_gaussians(raster, s
     for a, b in ((got[~blends], base[~blends]), (rows[~blends], want[~blends])):
         assert np.isfinite(a).all()
         np.testing.assert_allclose(a, b, rtol=1e-3, atol=1e-5 * np.abs(b).max())   # the order of the atomic sums
+
+
+@pytest.mark.parametrize("size", [(320, 200), (1184, 528)])
+def test_a_colour_that_is_not_finite_stays_with_the_gaussians_it_shares_pixels_with(raster, size):
+    """Gaussians far behind the others get an infinite red: what lies in front of them at a pixel has lost its
+    gradient, the other Gaussians of the tile have not."""
+    W, H = size
+    p = scenes.params(60_000, True, 33, 3)
+    p["means"][:, 3] = -2.0   # faint: lists of hundreds a pixel, blended to the end
+    far = np.argsort(p["means"][:, 2])[:40]   # the camera looks down -z
+    proj = _frame(W, H)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    dl = torch.rand((W * H, 4), generator=gen, device="cuda")
+    finite = _params_gpu(p)
+    base, want, _ = _records_and_gradients(raster, proj, finite, W, H, lambda t: dl, None)
+    p["sh"][far, 0] = np.inf
+    lost, rows, t = _records_and_gradients(raster, proj, _params_gpu(p), W, H, lambda t: dl, None)
+    one = torch.zeros_like(dl)
+    one[~torch.isfinite(t.colour[:, 0])] = 1.0   # the pixels that blend one of them
+    shares = np.any(_records_and_gradients(raster, proj, finite, W, H, lambda t: one, None)[0][:, 6:9] != 0, axis=1)
+    shares[far] = True
+    assert 100 < shares.sum() < 0.7 * (base != 0).any(1).sum() and not np.isfinite(lost[shares]).all()
+    for a, b in ((lost[~shares], base[~shares]), (rows[~shares], want[~shares])):
+        assert np.isfinite(a).all()
+        np.testing.assert_allclose(a, b, rtol=1e-3, atol=1e-5 * np.abs(b).max())   # the order of the atomic sums
