@@ -36,6 +36,7 @@ struct ath_raster {
     uint64_t* pairs[2] = {};   // halves of pairMemory, pairCapacity pairs each
     DeviceBuffer slotMemory, pairMemory, instances, sortScratch;   // sortScratch: the pair sort's histograms, then its look-back words
     DeviceBuffer inspect;        // ath_raster_frame_buffers' own: a slot a pair; the slots' rects and first pairs
+    cudaStream_t inspectStream = nullptr;   // made by its first call
     DeviceBuffer zeroed;         // what a frame starts at zero, cleared at once (FrameZeroed): its words first
     uint2* ranges = nullptr;     // the last frame's, there
     PinnedBuffer wordsHost;      // kFrameWords: a frame that waits (its handle's first, or timed) reads them here
@@ -342,6 +343,7 @@ extern "C" void ath_raster_destroy(ath_raster* r) {
     for (cudaEvent_t& e : r->countDone)
         if (e) cudaEventDestroy(e);
     if (r->frameDone) cudaEventDestroy(r->frameDone);
+    if (r->inspectStream) cudaStreamDestroy(r->inspectStream);
     delete r;
 }
 
@@ -903,8 +905,9 @@ extern "C" ath_status ath_raster_frame_buffers(ath_raster* r, ath_frame_buffers*
     uint64_t* const lookback = reinterpret_cast<uint64_t*>(inspect + scanAt);
     uint32_t* const ticketAndStatus = reinterpret_cast<uint32_t*>(lookback + blocks);
     uint64_t* const pairKeys = r->pairs[r->lastSorted ^ 1u];   // the pair buffer the sort left spare
-    // the frame is done: a stream that no other work waits for, or is waited for by
-    const cudaStream_t stream = cudaStreamPerThread;
+    // the frame is done: a stream that waits for no other, the legacy one included
+    if (err == cudaSuccess && !r->inspectStream) err = cudaStreamCreateWithFlags(&r->inspectStream, cudaStreamNonBlocking);
+    const cudaStream_t stream = r->inspectStream;
     if (err == cudaSuccess) err = cudaMemsetAsync(lookback, 0, blocks * 8 + 8, stream);
     if (err == cudaSuccess)
         err = launchInspectPairs(r->pairs[r->lastSorted], pairs, r->slot.keys, r->lastSlots, pairKeys, pairSplats, stream);
